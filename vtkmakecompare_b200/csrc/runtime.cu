@@ -1483,9 +1483,11 @@ static bool build_line_tables(nse_ctx* x) {
   const nse_config& c = x->cfg;
   int L = std::max(d.nx, std::max(d.ny, d.nz)) + 2;
   size_t per = 10 * (size_t)L;
-  if (!x->ltab.ensure(7 * per * sizeof(double))) return false;
+  x->part = !(c.flags & NSE_FLAG_EXACT) && part_lines_supported(d);
   size_t nfl = 4 * ((size_t)d.nx * d.nz + (size_t)d.nx * d.ny + (size_t)d.ny * d.nz);
   if (!x->lflags.ensure(nfl)) return false;
+  // the sequential solver's tables, where the partitioned one does not apply
+  if (!x->part && !x->ltab.ensure(7 * per * sizeof(double))) return false;
   double* base = x->ltab.as<double>();
   struct T { int n, kind; const double *D, *D12; bool temp; } spec[7] = {
       {d.ny, LK_UL_U, x->g.dy, x->g.dy12, false}, {d.ny, LK_UL_V, x->g.dy, x->g.dy12, false},
@@ -1493,7 +1495,7 @@ static bool build_line_tables(nse_ctx* x) {
       {d.nz, LK_CYC_T, x->g.dz, x->g.dz12, true}, {d.nx, LK_CYC_VEL, x->g.dx, x->g.dx12, false},
       {d.nx, LK_CYC_T, x->g.dx, x->g.dx12, true}};
   std::vector<double> dens(7);
-  for (int t = 0; t < 7; ++t) {
+  for (int t = 0; t < 7 && !x->part; ++t) {
     LineArgs a{};
     a.beta = spec[t].temp ? c.dt / c.Re / c.Sc / 2.0 : c.dt / c.Re / 2.0;
     a.dt = c.dt; a.eta = c.eta; a.r0 = c.rho_cp; a.l0 = c.thc;
@@ -1509,8 +1511,7 @@ static bool build_line_tables(nse_ctx* x) {
   }
   if (!NSE_CUDA(cudaStreamSynchronize(x->own))) return false;
   for (int t = 0; t < 7; ++t) x->tab[t].den = dens[t];
-  x->part = !(c.flags & NSE_FLAG_EXACT) && part_lines_supported(d);
-  if (x->mixed && !x->part) {
+  if (x->mixed && !(x->part && x_rows_per_lane(d.nx) > 0)) {
     set_error(NSE_ERR_ARG,
               "nse_ctx_create: the mixed-precision form needs nx = 32*M (M in 3,4,5,6,8,16), "
               "12 to 512 cells in y and z, and no NSE_FLAG_EXACT");
@@ -1648,7 +1649,8 @@ static bool refresh_line_flags(nse_ctx* x, cudaStream_t s) {
       x->nmasked[dir][comp] = (int)nids;
       if (!x->slots[dir][comp].ensure(nlines * sizeof(int)) ||
           !x->ids[dir][comp].ensure(std::max<size_t>(1, nids) * sizeof(int)) ||
-          !x->mtab[dir][comp].ensure(std::max<size_t>(1, nids) * stride * sizeof(double)))
+          (!x->part &&
+           !x->mtab[dir][comp].ensure(std::max<size_t>(1, nids) * stride * sizeof(double))))
         return false;
       if (!NSE_CUDA(cudaMemcpyAsync(x->slots[dir][comp].p, slot, nlines * sizeof(int),
                                     cudaMemcpyHostToDevice, s)))
@@ -1657,8 +1659,9 @@ static bool refresh_line_flags(nse_ctx* x, cudaStream_t s) {
           !NSE_CUDA(cudaMemcpyAsync(x->ids[dir][comp].p, idl, nids * sizeof(int),
                                     cudaMemcpyHostToDevice, s)))
         return false;
-      launch_line_tables_masked(dir, kind, d, x->g, c1, a, x->ids[dir][comp].as<int>(),
-                                (int)nids, x->mtab[dir][comp].as<double>(), s);
+      if (!x->part)
+        launch_line_tables_masked(dir, kind, d, x->g, c1, a, x->ids[dir][comp].as<int>(),
+                                  (int)nids, x->mtab[dir][comp].as<double>(), s);
       if (x->part) {
         size_t ps = part_table_stride(dir, kind, d);
         if (!x->pmtab[dir][comp].ensure(std::max<size_t>(1, nids) * ps * sizeof(double)))
@@ -2394,7 +2397,7 @@ static void autotune_lines(nse_ctx* x) {
       }
       std::vector<int> cand;
       if (dir == 0) {
-        if (x_nl_candidates(x) < 2) continue;
+        if (x_rows_per_lane(d.nx) == 0 || x_nl_candidates(x) < 2) continue;
         cand = {2, 1};
         // the staged loads (one warp per line, M = nx/32 even)
         const int M = x_rows_per_lane(d.nx);
