@@ -4,7 +4,8 @@ import numpy as np
 import pytest
 
 from tests._helpers import rel_l2
-from tests.test_gpu_step import make_case, make_ctx, run_oracle
+from tests.test_gpu_step import STATE, make_case, make_ctx, run_oracle
+from vtkmakecompare_b200 import solver as S
 
 pytestmark = pytest.mark.gpu
 
@@ -23,3 +24,37 @@ def test_x_lines_of_any_length_match_oracle(n):
         ctx.step(3)
         for k in ("u", "v", "w", "p", "T", "u_ta", "T_pre"):
             assert rel_l2(ctx.download(k), ref.f[k]) < 1e-10, k
+
+
+# Inside one call, steps that another two follow write only what the next step
+# reads (k_correct_step, the wrapped divergence, u_ta from phi under the mask);
+# one call per step writes every field every time.  Same bits, with a mask that
+# crosses the periodic faces and touches both walls, on grids with remainders of
+# the correction's 32 x 8 x 4 tiles and without; replayed and eager steps.
+@pytest.mark.parametrize("prec,n", [(S.FP64, (50, 15, 20)), (S.FP64, (64, 16, 12)),
+                                    (S.FP64, (90, 14, 25)), (S.MIXED, (96, 17, 15)),
+                                    (S.MIXED, (64, 24, 18))])
+def test_steps_of_one_call_match_calls_of_one_step(prec, n):
+    g, f, _, par = make_case(*n, seed=21)
+    X, Y, Z = np.ogrid[:n[0], :n[1], :n[2]]
+    c1 = np.asfortranarray(0.5 * ((X < 3) | (X >= n[0] - 2)) + 0.25 * (Z < 2) +
+                           0.25 * ((Y < 2) | (Y >= n[1] - 2)) + 0.0 * X)
+    out = []
+    for calls in ([1] * 13, [13], [2, 3, 4, 4]):
+        cfg = S.Config(*n, par["dt"], par["Re"], par["Sc"], 50.0, g["xl"], g["yl"], g["zl"],
+                       y0=-1.0, ystretch=2.0, body_force=par["force"], t_bot=par["tbot"],
+                       t_solid=par["tsolid"], precision=prec)
+        with S.Context(cfg) as ctx:
+            for k in ("u", "v", "w", "T"):
+                ctx.upload(k, f[k])
+            ctx.upload("cellvalue", c1)
+            ctx.project()
+            ctx.start()
+            ctx.set_shapes(0, 0)
+            ctx.set_line_shapes(0, 2)
+            for m in calls:
+                ctx.step(m)
+            out.append({k: ctx.download(k) for k in STATE})
+    for other in out[1:]:
+        for k in STATE:
+            assert np.array_equal(out[0][k], other[k]), k

@@ -79,13 +79,19 @@ bool run_forward(nse_adjoint* a) {
   const double w = 1.0 / (double)(N - n0 + 1);
   double* J = a->J.as<double>();
   if (!NSE_CUDA(cudaMemsetAsync(J, 0, 2 * sizeof(double), ci.s))) return false;
+  int in = END_FULL;
   for (int n = 1; n <= N; ++n) {
     if ((n - 1) % K == 0) {
       const int m = (n - 1) / K;
       a->ck_l[m] = ctx_get_l(a->x);
       if (!copy_fields(a, a->field(a->ck, (size_t)m * NS), kState, NS, false)) return false;
     }
-    ctx_step_rec(a->x, nullptr);
+    // every field after the last two steps, what a checkpoint holds before
+    // one, else what the next step reads
+    int out = n + 2 > N ? END_FULL : (n % K == 0 ? END_TA : END_LEAN);
+    if (!ctx_lean_ok(a->x)) out = END_FULL;
+    ctx_step_rec(a->x, nullptr, in, out);
+    in = out;
     if (n >= n0)
       launch_wall_flux(ci.d, g, ctx_field(a->x, NSE_T), c.t_bot, c.thc, c.xl, c.zl, w, J, ci.s);
   }
@@ -300,11 +306,15 @@ int nse_adjoint_gradient(nse_adjoint* a, double* J, double* grad_c1) {
     const int first = m * K + 1, last = std::min(N, first + K - 1);
     if (!copy_fields(a, a->field(a->ck, (size_t)m * NS), kState, NS, true)) return NSE_ERR_CUDA;
     ctx_set_l(a->x, a->ck_l[m]);
+    int in = END_FULL;
     for (int n = first; n <= last; ++n) {
       const int r = n - first;
       if (!copy_fields(a, a->field(a->seg, (size_t)r * kSeg), segIds, kSeg, false))
         return NSE_ERR_CUDA;
-      ctx_step_rec(a->x, recp.data() + (size_t)r * kRec);
+      // the reverse sweep reads u_ta of every step, but no p, u_ep2 or divu
+      const int out = ctx_lean_ok(a->x) ? END_TA : END_FULL;
+      ctx_step_rec(a->x, recp.data() + (size_t)r * kRec, in, out);
+      in = out;
     }
     for (int n = last; n >= first; --n) {
       const int r = n - first;

@@ -159,7 +159,7 @@ void launch_rhs_fast(const Dims& d, const GridDev& g, const GridRcp& rg, const S
                      const double* u_ta, const double* v_ta, const double* w_ta,
                      double* u_pre, double* v_pre, double* w_pre, double* T_pre,
                      const double* c1, double* u_a, double* v_a, double* w_a, double* u_T,
-                     cudaStream_t s, int shape = 0);
+                     cudaStream_t s, int shape = 0, const double* phi = nullptr);
 
 // ADI line solves; mask is c1 (nx,ny,nz); comp: 0 u (c2), 1 v (c3), 2 w (c4)
 struct LineScratch {
@@ -239,11 +239,12 @@ void launch_fft_fwd_x(const PoissonPlan& pp, const Dims& d, const double* FP,
                       const GridRcp* rg = nullptr, int j0 = 0, int nj = 0);
 void launch_fft_z(const PoissonPlan& pp, bool inverse, cudaStream_t s, int j0 = 0, int nj = 0);
 // divergence right-hand side of mkp.f:90-97 (reciprocal spacings) into the
-// P2S sample layout of `out`, for the forward x pass in src_mode 0
+// P2S sample layout of `out`, for the forward x pass in src_mode 0; wrap: the
+// ghosts of u*, v*, w* are not read (the values SET_BC gives them are used)
 void launch_div_src(const Dims& d, const GridRcp& rg, const double* ut, const double* vt,
-                    const double* wt, double dt, double* out, cudaStream_t s);
+                    const double* wt, double dt, double* out, bool wrap, cudaStream_t s);
 void launch_div_src32(const Dims& d, const GridRcp& rg, const float* ut, const float* vt,
-                      const float* wt, double dt, double* out, cudaStream_t s);
+                      const float* wt, double dt, double* out, bool wrap, cudaStream_t s);
 
 void launch_spn(const PoissonPlan& pp, bool do_spn, bool do_sp0b, cudaStream_t s);
 // SPN pivot tables of the two-ended elimination (0 from spn_split: no
@@ -295,6 +296,17 @@ void launch_correct_pipe(const Dims& d, const GridRcp& rg, const double* PHI, co
                          double* v_ep2, double* w_ep2, double* divu, double dt, cudaStream_t s,
                          int shape = 0);
 
+// The correction between two steps of one nse_step call: u, v, w (interior
+// and the ghosts SET_BC gives them) from phi and u*, v*, w*, of which only
+// interior cells are read; u_ta too when given.  Nobody sees p, u_ep2, divu
+// or (the next right-hand side takes it from phi) u_ta of such a step.
+void launch_correct_step(const Dims& d, const GridRcp& rg, const double* PHI, const double* ut,
+                         const double* vt, const double* wt, double* u, double* v, double* w,
+                         double* u_ta, double* v_ta, double* w_ta, double dt, cudaStream_t s);
+void launch_correct_step_f32(const Dims& d, const GridRcp& rg, const double* PHI, const float* ut,
+                             const float* vt, const float* wt, double* u, double* v, double* w,
+                             double dt, cudaStream_t s);
+
 // level set (set_levelset.f)
 void launch_levelset_iter(const Dims& d, const GridDev& g, const double* phi0,
                           const double* phi, double* phi_new, double dtau, cudaStream_t s);
@@ -322,8 +334,14 @@ double* ctx_field(nse_ctx* x, int id);
 int ctx_get_l(nse_ctx* x);
 void ctx_set_l(nse_ctx* x, int l);
 // one step of the context; with rec given, the line-solve passes record their
-// inputs and outputs (16 padded fields, see nse_ctx::rec)
-void ctx_step_rec(nse_ctx* x, double* const* rec);
+// inputs and outputs (16 padded fields, see nse_ctx::rec).  in, out: see
+// StepEnd (out is taken as END_FULL where ctx_lean_ok says no)
+void ctx_step_rec(nse_ctx* x, double* const* rec, int in, int out);
+// What a step leaves behind, and what the next one may start from.  END_FULL:
+// every field, as MKP writes them.  END_LEAN: u, v, w with their ghosts, T and
+// the histories (phi holds the pressure); END_TA: u_ta, v_ta, w_ta as well.
+enum StepEnd { END_FULL = 0, END_LEAN, END_TA };
+bool ctx_lean_ok(nse_ctx* x);
 // the line solve of (dir, comp) of the step on the field f (ft = fb = 0)
 void ctx_line_solve(nse_ctx* x, int dir, int comp, double* f, cudaStream_t s);
 

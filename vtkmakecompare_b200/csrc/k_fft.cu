@@ -124,13 +124,19 @@ struct FwdSrc {
   double rdx2, rdz2;  // 1/dx^2, 1/dz^2 of the uniform x, z spacings
 };
 
-// FP64 divergence right-hand side at cell (I, J, K) (all three >= 1)
-template <class S>
+// FP64 divergence right-hand side at cell (I, J, K) (all three >= 1); WRAP:
+// from interior cells alone, with the values SET_BC gives the ghosts
+// (periodic u and w, v = 0 on both walls)
+template <bool WRAP = false, class S>
 __device__ __forceinline__ double div_rhs(const Dims& d, const FwdSrc<S>& q, int I, int J, int K) {
   long c = d.P(I, J, K);
-  const double du = (double)q.ut[c] - (double)q.ut[c - 1];
-  const double dv = (double)q.vt[c] - (double)q.vt[c - d.sx];
-  const double dw = (double)q.wt[c] - (double)q.wt[c - d.sy];
+  const long xm = WRAP && I == 1 ? c + d.nx - 1 : c - 1;
+  const long zm = WRAP && K == 1 ? c + (d.nz - 1) * d.sy : c - d.sy;
+  const double v0 = WRAP && J == d.ny ? 0.0 : (double)q.vt[c];
+  const double v1 = WRAP && J == 1 ? 0.0 : (double)q.vt[c - d.sx];
+  const double du = (double)q.ut[c] - (double)q.ut[xm];
+  const double dv = v0 - v1;
+  const double dw = (double)q.wt[c] - (double)q.wt[zm];
   if (q.use_rcp)
     return (du * q.rg.rdx[I] + dv * q.rg.rdy[J] + dw * q.rg.rdz[K]) * (1.0 / q.dt);
   return (du / q.g.dx[I] + dv / q.g.dy[J] + dw / q.g.dz[K]) / q.dt;
@@ -144,14 +150,14 @@ __device__ __forceinline__ double div_rhs(const Dims& d, const FwdSrc<S>& q, int
 // for two rows at once and stays latency-bound (0.180 ms at 256x192x256);
 // this streaming kernel plus the plain transform take 0.145 ms, with
 // identical values (the same expression, evaluated once per cell).
-template <class S>
+template <class S, bool WRAP>
 __global__ void __launch_bounds__(128) k_div_src(Dims d, FwdSrc<S> q, double* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int J = 1 + blockIdx.y;
   const int k = blockIdx.z;
   if (i >= d.nx) return;
   const int I = (i == 0) ? d.nx : i, K = (k == 0) ? d.nz : k;
-  out[d.P(i, J, k)] = div_rhs(d, q, I, J, K);
+  out[d.P(i, J, k)] = div_rhs<WRAP>(d, q, I, J, K);
 }
 
 // ------------------------------------------------------------- x forward --
@@ -1132,20 +1138,21 @@ void launch_fft_fwd_x(const PoissonPlan& pp, const Dims& d, const double* FP,
 
 template <class S>
 static void div_src(const Dims& d, const GridRcp& rg, const S* ut, const S* vt, const S* wt,
-                    double dt, double* out, cudaStream_t s) {
+                    double dt, double* out, bool wrap, cudaStream_t s) {
   FwdSrc<S> q{};
   q.ut = ut; q.vt = vt; q.wt = wt; q.rg = rg; q.use_rcp = 1; q.dt = dt;
   dim3 grid((d.nx + 127) / 128, d.ny, d.nz);
   count_launch();
-  k_div_src<S><<<grid, 128, 0, s>>>(d, q, out);
+  if (wrap) k_div_src<S, true><<<grid, 128, 0, s>>>(d, q, out);
+  else k_div_src<S, false><<<grid, 128, 0, s>>>(d, q, out);
 }
 void launch_div_src(const Dims& d, const GridRcp& rg, const double* ut, const double* vt,
-                    const double* wt, double dt, double* out, cudaStream_t s) {
-  div_src<double>(d, rg, ut, vt, wt, dt, out, s);
+                    const double* wt, double dt, double* out, bool wrap, cudaStream_t s) {
+  div_src<double>(d, rg, ut, vt, wt, dt, out, wrap, s);
 }
 void launch_div_src32(const Dims& d, const GridRcp& rg, const float* ut, const float* vt,
-                      const float* wt, double dt, double* out, cudaStream_t s) {
-  div_src<float>(d, rg, ut, vt, wt, dt, out, s);
+                      const float* wt, double dt, double* out, bool wrap, cudaStream_t s) {
+  div_src<float>(d, rg, ut, vt, wt, dt, out, wrap, s);
 }
 
 // g0, ng: the groups of 16 kx columns to transform (ng = 0: all; only the

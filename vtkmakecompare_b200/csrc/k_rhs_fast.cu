@@ -15,9 +15,9 @@ void launch_rhs_fast(const Dims& d, const GridDev& g, const GridRcp& rg, const S
                      const double* u_ta, const double* v_ta, const double* w_ta,
                      double* u_pre, double* v_pre, double* w_pre, double* T_pre,
                      const double* c1, double* u_a, double* v_a, double* w_a, double* u_T,
-                     cudaStream_t s, int shape) {
+                     cudaStream_t s, int shape, const double* phi) {
   rhs_fast<double, double>(d, g, rg, sp, u, v, w, T, u_ta, v_ta, w_ta, u_pre, v_pre, w_pre,
-                           T_pre, c1, u_a, v_a, w_a, u_T, s, shape);
+                           T_pre, c1, u_a, v_a, w_a, u_T, phi, s, shape);
 }
 
 }  // namespace nse
@@ -82,6 +82,12 @@ void launch_correct_fast(const Dims& d, const GridRcp& rg, const double* PHI, co
 }  // namespace nse
 
 namespace nse {
+
+// f - dt g with each operation rounded on its own, so that every kernel that
+// corrects a velocity gives the same bits whether or not it also stores dt g
+__device__ __forceinline__ double corrected(double f, double dt, double g) {
+  return __dsub_rn(f, __dmul_rn(dt, g));
+}
 
 // ----------------------------------------------------- pipelined correction
 // mkp.f:141-217 for interior cells (1..n in every direction), marching in z
@@ -262,9 +268,9 @@ __global__ void __launch_bounds__(TXW * TY, MINB) k_correct_pipe(
       const double ph = PH(qc, 0, 0), phx = PH(qc, 1, 0), phy = PH(qc, 0, 1), phz = PH(qp, 0, 0),
                    phxm = PH(qc, -1, 0), phym = PH(qc, 0, -1), phzm = PH(qm, 0, 0);
       const double gx = (phx - ph) * rx12, gy = (phy - ph) * ry12, gz = (phz - ph) * rz12;
-      const double un = (double)fc[Lay::ui(tx, ty, 0)] - dt * gx;
-      const double vn = (double)fc[Lay::VO + Lay::vi(tx, ty, 0)] - dt * gy;
-      const double wn = (double)fc[Lay::WO + Lay::wi(tx, ty)] - dt * gz;
+      const double un = corrected((double)fc[Lay::ui(tx, ty, 0)], dt, gx);
+      const double vn = corrected((double)fc[Lay::VO + Lay::vi(tx, ty, 0)], dt, gy);
+      const double wn = corrected((double)fc[Lay::WO + Lay::wi(tx, ty)], dt, gz);
       const double um = (double)fc[Lay::ui(tx, ty, -1)] - dt * ((ph - phxm) * rx12m);
       const double vm = (double)fc[Lay::VO + Lay::vi(tx, ty, -1)] - dt * ((ph - phym) * ry12m);
       const double wm = (double)fm[Lay::WO + Lay::wi(tx, ty)] - dt * ((ph - phzm) * rz12m);
@@ -314,12 +320,112 @@ __global__ void k_correct_faces(Dims d, GridRcp rg, const double* __restrict__ P
   double gx = (LD(PHI, c + 1) - ph) * LD(rg.rdx12, i);
   double gy = (LD(PHI, c + d.sx) - ph) * LD(rg.rdy12, j);
   double gz = (LD(PHI, c + d.sy) - ph) * LD(rg.rdz12, k);
-  u[c] = (double)LD(ut, c) - dt * gx;
-  v[c] = (double)LD(vt, c) - dt * gy;
-  w[c] = (double)LD(wt, c) - dt * gz;
+  u[c] = corrected((double)LD(ut, c), dt, gx);
+  v[c] = corrected((double)LD(vt, c), dt, gy);
+  w[c] = corrected((double)LD(wt, c), dt, gz);
   u_ta[c] = (H)(dt * gx);
   v_ta[c] = (H)(dt * gy);
   w_ta[c] = (H)(dt * gz);
+}
+
+// ------------------------------------------- correction between two steps
+// u = u* - dt grad(phi) and no more: of a step that another step of the same
+// call follows, p, u_ep2 and divu are overwritten unseen, and u_ta is needed
+// only under the mask, where the right-hand side forms it from phi.  4 fields
+// in and 3 out instead of 7 and 11, and no launch around it: neighbours past
+// the last cell are taken at their periodic image (PHIBC's copies are not
+// read), and the thread that owns a boundary cell also writes the ghosts that
+// SET_BC copies from it.  Bound by HBM; each thread takes CSZ planes so that
+// all its loads are in flight at once.
+constexpr int CSZ = 4;
+template <class H, bool TA>
+__global__ void __launch_bounds__(256) k_correct_step(
+    Dims d, GridRcp rg, const double* __restrict__ PHI, const H* __restrict__ UT,
+    const H* __restrict__ VT, const H* __restrict__ WT, double* __restrict__ u,
+    double* __restrict__ v, double* __restrict__ w, H* __restrict__ u_ta, H* __restrict__ v_ta,
+    H* __restrict__ w_ta, double dt) {
+  const int i = 1 + blockIdx.x * 32 + threadIdx.x, j = 1 + blockIdx.y * 8 + threadIdx.y;
+  const int k0 = 1 + blockIdx.z * CSZ;
+  if (i > d.nx || j > d.ny) return;
+  const int nk = min(CSZ, d.nz - k0 + 1);
+  const long c0 = d.P(i, j, k0);
+  const long xp = i < d.nx ? 1 : 1 - d.nx;
+  const bool top = j == d.ny;
+  const double rx12 = LD(rg.rdx12, i), ry12 = LD(rg.rdy12, j);
+  double ph[CSZ + 1], px[CSZ], py[CSZ], us[CSZ], vs[CSZ], ws[CSZ];
+#pragma unroll
+  for (int q = 0; q < CSZ; ++q) {
+    const long c = c0 + min(q, nk - 1) * d.sy;
+    ph[q] = LD(PHI, c);
+    px[q] = LD(PHI, c + xp);
+    py[q] = LD(PHI, top ? c : c + d.sx);
+    us[q] = (double)LD(UT, c);
+    vs[q] = (double)LD(VT, c);
+    ws[q] = (double)LD(WT, c);
+  }
+  const double pn = LD(PHI, k0 + nk > d.nz ? d.P(i, j, 1) : c0 + nk * d.sy);
+  const bool edge = i == 1 || i == d.nx || j == 1 || top;
+#pragma unroll
+  for (int q = 0; q < CSZ; ++q) {
+    if (q >= nk) break;
+    const int k = k0 + q;
+    const long c = c0 + q * d.sy;
+    const double pz = q == nk - 1 ? pn : ph[q < CSZ - 1 ? q + 1 : q];
+    const double gx = (px[q] - ph[q]) * rx12, gy = (py[q] - ph[q]) * ry12,
+                 gz = (pz - ph[q]) * LD(rg.rdz12, k);
+    const double un = corrected(us[q], dt, gx), wn = corrected(ws[q], dt, gz);
+    const double vn = top ? 0.0 : corrected(vs[q], dt, gy);  // the wall face
+    u[c] = un;
+    v[c] = vn;
+    w[c] = wn;
+    if constexpr (TA) {
+      u_ta[c] = (H)(dt * gx);
+      v_ta[c] = (H)(dt * gy);
+      w_ta[c] = (H)(dt * gz);
+    }
+    if (edge || k == 1 || k == d.nz) {
+      // the ghost images of this cell: periodic in x and z, u and w negated
+      // behind the walls (v's wall faces are zero already)
+      const int xi[3] = {i, i == 1 ? d.nx + 1 : -1, i == d.nx ? 0 : -1};
+      const int zi[3] = {k, k == 1 ? d.nz + 1 : -1, k == d.nz ? 0 : -1};
+      const int yi[3] = {j, j == 1 ? 0 : -1, top ? d.ny + 1 : -1};
+      for (int a = 0; a < 3; ++a)
+        for (int b = 0; b < 3; ++b) {
+          if (xi[a] < 0 || zi[b] < 0) continue;
+          for (int e = 0; e < 3; ++e) {
+            if (yi[e] < 0 || a + b + e == 0) continue;
+            const long g = d.P(xi[a], yi[e], zi[b]);
+            u[g] = e ? -un : un;
+            w[g] = e ? -wn : wn;
+            if (e == 0) v[g] = vn;
+          }
+        }
+    }
+  }
+}
+
+template <class H>
+static void correct_step(const Dims& d, const GridRcp& rg, const double* PHI, const H* ut,
+                         const H* vt, const H* wt, double* u, double* v, double* w, H* u_ta,
+                         H* v_ta, H* w_ta, double dt, cudaStream_t s) {
+  dim3 grid((d.nx + 31) / 32, (d.ny + 7) / 8, (d.nz + CSZ - 1) / CSZ), block(32, 8);
+  count_launch();
+  if (u_ta)
+    k_correct_step<H, true><<<grid, block, 0, s>>>(d, rg, PHI, ut, vt, wt, u, v, w, u_ta, v_ta,
+                                                   w_ta, dt);
+  else
+    k_correct_step<H, false><<<grid, block, 0, s>>>(d, rg, PHI, ut, vt, wt, u, v, w, u_ta, v_ta,
+                                                    w_ta, dt);
+}
+void launch_correct_step(const Dims& d, const GridRcp& rg, const double* PHI, const double* ut,
+                         const double* vt, const double* wt, double* u, double* v, double* w,
+                         double* u_ta, double* v_ta, double* w_ta, double dt, cudaStream_t s) {
+  correct_step<double>(d, rg, PHI, ut, vt, wt, u, v, w, u_ta, v_ta, w_ta, dt, s);
+}
+void launch_correct_step_f32(const Dims& d, const GridRcp& rg, const double* PHI, const float* ut,
+                             const float* vt, const float* wt, double* u, double* v, double* w,
+                             double dt, cudaStream_t s) {
+  correct_step<float>(d, rg, PHI, ut, vt, wt, u, v, w, nullptr, nullptr, nullptr, dt, s);
 }
 
 template <class H, int TY, int NS, int MINB, int TM = 0, int KC = CKCHUNK>

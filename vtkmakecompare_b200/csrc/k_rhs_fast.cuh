@@ -230,7 +230,8 @@ __global__ void __launch_bounds__(TXW * TY, MINB) k_rhs_fast(
     const H* __restrict__ U_TA, const H* __restrict__ V_TA, const H* __restrict__ W_TA,
     H* __restrict__ U_PRE, H* __restrict__ V_PRE, H* __restrict__ W_PRE, H* __restrict__ T_PRE,
     const double* __restrict__ C1, H* __restrict__ U_A, H* __restrict__ V_A,
-    H* __restrict__ W_A, H* __restrict__ U_T, const __grid_constant__ RhsMaps tm) {
+    H* __restrict__ W_A, H* __restrict__ U_T, const double* __restrict__ PHI,
+    const __grid_constant__ RhsMaps tm) {
   extern __shared__ __align__(128) char smc[];
   char* sm = smc;
   using Lay = RhsLay<H, TY, TM>;
@@ -347,6 +348,12 @@ __global__ void __launch_bounds__(TXW * TY, MINB) k_rhs_fast(
       const R c4 = (K < d.nz) ? (cc1 + C1AT(pp, 0, 0)) * R(0.5) : cc1;
       const H* hist = reinterpret_cast<const H*>(pc + Lay::HOFF) + t0;
       const bool solid = (c2 != R(0)) || (c3 != R(0)) || (c4 != R(0)) || (cc1 != R(0));
+      // u_ta, v_ta, w_ta: the fields, or with PHI given dt grad(phi) of the
+      // previous step, whose correction then did not write them (the same
+      // value: the correction's expression, from interior cells of phi)
+      auto ta = [&](const H* f, long nb, double r12) {
+        return PHI ? (R)(H)(sp.dt * ((LD(PHI, nb) - LD(PHI, c)) * r12)) : (R)LD(f, c);
+      };
     // u
     {
       const R uc = AT(pc, 0, 0, 0), uxp = AT(pc, 0, 1, 0), uxm = AT(pc, 0, -1, 0),
@@ -369,7 +376,7 @@ __global__ void __launch_bounds__(TXW * TY, MINB) k_rhs_fast(
       R ua = a1 * uv + a2 * (R)hist[0] + kd * L;
       U_PRE[c] = uv;
       if (solid && c2 != R(0)) {
-        ua += (R)sp.eta * c2 * LD(U_TA, c) * DT;
+        ua += (R)sp.eta * c2 * ta(U_TA, I < d.nx ? c + 1 : c + 1 - d.nx, LD(rg.rdx12, I)) * DT;
         U_A[c] = (uc + ua) / (R(1) + (R)sp.eta * c2 * DT);
       } else {
         U_A[c] = uc + ua;
@@ -396,7 +403,8 @@ __global__ void __launch_bounds__(TXW * TY, MINB) k_rhs_fast(
                  ((vzp - vc) * rz12 - (vc - vzm) * rz12m) * rz;
       R va = a1 * vv + a2 * (R)hist[TILE] + kd * L;
       V_PRE[c] = vv;
-      if (solid && c3 != R(0)) va += (R)sp.eta * c3 * LD(V_TA, c) * DT;
+      if (solid && c3 != R(0))
+        va += (R)sp.eta * c3 * ta(V_TA, J < d.ny ? c + d.sx : c, LD(rg.rdy12, J)) * DT;
       if (J == d.ny) va = R(0);  // set_bc(u_a,v_a,...) zeroes v_a(:,ny,:)
       if (solid && c3 != R(0)) V_A[c] = (vc + va) / (R(1) + (R)sp.eta * c3 * DT);
       else V_A[c] = vc + va;
@@ -423,7 +431,8 @@ __global__ void __launch_bounds__(TXW * TY, MINB) k_rhs_fast(
       R wa = a1 * wv + a2 * (R)hist[2 * TILE] + kd * L;
       W_PRE[c] = wv;
       if (solid && c4 != R(0)) {
-        wa += (R)sp.eta * c4 * LD(W_TA, c) * DT;
+        wa += (R)sp.eta * c4 *
+              ta(W_TA, K < d.nz ? c + d.sy : c - (d.nz - 1) * d.sy, LD(rg.rdz12, K)) * DT;
         W_A[c] = (wc + wa) / (R(1) + (R)sp.eta * c4 * DT);
       } else {
         W_A[c] = wc + wa;
@@ -485,7 +494,8 @@ template <class H, class CT, int TY, int NS, int MINB, int TM = 0>
 static bool rhs_go(const Dims& d, const GridDev& g, const GridRcp& rg, const StepParams& sp,
                    const double* u, const double* v, const double* w, const double* T,
                    const H* u_ta, const H* v_ta, const H* w_ta, H* u_pre, H* v_pre, H* w_pre,
-                   H* T_pre, const double* c1, H* u_a, H* v_a, H* w_a, H* u_T, cudaStream_t s) {
+                   H* T_pre, const double* c1, H* u_a, H* v_a, H* w_a, H* u_T, const double* phi,
+                   cudaStream_t s) {
   RhsMaps tm;
   memset(&tm, 0, sizeof(tm));
   size_t smem = (size_t)NS * RhsLay<H, TY, TM>::SLOT;
@@ -506,7 +516,7 @@ static bool rhs_go(const Dims& d, const GridDev& g, const GridRcp& rg, const Ste
   cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   count_launch();
   kern<<<grid, block, smem, s>>>(d, g, rg, sp, u, v, w, T, u_ta, v_ta, w_ta, u_pre, v_pre, w_pre,
-                                 T_pre, c1, u_a, v_a, w_a, u_T, tm);
+                                 T_pre, c1, u_a, v_a, w_a, u_T, phi, tm);
   return true;
 }
 
@@ -523,15 +533,15 @@ static void rhs_fast(const Dims& d, const GridDev& g, const GridRcp& rg, const S
                      const double* u, const double* v, const double* w, const double* T,
                      const H* u_ta, const H* v_ta, const H* w_ta, H* u_pre, H* v_pre, H* w_pre,
                      H* T_pre, const double* c1, H* u_a, H* v_a, H* w_a, H* u_T,
-                     cudaStream_t s, int shape) {
+                     const double* phi, cudaStream_t s, int shape) {
   using Sh = RhsShape<H, CT>;
 #define NSE_RHS_GO(TY_, NS_, MB_)                                                           \
   rhs_go<H, CT, TY_, NS_, MB_>(d, g, rg, sp, u, v, w, T, u_ta, v_ta, w_ta, u_pre, v_pre,    \
-                               w_pre, T_pre, c1, u_a, v_a, w_a, u_T, s)
+                               w_pre, T_pre, c1, u_a, v_a, w_a, u_T, phi, s)
   constexpr int TM = sizeof(H) == 8 ? 1 : 2;
 #define NSE_RHS_TMA(TY_, NS_, MB_)                                                              \
   done = rhs_go<H, CT, TY_, NS_, MB_, TM>(d, g, rg, sp, u, v, w, T, u_ta, v_ta, w_ta, u_pre,    \
-                                          v_pre, w_pre, T_pre, c1, u_a, v_a, w_a, u_T, s)
+                                          v_pre, w_pre, T_pre, c1, u_a, v_a, w_a, u_T, phi, s)
   {
     bool done = false;
     if (shape == 4) NSE_RHS_TMA(4, 5, 3);

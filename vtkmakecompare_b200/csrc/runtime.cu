@@ -60,7 +60,7 @@ void launch_rhs_f32(const Dims& d, const GridDev& g, const GridRcp& rg, const St
                     const float* u_ta, const float* v_ta, const float* w_ta, float* u_pre,
                     float* v_pre, float* w_pre, float* T_pre, const double* c1, float* u_a,
                     float* v_a, float* w_a, float* u_T, bool math64, cudaStream_t s,
-                    int shape = 0);
+                    int shape = 0, const double* phi = nullptr);
 void launch_correct_f32(const Dims& d, const GridRcp& rg, const double* PHI, const float* ut,
                         const float* vt, const float* wt, double* p, double* u, double* v,
                         double* w, float* u_ta, float* v_ta, float* w_ta, float* u_ep2,
@@ -1428,12 +1428,16 @@ struct nse_ctx {
   // form of the fast two-ended SPN, TMA tiles or cp.async staging
   // (autotune_spn_form; the plan's spn_cp)
   bool spn_tuned = false;
-  // one-step CUDA graphs of nse_step (step_replay), one per temperature
-  // buffer a step starts from, with the buffer pair the step leaves behind
-  cudaGraphExec_t sg[2] = {nullptr, nullptr};
-  void* sg_t[2] = {nullptr, nullptr};
-  DBuf sg_T[2], sg_uT[2];
-  long long sg_nk[2] = {0, 0};    // kernels in each graph
+  // one-step CUDA graphs of nse_step (step_replay), one per way the step
+  // starts and ends (kind) and temperature buffer it starts from, with the
+  // buffer pair it leaves behind
+  struct StepGraph {
+    cudaGraphExec_t ex = nullptr;
+    int kind = -1, uses = 0;
+    void* t = nullptr;
+    DBuf T, uT;
+    long long nk = 0;  // kernels in the graph
+  } sg[8];
   unsigned long long sg_sig = 0;  // launch shapes the graphs were captured with
   void* hpin = nullptr;           // pinned staging of the masked line lists
   size_t hpin_n = 0;              // its capacity (ints)
@@ -1466,10 +1470,9 @@ unsigned long long shape_sig(const nse_ctx* x) {
   return h;
 }
 void drop_step_graphs(nse_ctx* x) {
-  for (int k = 0; k < 2; ++k) {
-    if (x->sg[k]) cudaGraphExecDestroy(x->sg[k]);
-    x->sg[k] = nullptr;
-    x->sg_t[k] = nullptr;
+  for (auto& g : x->sg) {
+    if (g.ex) cudaGraphExecDestroy(g.ex);
+    g.ex = nullptr;
   }
 }
 }  // namespace
@@ -2201,7 +2204,8 @@ static void autotune_correct(nse_ctx* x, const H* ut, const H* vt, const H* wt) 
 // MKP in the mixed-precision form: FP32 u*, v*, w*; the FP64 solve of their
 // FP64 divergence (or, with NSE_FLAG_POISSON32, the FP32 spectral solve with
 // FP64 residual refinement); FP64 correction of the FP64 state
-static void ctx_mkp_f32(nse_ctx* x, const float* ut, const float* vt, const float* wt) {
+static void ctx_mkp_f32(nse_ctx* x, const float* ut, const float* vt, const float* wt,
+                        int out = END_FULL) {
   const Dims& d = x->d;
   cudaStream_t s = x->stream;
   const PoissonPlan& pp = x->pb.pp;
@@ -2210,11 +2214,11 @@ static void ctx_mkp_f32(nse_ctx* x, const float* ut, const float* vt, const floa
   const bool p64 = (x->cfg.flags & NSE_FLAG_POISSON32) == 0;
   mark(x, PH_FFTX_F);
   if (p64 && poisson3(x)) {
-    launch_div_src32(d, x->rg, ut, vt, wt, dt, phi, s);
+    launch_div_src32(d, x->rg, ut, vt, wt, dt, phi, false, s);
     ctx_poisson64(x, phi, true);
   } else if (p64) {
     autotune_mid(x);
-    launch_div_src32(d, x->rg, ut, vt, wt, dt, phi, s);
+    launch_div_src32(d, x->rg, ut, vt, wt, dt, phi, out != END_FULL, s);
     launch_fft_fwd_x(pp, d, phi, nullptr, nullptr, nullptr, x->g, 1.0, 0, s);
   } else {
     launch_fft_fwd_x_f32(pp, d, x->g, x->rg, ut, vt, wt, dt, nullptr, dx, dz, 1, s);
@@ -2233,6 +2237,11 @@ static void ctx_mkp_f32(nse_ctx* x, const float* ut, const float* vt, const floa
     mark(x, PH_FFTX_I);
     if (p64) launch_fft_inv_x(pp, d, phi, s);
     else launch_fft_inv_x_f32(pp, d, phi, false, s);
+    if (out != END_FULL) {
+      launch_correct_step_f32(d, x->rg, phi, ut, vt, wt, F(x, NSE_U), F(x, NSE_V), F(x, NSE_W),
+                              dt, s);
+      return;
+    }
     mark(x, PH_PHIBC);
     launch_phibc(d, phi, s);
   }
@@ -2255,8 +2264,10 @@ static void ctx_mkp_f32(nse_ctx* x, const float* ut, const float* vt, const floa
 }
 
 // MKP (mkp.f:9-220) with u_temp = (ut, vt, wt); writes u, v, w, p, u_ta,
-// u_ep2, divu of the context and leaves phi in the NSE_PHI field
-static void ctx_mkp(nse_ctx* x, const double* ut, const double* vt, const double* wt) {
+// u_ep2, divu of the context (what `out` asks for of them) and leaves phi in
+// the NSE_PHI field
+static void ctx_mkp(nse_ctx* x, const double* ut, const double* vt, const double* wt,
+                    int out = END_FULL) {
   const Dims& d = x->d;
   cudaStream_t s = x->stream;
   double* phi = F(x, NSE_PHI);
@@ -2264,12 +2275,12 @@ static void ctx_mkp(nse_ctx* x, const double* ut, const double* vt, const double
   const GridRcp* rg = (x->cfg.flags & NSE_FLAG_EXACT) ? nullptr : &x->rg;
   mark(x, PH_FFTX_F);
   if (rg && poisson3(x)) {
-    launch_div_src(d, *rg, ut, vt, wt, x->cfg.dt, phi, s);
+    launch_div_src(d, *rg, ut, vt, wt, x->cfg.dt, phi, false, s);
     ctx_poisson64(x, phi, true);
   } else if (rg) {
     autotune_mid(x);
     // phi is free until the inverse x pass: it holds the divergence samples
-    launch_div_src(d, *rg, ut, vt, wt, x->cfg.dt, phi, s);
+    launch_div_src(d, *rg, ut, vt, wt, x->cfg.dt, phi, out != END_FULL, s);
     launch_fft_fwd_x(pp, d, phi, nullptr, nullptr, nullptr, x->g, 1.0, 0, s);
   } else {
     launch_fft_fwd_x(pp, d, nullptr, ut, vt, wt, x->g, x->cfg.dt, 1, s, rg);
@@ -2287,6 +2298,13 @@ static void ctx_mkp(nse_ctx* x, const double* ut, const double* vt, const double
     }
     mark(x, PH_FFTX_I);
     launch_fft_inv_x(pp, d, phi, s);
+    if (out != END_FULL) {
+      const bool ta = out == END_TA;
+      launch_correct_step(d, x->rg, phi, ut, vt, wt, F(x, NSE_U), F(x, NSE_V), F(x, NSE_W),
+                          ta ? F(x, NSE_U_TA) : nullptr, ta ? F(x, NSE_V_TA) : nullptr,
+                          ta ? F(x, NSE_W_TA) : nullptr, x->cfg.dt, s);
+      return;
+    }
     mark(x, PH_PHIBC);
     launch_phibc(d, phi, s);
   }
@@ -2549,7 +2567,7 @@ static void autotune_rhs(nse_ctx* x, const StepParams& sp) {
 
 // one time step in the mixed-precision form: FP64 state u, v, w, T, p;
 // FP32 right-hand side, line sweeps and transforms
-static void ctx_step_f32(nse_ctx* x) {
+static void ctx_step_f32(nse_ctx* x, int in, int out) {
   const Dims& d = x->d;
   const nse_config& c = x->cfg;
   cudaStream_t s = x->stream;
@@ -2564,12 +2582,13 @@ static void ctx_step_f32(nse_ctx* x) {
   float *ua = x->ua.as<float>(), *va = x->va.as<float>(), *wa = x->wa.as<float>();
   float* uT = x->uT.as<float>();
   mark(x, PH_BC);
-  launch_set_bc(d, u, v, w, p, T, c.t_bot, c.t_top, 31, s);
+  if (in == END_FULL) launch_set_bc(d, u, v, w, p, T, c.t_bot, c.t_top, 31, s);
   mark(x, PH_RHS);
   autotune_rhs(x, sp);
   launch_rhs_f32(d, x->g, x->rg, sp, u, v, w, T, F32(x, NSE_U_TA), F32(x, NSE_V_TA),
                  F32(x, NSE_W_TA), F32(x, NSE_U_PRE), F32(x, NSE_V_PRE), F32(x, NSE_W_PRE),
-                 F32(x, NSE_T_PRE), c1, ua, va, wa, uT, x->math64, s, x->rhs_shape);
+                 F32(x, NSE_T_PRE), c1, ua, va, wa, uT, x->math64, s, x->rhs_shape,
+                 in == END_LEAN ? F(x, NSE_PHI) : nullptr);
   refresh_line_flags(x, s);
   autotune_lines(x);
   float* fa[3] = {ua, va, wa};
@@ -2609,8 +2628,9 @@ static void ctx_step_f32(nse_ctx* x) {
     for (int q = 0; q < 2; ++q) NSE_CUDA(cudaStreamWaitEvent(s, x->ljoin[q], 0));
     for (int ph = PH_ZVEL; ph <= PH_ZT; ++ph) mark(x, ph);
     mark(x, PH_BC2);
-    launch_set_bc_f32(d, ua, va, wa, p, T, c.t_bot, c.t_top, 1 | 2 | 4 | 8, s);
-    ctx_mkp_f32(x, ua, va, wa);
+    if (out == END_FULL)
+      launch_set_bc_f32(d, ua, va, wa, p, T, c.t_bot, c.t_top, 1 | 2 | 4 | 8, s);
+    ctx_mkp_f32(x, ua, va, wa, out);
     NSE_CUDA(cudaStreamWaitEvent(s, x->ljoin[2], 0));
     if (x->prof_n < x->prof_cap) x->prof_n++;
     x->l += 1;
@@ -2638,10 +2658,27 @@ static void ctx_step_f32(nse_ctx* x) {
   x->l += 1;
 }
 
-// one time step, nse_dominik.f:290-446
-static void ctx_step(nse_ctx* x) {
+// Whether a step may end lean (StepEnd): the concurrent fast forms with the
+// FP64 five-launch solve, once the first step has chosen the launch shapes
+static bool lean_ok(nse_ctx* x) {
+  return x->part && x->corr_tuned && concurrent(x) &&
+         !(x->cfg.flags & (NSE_FLAG_EXACT | NSE_FLAG_CHECK_FINITE)) &&
+         !(x->mixed && (x->cfg.flags & NSE_FLAG_POISSON32)) && !poisson3(x);
+}
+// How step n of a call of nsteps (1-based) ends: the last two write every
+// field (u_ep2 of the last reads p and u_ta of the one before it), the others
+// what the next step reads.  Measured at 256x192x256: 0.40 ms for the whole
+// correction with its faces and 0.06 for the four launches around it (PHIBC,
+// SET_BC before and after it), against 0.12 ms for k_correct_step.
+static int step_end(nse_ctx* x, int n, int nsteps) {
+  return n + 2 <= nsteps && lean_ok(x) ? END_LEAN : END_FULL;
+}
+
+// one time step, nse_dominik.f:290-446; in: how the step before it in the same
+// call ended (END_FULL for the first), out: how this one ends
+static void ctx_step(nse_ctx* x, int in = END_FULL, int out = END_FULL) {
   if (x->mixed) {
-    ctx_step_f32(x);
+    ctx_step_f32(x, in, out);
     return;
   }
   const Dims& d = x->d;
@@ -2660,7 +2697,7 @@ static void ctx_step(nse_ctx* x) {
   LineScratch sc{x->sa.as<double>(), x->sb.as<double>()};
   // :290 set_bc(u,v,w,p,T)
   mark(x, PH_BC);
-  launch_set_bc(d, u, v, w, p, T, c.t_bot, c.t_top, 31, s);
+  if (in == END_FULL) launch_set_bc(d, u, v, w, p, T, c.t_bot, c.t_top, 31, s);
   mark(x, PH_RHS);
   // :299-396 explicit terms, AB2, set_bc(u_a,...) and the penalised updates
   if (!(c.flags & NSE_FLAG_EXACT) && !x->rec) autotune_rhs(x, sp);
@@ -2671,7 +2708,8 @@ static void ctx_step(nse_ctx* x) {
   else
     launch_rhs_fast(d, x->g, x->rg, sp, u, v, w, T, F(x, NSE_U_TA), F(x, NSE_V_TA),
                     F(x, NSE_W_TA), F(x, NSE_U_PRE), F(x, NSE_V_PRE), F(x, NSE_W_PRE),
-                    F(x, NSE_T_PRE), c1, ua, va, wa, uT, s, x->rhs_shape);
+                    F(x, NSE_T_PRE), c1, ua, va, wa, uT, s, x->rhs_shape,
+                    in == END_LEAN ? F(x, NSE_PHI) : nullptr);
   // :397 solve_u_temp: per component y, z, x line solves
   // (timed per direction: all y solves, then z, then x of the three fields;
   // the fields are independent, so this order gives the same values as
@@ -2737,8 +2775,9 @@ static void ctx_step(nse_ctx* x) {
     for (int q = 0; q < 2; ++q) NSE_CUDA(cudaStreamWaitEvent(s, x->ljoin[q], 0));
     for (int ph = PH_ZVEL; ph <= PH_ZT; ++ph) mark(x, ph);
     mark(x, PH_BC2);
-    launch_set_bc(d, ua, va, wa, p, T, c.t_bot, c.t_top, 1 | 2 | 4 | 8, s);
-    ctx_mkp(x, ua, va, wa);
+    if (out == END_FULL)
+      launch_set_bc(d, ua, va, wa, p, T, c.t_bot, c.t_top, 1 | 2 | 4 | 8, s);
+    ctx_mkp(x, ua, va, wa, out);
     NSE_CUDA(cudaStreamWaitEvent(s, x->ljoin[2], 0));
     if (x->prof_n < x->prof_cap) x->prof_n++;
     x->l += 1;
@@ -2790,9 +2829,10 @@ bool ctx_info(nse_ctx* x, CtxInfo& out) {
 double* ctx_field(nse_ctx* x, int id) { return F(x, id); }
 int ctx_get_l(nse_ctx* x) { return x->l; }
 void ctx_set_l(nse_ctx* x, int l) { x->l = l; }
-void ctx_step_rec(nse_ctx* x, double* const* rec) {
+bool ctx_lean_ok(nse_ctx* x) { return lean_ok(x); }
+void ctx_step_rec(nse_ctx* x, double* const* rec, int in, int out) {
   x->rec = rec;
-  ctx_step(x);
+  ctx_step(x, in, out);
   x->rec = nullptr;
 }
 // the step's line solve of (dir, comp) applied to the field f with zero wall
@@ -2823,42 +2863,45 @@ extern "C" {
 
 // One step as a replay of a captured CUDA graph of one step.  The step's
 // launches depend on the host-side state only through the step counter
-// (l == 1 is the Euler start) and the temperature buffer pair (the FP64 form
-// swaps T and its work buffer every step), so from the third step on a step
-// is the replay of the graph captured from the same starting buffer.  The
-// first two steps, steps after the mask changed, profiled and recorded steps,
-// and steps on a stream that is being captured run eagerly (false).  The
+// (l == 1 is the Euler start), the way it starts and ends (in, out) and the
+// temperature buffer pair (the FP64 form swaps T and its work buffer every
+// step), so the second and later steps of one kind and starting buffer replay
+// its graph.  Step l = 1, the first of each kind and buffer, steps after the
+// mask changed, profiled and recorded steps, and steps on a stream that is
+// being captured run eagerly (false).  The
 // capture leaves the host-side state of the step behind (counter, buffer
 // pair) and is launched at once; a replay sets that state the same way.
 // Returns 1 (replayed), 0 (step eagerly) or -1 (a CUDA error).  A launch
 // shape, a masked line list's length or a table's place that differs from
 // the capture drops the graphs (a new mask is tabulated by an eager step).
-static int step_replay(nse_ctx* x) {
-  if (x->sg_off || x->l < 3 || x->mask_dirty || x->prof_n < x->prof_cap || x->rec) return 0;
+static int step_replay(nse_ctx* x, int in, int out) {
+  if (x->sg_off || x->mask_dirty || x->prof_n < x->prof_cap || x->rec) return 0;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(x->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
     return 0;
+  void* t0 = x->f[NSE_T].p;
+  const int kind = 2 * (in != END_FULL) + (out != END_FULL);
+  nse_ctx::StepGraph* g = nullptr;
+  for (auto& q : x->sg)
+    if (q.kind == kind && q.t == t0) g = &q;
+  for (auto& q : x->sg)
+    if (!g && q.kind < 0) g = &q;
+  if (!g) return 0;  // (four kinds and two buffers: never)
+  g->kind = kind;
+  g->t = t0;
+  if (++g->uses < 2 || x->l < 2) return 0;
   const unsigned long long sig = shape_sig(x);
   if (sig != x->sg_sig) {
     drop_step_graphs(x);
     x->sg_sig = sig;
   }
-  void* t0 = x->f[NSE_T].p;
-  int q = -1;
-  for (int k = 0; k < 2; ++k)
-    if (x->sg[k] && x->sg_t[k] == t0) q = k;
-  if (q >= 0) {
-    if (!NSE_CUDA(cudaGraphLaunch(x->sg[q], x->stream))) return -1;
-    count_launches(x->sg_nk[q]);
-    x->f[NSE_T] = x->sg_T[q];
-    x->uT = x->sg_uT[q];
+  if (g->ex) {
+    if (!NSE_CUDA(cudaGraphLaunch(g->ex, x->stream))) return -1;
+    count_launches(g->nk);
+    x->f[NSE_T] = g->T;
+    x->uT = g->uT;
     x->l += 1;
     return 1;
-  }
-  q = x->sg[0] ? 1 : 0;
-  if (x->sg[q]) {
-    cudaGraphExecDestroy(x->sg[q]);
-    x->sg[q] = nullptr;
   }
   const int l0 = x->l;
   const DBuf T0 = x->f[NSE_T], uT0 = x->uT;
@@ -2868,13 +2911,13 @@ static int step_replay(nse_ctx* x) {
     return 0;
   }
   const long long k0 = g_launches.load();
-  ctx_step(x);
+  ctx_step(x, in, out);
   const long long nk = g_launches.load() - k0;  // counted once: the launch below
-  cudaGraph_t g = nullptr;
-  const cudaError_t ce = cudaStreamEndCapture(x->stream, &g);
+  cudaGraph_t gr = nullptr;
+  const cudaError_t ce = cudaStreamEndCapture(x->stream, &gr);
   cudaGraphExec_t ex = nullptr;
-  const bool ok = ce == cudaSuccess && g && cudaGraphInstantiate(&ex, g, 0) == cudaSuccess;
-  if (g) cudaGraphDestroy(g);
+  const bool ok = ce == cudaSuccess && gr && cudaGraphInstantiate(&ex, gr, 0) == cudaSuccess;
+  if (gr) cudaGraphDestroy(gr);
   if (!ok) {
     // nothing ran: put the host-side state back and step eagerly
     cudaGetLastError();
@@ -2893,20 +2936,22 @@ static int step_replay(nse_ctx* x) {
     x->uT = uT0;
     return -1;
   }
-  x->sg[q] = ex;
-  x->sg_nk[q] = nk;
-  x->sg_t[q] = t0;
-  x->sg_T[q] = x->f[NSE_T];
-  x->sg_uT[q] = x->uT;
+  g->ex = ex;
+  g->nk = nk;
+  g->T = x->f[NSE_T];
+  g->uT = x->uT;
   return 1;
 }
 
 int nse_step(nse_ctx* x, int nsteps) {
   if (!x || nsteps < 0) return NSE_ERR_ARG;
-  for (int n = 0; n < nsteps; ++n) {
-    const int r = step_replay(x);
+  int in = END_FULL;
+  for (int n = 1; n <= nsteps; ++n) {
+    const int out = step_end(x, n, nsteps);
+    const int r = step_replay(x, in, out);
     if (r < 0) return status_or(NSE_ERR_CUDA);
-    if (r == 0) ctx_step(x);
+    if (r == 0) ctx_step(x, in, out);
+    in = out;
     if (!NSE_CUDA(cudaGetLastError())) return status_or(NSE_ERR_CUDA);
     if (x->cfg.flags & 1) {  // check for non-finite values after every step
       double m[6];
@@ -3154,13 +3199,15 @@ struct nse_ensemble {
   bool own_origin = true;
   cudaEvent_t fork = nullptr;
   std::vector<cudaEvent_t> join;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  // each case's temperature buffer when the graph was captured: the FP64
+  // by how the step before it ended and how its second step ends (the first
+  // of two steps of a call ends lean unless it is the last but one)
+  cudaGraphExec_t exec[2][2] = {};
+  long long nk[2][2] = {};  // kernels in each graph (counted once per replay)
+  int uses[2][2] = {};
+  // each case's temperature buffer when a graph was captured: the FP64
   // form swaps it with the work buffer every step, so a replay is valid only
   // after an even number of eager steps since the capture
   std::vector<void*> tbuf;
-  long long nk = 0;  // kernels in the graph (counted once per replay)
 };
 
 namespace nse {
@@ -3181,26 +3228,27 @@ static bool ens_fork_from_origin(nse_ensemble* e) {
   return true;
 }
 
-static bool ens_eager_step(nse_ensemble* e) {
+static bool ens_eager_step(nse_ensemble* e, int in, int out) {
   for (nse_ctx* x : e->cases) {
-    ctx_step(x);
+    ctx_step(x, in, out);
     if (!NSE_CUDA(cudaGetLastError())) return false;
   }
   return true;
 }
 
-static bool ens_capture(nse_ensemble* e) {
+static bool ens_capture(nse_ensemble* e, int in, int mid, int out) {
   std::vector<int> l0;
   for (nse_ctx* x : e->cases) l0.push_back(x->l);
-  e->tbuf.clear();
-  for (nse_ctx* x : e->cases) e->tbuf.push_back(x->f[NSE_T].p);
+  if (e->tbuf.empty())
+    for (nse_ctx* x : e->cases) e->tbuf.push_back(x->f[NSE_T].p);
+  long long& nk = e->nk[in != END_FULL][out != END_FULL];
   if (!NSE_CUDA(cudaStreamBeginCapture(e->origin, cudaStreamCaptureModeRelaxed))) return false;
   const long long k0 = g_launches.load();
   bool ok = ens_fork_from_origin(e);
   for (int st = 0; ok && st < 2; ++st)
-    for (nse_ctx* x : e->cases) ctx_step(x);
-  e->nk = g_launches.load() - k0;
-  count_launches(-e->nk);  // counted by each replay instead
+    for (nse_ctx* x : e->cases) ctx_step(x, st ? mid : in, st ? out : mid);
+  nk = g_launches.load() - k0;
+  count_launches(-nk);  // counted by each replay instead
   ok = ok && ens_join_into_origin(e);
   cudaGraph_t g = nullptr;
   cudaError_t ce = cudaStreamEndCapture(e->origin, &g);
@@ -3209,8 +3257,9 @@ static bool ens_capture(nse_ensemble* e) {
     if (g) cudaGraphDestroy(g);
     return false;
   }
-  e->graph = g;
-  return NSE_CUDA(cudaGraphInstantiate(&e->exec, g, 0));
+  ok = NSE_CUDA(cudaGraphInstantiate(&e->exec[in != END_FULL][out != END_FULL], g, 0));
+  cudaGraphDestroy(g);
+  return ok;
 }
 
 }  // namespace nse
@@ -3255,30 +3304,46 @@ int nse_ensemble_create(nse_ctx** cases, int n, int nstreams, nse_ensemble** out
 
 int nse_ensemble_step(nse_ensemble* e, int nsteps) {
   if (!e || nsteps < 0) return NSE_ERR_ARG;
-  bool ok = true;
+  bool ok = true, on_graph = false;
+  int in = END_FULL;
   while (ok && nsteps > 0) {
     // eager: the first step of a case, a mask being (re)tabulated, profiled
     // steps, a temperature buffer out of the captured parity, or one step left
-    bool eager = nsteps < 2;
-    for (nse_ctx* x : e->cases)
+    bool eager = nsteps < 2, lean = true;
+    for (nse_ctx* x : e->cases) {
       eager = eager || x->l <= 1 || x->mask_dirty || x->prof_n < x->prof_cap;
-    if (!eager && e->exec)
-      for (size_t i = 0; i < e->cases.size(); ++i)
-        eager = eager || e->cases[i]->f[NSE_T].p != e->tbuf[i];
+      lean = lean && lean_ok(x);
+    }
+    // how the next two steps end (every case the same way; step_end)
+    const int e1 = lean && nsteps > 2 ? END_LEAN : END_FULL;
+    const int e2 = lean && nsteps > 3 ? END_LEAN : END_FULL;
+    // three left: one eagerly, so that a pair ends the call
+    eager = eager || (lean && nsteps == 3);
+    for (size_t i = 0; i < e->tbuf.size(); ++i)
+      eager = eager || e->cases[i]->f[NSE_T].p != e->tbuf[i];
+    // the first and the last two steps of a call take a graph of their own
+    // from the second call on (its capture costs more than one eager step)
+    const int a = in != END_FULL, b = e2 != END_FULL;
+    eager = eager || (lean && a + b < 2 && ++e->uses[a][b] < 2);
     if (eager) {
-      ok = ens_eager_step(e);
+      if (on_graph) ok = ens_fork_from_origin(e);
+      on_graph = false;
+      ok = ok && ens_eager_step(e, in, e1);
+      in = e1;
       --nsteps;
       continue;
     }
-    if (!e->exec) ok = ens_capture(e);
-    ok = ok && ens_join_into_origin(e);
-    for (; ok && nsteps >= 2; nsteps -= 2) {
-      ok = NSE_CUDA(cudaGraphLaunch(e->exec, e->origin));
-      if (ok) count_launches(e->nk);
-      for (nse_ctx* x : e->cases) x->l += 2;
-    }
-    ok = ok && ens_fork_from_origin(e);
+    if (!on_graph) ok = ok && ens_join_into_origin(e);
+    on_graph = true;
+    cudaGraphExec_t& ex = e->exec[a][b];
+    if (!ex) ok = ok && ens_capture(e, in, e1, e2);
+    ok = ok && NSE_CUDA(cudaGraphLaunch(ex, e->origin));
+    if (ok) count_launches(e->nk[a][b]);
+    for (nse_ctx* x : e->cases) x->l += 2;
+    in = e2;
+    nsteps -= 2;
   }
+  if (on_graph) ok = ens_fork_from_origin(e) && ok;
   return ok ? NSE_OK : status_or(NSE_ERR_CUDA);
 }
 
@@ -3304,8 +3369,9 @@ int nse_ensemble_destroy(nse_ensemble* e) {
   for (cudaStream_t st : e->streams)
     if (st) cudaStreamSynchronize(st);
   for (size_t i = 0; i < e->cases.size(); ++i) e->cases[i]->stream = e->saved[i];
-  if (e->exec) cudaGraphExecDestroy(e->exec);
-  if (e->graph) cudaGraphDestroy(e->graph);
+  for (auto& row : e->exec)
+    for (cudaGraphExec_t ex : row)
+      if (ex) cudaGraphExecDestroy(ex);
   for (cudaEvent_t ev : e->join)
     if (ev) cudaEventDestroy(ev);
   if (e->fork) cudaEventDestroy(e->fork);
