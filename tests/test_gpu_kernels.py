@@ -3,6 +3,7 @@ the smallest and largest lengths of each launch shape."""
 import numpy as np
 import pytest
 
+from oracle import oracle as O
 from tests._helpers import rel_l2
 from tests.test_gpu_step import STATE, make_case, make_ctx, run_oracle
 from vtkmakecompare_b200 import solver as S
@@ -58,3 +59,28 @@ def test_steps_of_one_call_match_calls_of_one_step(prec, n):
     for other in out[1:]:
         for k in STATE:
             assert np.array_equal(out[0][k], other[k]), k
+
+
+# Level-set sweeps, bit for bit: a rough field (ridges, where both one-sided
+# slopes count), zeros (NaN in the reference) and ghosts of its own, on grids with
+# remainders of the 32 x 8 blocks; sweep counts below, at and past the replayed graph.
+# Values too large for reciprocal quotients and infinities take the dividing form.
+@pytest.mark.parametrize("n,nnn,big", [((36, 9, 5), 0, 0), ((30, 8, 3), 1, 0), ((64, 17, 6), 40, 0),
+                                       ((6, 5, 4), 128, 0), ((40, 12, 9), 129, 0),
+                                       ((32, 8, 4), 200, 0), ((90, 60, 75), 5, 0),
+                                       ((30, 8, 5), 30, 1e190), ((30, 8, 5), 3, np.inf),
+                                       ((30, 8, 5), 3, 1e-200)])
+def test_levelset_sweeps_match_oracle_bit_for_bit(n, nnn, big):
+    rng = np.random.default_rng(nnn + n[0])
+    g = O.Grid(*n, 2.0, 1.5, 1.0, y0=-0.5, gamma=1.3)
+    phi0 = np.asfortranarray(0.3 * rng.standard_normal([m + 2 for m in n]))
+    if nnn < 100:
+        phi0[3, 3, 2] = 0.0
+    if big:
+        phi0[5, 4, 3] = big
+        phi0[0, 2, 2] = -big
+    phi, _ = O.set_levelset(g, phi0, nnn=nnn, dtau=1.0e-3, width=1.5)
+    cfg = S.Config(*n, 1e-3, 100.0, 1.0, 1.0, 2.0, 1.5, 1.0, y0=-0.5, ystretch=1.3)
+    with S.Context(cfg) as ctx:
+        got = ctx.levelset(phi0, nnn=nnn, dtau=1.0e-3, width=1.5)
+    assert np.array_equal(got, phi, equal_nan=True)

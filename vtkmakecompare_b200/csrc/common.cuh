@@ -308,8 +308,11 @@ void launch_correct_step_f32(const Dims& d, const GridRcp& rg, const double* PHI
                              double dt, cudaStream_t s);
 
 // level set (set_levelset.f)
-void launch_levelset_iter(const Dims& d, const GridDev& g, const double* phi0,
-                          const double* phi, double* phi_new, double dtau, cudaStream_t s);
+void launch_levelset_sign(const Dims& d, const double* phi, double* sg, double dtau, int* big,
+                          cudaStream_t s);
+void launch_levelset_iter(const Dims& d, const GridDev& g, const GridRcp* rg, const double* sg,
+                          const double* phi, double* phi_new, double dtau, int* big,
+                          bool ghosts, bool chained, cudaStream_t s);
 void launch_levelset_bc(const Dims& d, double* phi, cudaStream_t s);
 void launch_levelset_mask(const Dims& d, const GridDev& g, const double* phi,
                           double* cellvalue1, double width, cudaStream_t s);

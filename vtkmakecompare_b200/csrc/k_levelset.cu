@@ -1,45 +1,124 @@
 // k_levelset.cu -- level-set reinitialisation and mask (set_levelset.f:1-199)
 // and the FP64 monitor reductions.  Built with --fmad=false: the update
 // phi - dt*S*G rounds like the reference.
+#include <cmath>
+
 #include "common.cuh"
 
 namespace nse {
 
 #define LD(p, i) __ldg((p) + (i))
 
-// one sweep of set_levelset.f:32-96 into phi_new (interior cells)
-__global__ void k_levelset_iter(Dims d, GridDev g, const double* __restrict__ phi0,
-                                const double* __restrict__ phi, double* __restrict__ out,
-                                double dtau) {
-  int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
-  int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
-  int k = 1 + blockIdx.z;
-  if (i > d.nx || j > d.ny) return;
+// sg = dtau S(phi) on the interior, S = phi / sqrt(phi^2 + epsilon^2) of the
+// input field: the factor of every sweep's update (set_levelset.f:80-96), NaN
+// where phi is 0.  Sets *big where a value, ghosts included, is kBig or more.
+constexpr double kBig = 0x1p600;
+__global__ void k_levelset_sign(Dims d, const double* __restrict__ phi, double* sg, double dtau,
+                                int* big) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int k = blockIdx.z;
+  if (i > d.nx + 1 || j > d.ny + 1) return;
   const double epsilon = 1.0 - 1;  // the reference's PARAMETER(epsilon=1.0d0-1)
-  long c = d.P(i, j, k);
-  double pc = LD(phi, c);
-  double a = (pc - LD(phi, c - 1)) / LD(g.dx12, i - 1);
-  double b = (LD(phi, c + 1) - pc) / LD(g.dx, i);
-  double cc = (pc - LD(phi, c - d.sx)) / LD(g.dy12, j - 1);
-  double dd = (LD(phi, c + d.sx) - pc) / LD(g.dy12, j);
-  double e = (pc - LD(phi, c - d.sy)) / LD(g.dz12, k - 1);
-  double f = (LD(phi, c + d.sy) - pc) / LD(g.dz12, k);
-  double ap = a >= 0.0 ? a : 0.0, am = a >= 0.0 ? 0.0 : a;
-  double bp = b >= 0.0 ? b : 0.0, bm = b >= 0.0 ? 0.0 : b;
-  double cp = cc >= 0.0 ? cc : 0.0, cm = cc >= 0.0 ? 0.0 : cc;
-  double dp = dd >= 0.0 ? dd : 0.0, dm = dd >= 0.0 ? 0.0 : dd;
-  double ep = e >= 0.0 ? e : 0.0, em = e >= 0.0 ? 0.0 : e;
-  double fp = f >= 0.0 ? f : 0.0, fm = f >= 0.0 ? 0.0 : f;
-  double p0 = LD(phi0, c);
-  double sss = p0 / sqrt(p0 * p0 + epsilon * epsilon);
-  double GGG;
-  if (p0 > 0.0)
-    GGG = sqrt(fmax(ap * ap, bm * bm) + fmax(cp * cp, dm * dm) + fmax(ep * ep, fm * fm)) - 1.0;
-  else if (p0 < 0.0)
-    GGG = sqrt(fmax(am * am, bp * bp) + fmax(cm * cm, dp * dp) + fmax(em * em, fp * fp)) - 1.0;
-  else
-    GGG = 0.0;
-  out[c] = pc - dtau * sss * GGG;
+  const long c = d.P(i, j, k);
+  const double p0 = phi[c];
+  if (fabs(p0) >= kBig) *big = 1;
+  if (i >= 1 && i <= d.nx && j >= 1 && j <= d.ny && k >= 1 && k <= d.nz)
+    sg[c] = dtau * (p0 / sqrt(p0 * p0 + epsilon * epsilon));
+}
+
+// n / d from the correctly rounded reciprocal r of d: of the two FMA residual
+// corrections the first leaves less than one unit in the last place and the
+// second rounds correctly (Markstein, IBM J. Res. Dev. 34 (1990) 111: division
+// from a correctly rounded reciprocal).  |n| < 2 kBig and d within 2^+-200, so
+// nothing overflows; an n so small that its residual is not exact gives a
+// quotient whose square is lost beside the 1 the slope is compared with.
+__device__ __forceinline__ double quotient(double n, double d, double r) {
+  double q = __dmul_rn(n, r);
+  q = __fma_rn(__fma_rn(-q, d, n), r, q);
+  return __fma_rn(__fma_rn(-q, d, n), r, q);
+}
+// max(lo, hi, 0), a NaN counting as 0
+__device__ __forceinline__ double upwind(double lo, double hi) {
+  const double q = lo > 0.0 ? lo : 0.0;
+  return hi > q ? hi : q;
+}
+
+// One sweep of set_levelset.f:32-96 into `out` (interior cells), sg =
+// dtau S(phi0).  The reference squares the one-sided differences that point
+// towards the interface and takes the larger square; here the differences are
+// signed towards it and the larger positive one is squared, the same value.
+// The ghosts hold the nearest interior value (:107-124), so they are not read: a
+// difference across the boundary is 0 (GHOSTS: the first sweep, which reads
+// those of the input).  Each thread marches kc cells in z; a z difference
+// quotient serves both of its cells (x and y ones are formed by each: the
+// reference divides the two x sides by different spacings, and a ridge of
+// phi, where both sides count, crosses half of all warps).  *big: a value of
+// phi is too large for `quotient` (a sweep that writes one sets it, the
+// sweeps after it divide); so do grids with spacings out of its range (!RCP).
+// Bound by instruction issue (FP64, selects), not by memory: the sign factored
+// out, five quotients for seven divisions and a square root, and no separate
+// ghost pass take a sweep of 256x192x256 from 218 to 101 us (46 us of HBM
+// traffic), of 128x96x128 from 30.6 to 13.6, of 64x48x64 from 11.1 to 3.7.
+// Small grids are bound by the launches: each sweep starts while the last one
+// drains (programmatic dependent launch).
+template <bool GHOSTS, bool RCP>
+__global__ void __launch_bounds__(256, 4) k_levelset_iter(Dims d, GridDev g, GridRcp rg, int kc,
+                                                          const double* __restrict__ sg,
+                                                          const double* phi, double* out,
+                                                          int flip, int* big) {
+  const int i = 1 + blockIdx.x * 32 + threadIdx.x, j = 1 + blockIdx.y * 8 + threadIdx.y;
+  const int k0 = 1 + blockIdx.z * kc, k1 = min(d.nz, k0 + kc - 1);
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (i > d.nx || j > d.ny) return;
+  const long c0 = d.P(i, j, k0);
+  const double dxm = LD(g.dx12, i - 1), dxp = LD(g.dx, i), dym = LD(g.dy12, j - 1),
+               dyp = LD(g.dy12, j);
+  double rxm = 0.0, rxp = 0.0, rym = 0.0, ryp = 0.0;
+  if (RCP) {
+    rxm = LD(rg.rdx12, i - 1);
+    rxp = LD(rg.rdx, i);
+    rym = LD(rg.rdy12, j - 1);
+    ryp = LD(rg.rdy12, j);
+  }
+  // neighbours: the cell itself in place of a ghost
+  const int xm = GHOSTS || i > 1 ? -1 : 0, xp = GHOSTS || i < d.nx ? 1 : 0;
+  const int ym = GHOSTS || j > 1 ? -(int)d.sx : 0, yp = GHOSTS || j < d.ny ? (int)d.sx : 0;
+  const double* sp = sg + c0;
+  const double* p = phi + c0;
+  double* o = out + c0;
+  // everything above is older than the previous sweep, phi is its result
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const bool div = !RCP || *(volatile int*)big;
+  double pc = p[0];
+  const double pz = p[GHOSTS || k0 > 1 ? -d.sy : 0];
+  auto march = [&](auto quot) {
+    double qz = quot(pc - pz, LD(g.dz12, k0 - 1), RCP ? LD(rg.rdz12, k0 - 1) : 0.0);
+    for (int k = k0; k <= k1; ++k) {
+      const double pn = p[GHOSTS || k < d.nz ? d.sy : 0], s = LD(sp, 0);
+      // the sign of phi0 (sg carries that of dtau too); where sg is NaN so
+      // is the result, whatever the slopes are
+      const int neg = (__double2hiint(s) ^ flip) & 0x80000000;
+      auto to = [&](double v, int w) {
+        return __hiloint2double(__double2hiint(v) ^ w, __double2loint(v));
+      };
+      const double x = upwind(to(quot(pc - p[xm], dxm, rxm), neg),
+                              to(quot(pc - p[xp], dxp, rxp), neg));
+      const double y = upwind(to(quot(pc - p[ym], dym, rym), neg),
+                              to(quot(pc - p[yp], dyp, ryp), neg));
+      const double qn = quot(pn - pc, LD(g.dz12, k), RCP ? LD(rg.rdz12, k) : 0.0);
+      const double z = upwind(to(qz, neg), to(qn, neg ^ 0x80000000));
+      const double v = pc - s * (sqrt(x * x + y * y + z * z) - 1.0);
+      *o = v;
+      if (fabs(v) >= kBig) *big = 1;
+      qz = qn;
+      pc = pn;
+      p += d.sy;
+      o += d.sy;
+      sp += d.sy;
+    }
+  };
+  if (div) march([](double n, double e, double) { return n / e; });
+  else march([](double n, double e, double r) { return quotient(n, e, r); });
 }
 
 // Neumann ghosts of set_levelset.f:107-124 (z, then y, then x passes): the
@@ -100,12 +179,39 @@ static void interior_grid(const Dims& d, dim3& grid, dim3& block) {
   grid = dim3((d.nx + 63) / 64, (d.ny + 3) / 4, d.nz);
 }
 
-void launch_levelset_iter(const Dims& d, const GridDev& g, const double* phi0,
-                          const double* phi, double* phi_new, double dtau, cudaStream_t s) {
-  dim3 grid, block;
-  interior_grid(d, grid, block);
+void launch_levelset_sign(const Dims& d, const double* phi, double* sg, double dtau, int* big,
+                          cudaStream_t s) {
+  dim3 block(32, 8), grid((d.nx + 33) / 32, (d.ny + 9) / 8, d.nz + 2);
   count_launch();
-  k_levelset_iter<<<grid, block, 0, s>>>(d, g, phi0, phi, phi_new, dtau);
+  k_levelset_sign<<<grid, block, 0, s>>>(d, phi, sg, dtau, big);
+}
+// chained: the launch before this one on the stream is another sweep; rg: the
+// reciprocal spacings, null where a spacing is out of the kernel's range
+void launch_levelset_iter(const Dims& d, const GridDev& g, const GridRcp* rg, const double* sg,
+                          const double* phi, double* phi_new, double dtau, int* big,
+                          bool ghosts, bool chained, cudaStream_t s) {
+  // cells a thread marches: the z quotient and the x and y spacings are shared
+  // by more of them, as long as the chip stays full (us a sweep with 1, 2, 4
+  // and 8: 64x48x64 3.7 3.9 4.7 8.2; 81x64x80 6.8 5.9 6.1 9.8; 128x96x128
+  // 18.2 14.8 13.6 14.2; 160x128x160 39.6 30.6 26.7 25.3)
+  const int kc = d.ncell < 300000 ? 1 : d.ncell < 600000 ? 2 : d.ncell < 2500000 ? 4 : 8;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((d.nx + 31) / 32, (d.ny + 7) / 8, (d.nz + kc - 1) / kc);
+  cfg.blockDim = dim3(32, 8);
+  cfg.stream = s;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = chained ? 1 : 0;
+  const int flip = std::signbit(dtau) ? (int)0x80000000 : 0;
+  const GridRcp r = rg ? *rg : GridRcp{};
+  count_launch();
+#define NSE_LS(G_, RCP_) \
+  cudaLaunchKernelEx(&cfg, k_levelset_iter<G_, RCP_>, d, g, r, kc, sg, phi, phi_new, flip, big)
+  if (!rg) { if (ghosts) NSE_LS(true, false); else NSE_LS(false, false); }
+  else { if (ghosts) NSE_LS(true, true); else NSE_LS(false, true); }
+#undef NSE_LS
 }
 void launch_levelset_bc(const Dims& d, double* phi, cudaStream_t s) {
   long n = 2L * (d.ny + 2) * (d.nz + 2) + 2L * d.nx * (d.nz + 2) + 2L * d.nx * d.ny;

@@ -1275,18 +1275,61 @@ static void write_vtk(const char* path, const char* scalars, int nx, int ny, int
   fclose(f);
 }
 
-static bool run_levelset(const Dims& d, const GridDev& g, const double* dphi0, double* dphi,
-                         double* dtmp, double* dcv1, int nnn, double dtau, double width,
-                         cudaStream_t s) {
+// whether the level-set kernel's quotients may use reciprocals of these spacings
+static bool levelset_range(const double* a, int n) {
+  for (int i = 0; i < n; ++i)
+    if (!(a[i] > 0x1p-200 && a[i] < 0x1p200)) return false;
+  return true;
+}
+
+// nnn + 1 sweeps of phi0 into dphi and the mask; phi0's buffer is overwritten.
+// All but the first sweep run as replays of a graph of LS_SWEEPS of them: one
+// host call per 2 us kernel would bound small grids.
+static bool run_levelset(const Dims& d, const GridDev& g, const GridRcp* rg, double* dphi0,
+                         double* dphi, double* dtmp, double* dcv1, int nnn, double dtau,
+                         double width, cudaStream_t s) {
+  constexpr int LS_SWEEPS = 64;  // even: a replay ends in the buffer it began in
   if (!NSE_CUDA(cudaMemcpyAsync(dphi, dphi0, d.ntot * sizeof(double), cudaMemcpyDeviceToDevice, s)))
     return false;
+  // phi0's buffer takes dtau S(phi0), its first (ghost) entry the flag
+  int* big = reinterpret_cast<int*>(dphi0);
+  if (!NSE_CUDA(cudaMemsetAsync(big, 0, sizeof(int), s))) return false;
+  launch_levelset_sign(d, dphi, dphi0, dtau, big, s);
   double* cur = dphi;
   double* nxt = dtmp;
-  for (int it = 0; it <= nnn; ++it) {
-    launch_levelset_iter(d, g, dphi0, cur, nxt, dtau, s);
-    launch_levelset_bc(d, nxt, s);
+  int left = nnn + 1;
+  auto sweep = [&](bool first) {
+    launch_levelset_iter(d, g, rg, dphi0, cur, nxt, dtau, big, first, !first, s);
     double* t = cur; cur = nxt; nxt = t;
+    --left;
+  };
+  sweep(true);
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (left >= 2 * LS_SWEEPS && cudaStreamIsCapturing(s, &cs) == cudaSuccess &&
+      cs == cudaStreamCaptureStatusNone &&
+      cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed) == cudaSuccess) {
+    bool ok = true;
+    const int n = left;
+    for (int q = 0; q < LS_SWEEPS; ++q) sweep(false);
+    left = n;
+    count_launches(-LS_SWEEPS);  // counted by each replay instead
+    cudaGraph_t gr = nullptr;
+    cudaGraphExec_t ex = nullptr;
+    if (cudaStreamEndCapture(s, &gr) == cudaSuccess && gr &&
+        cudaGraphInstantiate(&ex, gr, 0) == cudaSuccess)
+      for (; ok && left >= LS_SWEEPS; left -= LS_SWEEPS) {
+        ok = NSE_CUDA(cudaGraphLaunch(ex, s));
+        count_launches(LS_SWEEPS);
+      }
+    cudaGetLastError();
+    if (gr) cudaGraphDestroy(gr);
+    if (ex) cudaGraphExecDestroy(ex);  // (freed once its replays have run)
+    if (!ok) return false;
+  } else {
+    cudaGetLastError();
   }
+  while (left > 0) sweep(false);
+  launch_levelset_bc(d, cur, s);
   if (cur != dphi &&
       !NSE_CUDA(cudaMemcpyAsync(dphi, cur, d.ntot * sizeof(double), cudaMemcpyDeviceToDevice, s)))
     return false;
@@ -1311,7 +1354,23 @@ void set_levelset_(const int* nx, const int* ny, const int* nz, const double* dx
   double* d0 = st.up(phi0, d.ntot);
   double *dphi = st.alloc(d.ntot), *dtmp = st.alloc(d.ntot), *dcv = st.alloc(d.ncell);
   if (!st.ok) return;
-  if (!run_levelset(d, g, d0, dphi, dtmp, dcv, 2000, 1.0e-3, 1.0, st.s)) return;
+  GridRcp rg{};
+  const GridRcp* rgp = nullptr;
+  std::vector<double> rcp[4];
+  if (levelset_range(dx + 1, d.nx) && levelset_range(dx12, d.nx + 1) &&
+      levelset_range(dy12, d.ny + 1) && levelset_range(dz12, d.nz + 1)) {
+    const double* src[4] = {dx, dx12, dy12, dz12};
+    const int len[4] = {d.nx + 2, d.nx + 2, d.ny + 2, d.nz + 2};
+    const double* dev[4];
+    for (int q = 0; q < 4; ++q) {
+      for (int i = 0; i < len[q]; ++i) rcp[q].push_back(1.0 / src[q][i]);
+      dev[q] = st.up(rcp[q].data(), len[q]);
+    }
+    if (!st.ok) return;
+    rg.rdx = dev[0]; rg.rdx12 = dev[1]; rg.rdy12 = dev[2]; rg.rdz12 = dev[3];
+    rgp = &rg;
+  }
+  if (!run_levelset(d, g, rgp, d0, dphi, dtmp, dcv, 2000, 1.0e-3, 1.0, st.s)) return;
   st.down(phi, dphi, d.ntot);
   st.down(cellvalue, dcv, d.ncell);
   if (!st.finish()) return;
@@ -2977,7 +3036,11 @@ int nse_levelset(nse_ctx* x, const double* phi0, double* phi_out, int nnn, doubl
   if (!NSE_CUDA(cudaMemcpyAsync(x->tmp.p, phi0, d.ntot * sizeof(double), cudaMemcpyHostToDevice, s)))
     return status_or(NSE_ERR_CUDA);
   x->mask_dirty = true;
-  if (!run_levelset(d, x->g, x->tmp.as<double>(), F(x, NSE_PHI), x->ua.as<double>(),
+  const bool in_range = levelset_range(x->hdx.data() + 1, d.nx) &&
+                        levelset_range(x->hdx12.data(), d.nx + 1) &&
+                        levelset_range(x->hdy12.data(), d.ny + 1) &&
+                        levelset_range(x->hdz12.data(), d.nz + 1);
+  if (!run_levelset(d, x->g, in_range ? &x->rg : nullptr, x->tmp.as<double>(), F(x, NSE_PHI), x->ua.as<double>(),
                     F(x, NSE_CELLVALUE), nnn, dtau, width, s))
     return status_or(NSE_ERR_CUDA);
   // keep the level set: NSE_PHI is the Poisson work field of the steps
