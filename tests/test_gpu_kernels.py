@@ -4,8 +4,10 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
-from tests._helpers import rel_l2
+from tests import test_gpu_dropin as D
+from tests._helpers import bit_equal, rand_field, rel_l2
 from tests.test_gpu_step import STATE, make_case, make_ctx, run_oracle
+from vtkmakecompare_b200 import legacy as G
 from vtkmakecompare_b200 import solver as S
 
 pytestmark = pytest.mark.gpu
@@ -84,3 +86,42 @@ def test_levelset_sweeps_match_oracle_bit_for_bit(n, nnn, big):
     with S.Context(cfg) as ctx:
         got = ctx.levelset(phi0, nnn=nnn, dtau=1.0e-3, width=1.5)
     assert np.array_equal(got, phi, equal_nan=True)
+
+
+# Drop-in calls large enough for the pinned slots: rows that fill a slot with and
+# without a remainder, few long rows, many short ones.  SET_CONVECT and PHIBC round
+# like the oracle, so whole fields and boxes are compared bit for bit; MKP and SPN
+# for what they leave alone.
+@pytest.mark.parametrize("n", [(90, 61, 50), (500, 7, 12), (20, 80, 90), (64, 62, 64)])
+def test_drop_ins_through_pinned_slots(n):
+    nx, ny, nz = n
+    g, go = D.grid(*n)
+    rng = np.random.default_rng(nx)
+    ref = [rand_field(rng, *n) for _ in range(7)]
+    got = [v.copy(order="F") for v in ref]
+    O.set_convect(*ref[:6], 0.01, go)
+    G.set_convect(*got[:6], 0.01, nx, ny, nz, g["dx"], g["dy"], g["dz"], g["dx12"], g["dy12"],
+                  g["dz12"])
+    O.phibc(nx, ny, nz, ref[6])
+    G.phibc(nx, ny, nz, got[6])
+    for a, b in zip(ref, got):
+        assert bit_equal(a, b)
+    f = {k: rand_field(rng, *n) for k in ("p", "us", "vs", "ws", "u_ta", "v_ta", "w_ta", "u_ep2",
+                                          "v_ep2", "w_ep2", "divu", "u", "v", "w")}
+    old = {k: v.copy(order="F") for k, v in f.items()}
+    G.mkp(f["p"], f["us"], f["vs"], f["ws"], 0.013, g["dx"], g["dy"], g["dz"], g["dx12"],
+          g["dy12"], g["dz12"], 1.0, nx, ny, nz, 1, f["u_ta"], f["v_ta"], f["w_ta"], f["u_ep2"],
+          f["v_ep2"], f["w_ep2"], f["divu"], f["u"], f["v"], f["w"], g["xl"], g["zl"])
+    for k in f:
+        written = np.zeros([m + 2 for m in n], bool)
+        if k in ("u", "v", "w", "u_ta", "v_ta", "w_ta"):
+            written[:-1, :-1, :-1] = True
+        elif k not in ("us", "vs", "ws"):
+            written[1:-1, 1:-1, 1:-1] = True
+        assert bit_equal(f[k][~written], old[k][~written]), k
+        assert not np.any(f[k][written] == old[k][written]) or k == "v", k
+    Y = np.asfortranarray(rng.standard_normal((nx // 2 + 1, ny + 2, nz + 2)) + 0j)
+    Z = Y.copy(order="F")
+    G.spn(*n, *O.mkp_coeffs(go), Z)
+    assert bit_equal(Z[:, [0, ny + 1]], Y[:, [0, ny + 1]]) and bit_equal(Z[..., nz:], Y[..., nz:])
+    assert np.array_equal(Z[0, :, 0], Y[0, :, 0]) and not np.any(Z[1:, 1:-1, :nz] == Y[1:, 1:-1, :nz])

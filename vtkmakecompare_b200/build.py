@@ -31,6 +31,7 @@ SOURCES = {
     "k_poisson2d.cu": [],
     "noalloc.cu": [],
     "tma.cu": [],
+    "staging.cu": [],
     "fortran_io.cu": [],
     "k_adjoint.cu": ["--fmad=false"],
     "adjoint.cu": [],

@@ -79,13 +79,19 @@ bool ensure_device();
 // counts every kernel launch issued by the library (nse_launch_count)
 void count_launch();
 
-// host <-> device copies of a sub-box of a padded field (entries i0..i1,
-// j0..j1, k0..k1 inclusive), used so a legacy call writes back exactly the
-// entries the reference routine writes
-bool copy_box_d2h(double* host, const double* dev, const Dims& d, int i0, int i1, int j0,
-                  int j1, int k0, int k1, cudaStream_t s);
-bool copy_box_h2d(double* dev, const double* host, const Dims& d, int i0, int i1, int j0,
-                  int j1, int k0, int k1, cudaStream_t s);
+// A copy between a caller's host array and the GPU (staging.cu): `bytes`
+// contiguous bytes of rows of `pitch`; towards the host, of the rows whose index
+// modulo `per` lies in lo..hi, the `width` bytes from `off` are written, so a
+// legacy call writes back exactly the entries the reference routine writes.
+struct HostCopy {
+  void* host;
+  void* dev;
+  size_t bytes, pitch, off, width;
+  int per, lo, hi;
+};
+// the copies of a list, queued on s in any order; towards the host they are done
+// on return
+bool host_copies(const HostCopy* list, int n, bool to_device, cudaStream_t s);
 
 // ------------------------------------------ reference output files (host) --
 // fortran_io.cu: OUTPUT / OUTFIELD / READFIELD files of nse_dominik.f:2606-2794

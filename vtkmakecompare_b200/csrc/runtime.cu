@@ -178,36 +178,15 @@ cudaStream_t legacy_stream() {
   return s;
 }
 
-static bool copy_box(double* dst, const double* src, const Dims& d, int i0, int i1, int j0,
-                     int j1, int k0, int k1, cudaMemcpyKind kind, cudaStream_t s) {
-  if (i0 == 0 && j0 == 0 && k0 == 0 && i1 == d.nx + 1 && j1 == d.ny + 1 && k1 == d.nz + 1)
-    return NSE_CUDA(cudaMemcpyAsync(dst, src, d.ntot * sizeof(double), kind, s));
-  cudaMemcpy3DParms p;
-  memset(&p, 0, sizeof(p));
-  size_t pitch = (size_t)(d.nx + 2) * sizeof(double);
-  p.srcPtr = make_cudaPitchedPtr((void*)src, pitch, d.nx + 2, d.ny + 2);
-  p.dstPtr = make_cudaPitchedPtr((void*)dst, pitch, d.nx + 2, d.ny + 2);
-  p.srcPos = make_cudaPos((size_t)i0 * sizeof(double), j0, k0);
-  p.dstPos = p.srcPos;
-  p.extent = make_cudaExtent((size_t)(i1 - i0 + 1) * sizeof(double), j1 - j0 + 1, k1 - k0 + 1);
-  p.kind = kind;
-  return NSE_CUDA(cudaMemcpy3DAsync(&p, s));
-}
-bool copy_box_d2h(double* host, const double* dev, const Dims& d, int i0, int i1, int j0,
-                  int j1, int k0, int k1, cudaStream_t s) {
-  return copy_box(host, dev, d, i0, i1, j0, j1, k0, k1, cudaMemcpyDeviceToHost, s);
-}
-bool copy_box_h2d(double* dev, const double* host, const Dims& d, int i0, int i1, int j0,
-                  int j1, int k0, int k1, cudaStream_t s) {
-  return copy_box(dev, host, d, i0, i1, j0, j1, k0, k1, cudaMemcpyHostToDevice, s);
-}
-
 // -------------------------------------------------------- legacy helpers --
-// A legacy call stages its arrays in arena slots; `Stage` hands them out.
+// A legacy call stages its arrays in arena slots; `Stage` hands them out and
+// collects the copies: those to the GPU start at flush(), before the call's
+// first kernel, those back at finish().
 struct Stage {
   int next = 0;
   cudaStream_t s = legacy_stream();
   bool ok = true;
+  std::vector<HostCopy> in, out;
   double* alloc(size_t n) {
     if (!ok) return nullptr;
     DBuf& b = arena(next++);
@@ -216,19 +195,42 @@ struct Stage {
   }
   double* up(const double* h, size_t n) {
     double* d = alloc(n);
-    if (d && !NSE_CUDA(cudaMemcpyAsync(d, h, n * sizeof(double), cudaMemcpyHostToDevice, s)))
-      ok = false;
-    return ok ? d : nullptr;
+    if (d) in.push_back(whole(const_cast<double*>(h), d, n));
+    return d;
+  }
+  bool flush() {
+    ok = ok && (in.empty() || host_copies(in.data(), (int)in.size(), true, s));
+    in.clear();
+    return ok;
   }
   bool down(double* h, const double* d, size_t n) {
-    if (!ok) return false;
-    if (!NSE_CUDA(cudaMemcpyAsync(h, d, n * sizeof(double), cudaMemcpyDeviceToHost, s)))
-      ok = false;
+    if (ok) out.push_back(whole(h, const_cast<double*>(d), n));
     return ok;
+  }
+  // entries i0..i1, j0..j1, k0..k1 of a padded field
+  bool down_box(double* h, const double* dv, const Dims& d, int i0, int i1, int j0, int j1, int k0,
+                int k1) {
+    const size_t w = sizeof(double), pitch = (size_t)d.sx * w, o = (size_t)k0 * d.sy;
+    if (ok)
+      out.push_back({h + o, const_cast<double*>(dv) + o, (size_t)(k1 - k0 + 1) * d.sy * w, pitch,
+                     (size_t)i0 * w, (size_t)(i1 - i0 + 1) * w, (int)(d.ny + 2), j0, j1});
+    return ok;
+  }
+  // planes J = 1..NY, K = 0..NZ-1 of a spectrum PHIT(0:NX/2, 0:NY+1, 0:NZ+1)
+  bool down_spec(double* h, const double* dv, int H, int ny, int nz) {
+    const size_t row = (size_t)H * 2 * sizeof(double);
+    if (ok)
+      out.push_back({h, const_cast<double*>(dv), row * (ny + 2) * nz, row, 0, row, ny + 2, 1, ny});
+    return ok;
+  }
+  static HostCopy whole(double* h, double* d, size_t n) {
+    const size_t b = n * sizeof(double);
+    return {h, d, b, b, 0, b, 1, 0, 0};
   }
   bool finish() {
     if (!ok) return false;
     if (!NSE_CUDA(cudaGetLastError())) return false;
+    if (!out.empty() && !host_copies(out.data(), (int)out.size(), false, s)) return ok = false;
     return NSE_CUDA(cudaStreamSynchronize(s));
   }
 };
@@ -266,7 +268,7 @@ void tridiag_(double* A, double* B, const int* NN) {
   Stage st;
   double* dA = st.up(A, 3 * (size_t)n);
   double* dB = st.up(B, n);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   launch_tridiag(dA, dB, n, 1, st.s);
   st.down(A, dA, 3 * (size_t)n);
   st.down(B, dB, n);
@@ -280,7 +282,7 @@ void ctridiag_(double* A, double* B, const int* NN) {
   Stage st;
   double* dA = st.up(A, 3 * (size_t)n);
   double* dB = st.up(B, 2 * (size_t)n);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   launch_tridiag(dA, dB, n, 2, st.s);
   st.down(A, dA, 3 * (size_t)n);
   st.down(B, dB, 2 * (size_t)n);
@@ -295,7 +297,7 @@ void trid2_(double* A, double* B, const int* M, const int* N) {
   double* dA = st.up(A, 3 * (size_t)n);
   double* dAm = st.up(A, 3 * (size_t)n);
   double* dB = st.up(B, (size_t)m * n);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   launch_trid2(dA, dAm, dB, m, n, st.s);
   st.down(A, dAm, 3 * (size_t)n);
   st.down(B, dB, (size_t)m * n);
@@ -312,7 +314,7 @@ void tdma_(const double* a, const double* b, const double* c, const double* r, d
   Stage st;
   double *da = st.up(a, L), *db = st.up(b, L), *dc = st.up(c, L), *dr = st.up(r, L);
   double *du = st.alloc(L), *dg = st.alloc(L);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   launch_tdma(da, db, dc, dr, du, dg, m, st.s);
   st.down(u, du, L);
   st.finish();
@@ -327,7 +329,7 @@ void cyclic_(const double* a, const double* b, const double* c, const double* al
   Stage st;
   double *da = st.up(a, L), *db = st.up(b, L), *dc = st.up(c, L), *dr = st.up(r, L);
   double *dx = st.alloc(L), *dbb = st.alloc(L), *dg = st.alloc(L), *dz = st.alloc(L);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   launch_cyclic_general(da, db, dc, *alpha, *beta, dr, dx, dbb, dg, dz, m, st.s);
   st.down(x, dx, L);
   st.finish();
@@ -346,7 +348,7 @@ void implicit_solver_(double* SUX, const int* nx, const double* dx, const double
   double* f = st.up(SUX, L);
   double *ddx = st.up(dx, L), *ddx12 = st.up(dx12, L), *dcu = st.up(CUX, n);
   double *g1 = st.alloc(L), *g2 = st.alloc(L);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   GridDev g{ddx, ddx, ddx, ddx12, ddx12, ddx12};
   launch_single_cyc(f, g1, g2, 0, n, g, *Re, 1.0, *dt, *eta, *ft, *fb, dcu, nullptr, nullptr,
                     st.s);
@@ -366,7 +368,7 @@ void implicit_uy_(double* SUY, const int* ny, const double* dy, const double* dy
   double* f = st.up(SUY, L);
   double *ddy = st.up(dy, L), *ddy12 = st.up(dy12, L), *dcu = st.up(CUY, n);
   double* lsc = st.alloc(L);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   GridDev g{ddy, ddy, ddy, ddy12, ddy12, ddy12};
   launch_single_ul(f, lsc, 0, n, g, *Re, 1.0, *dt, *eta, *ft, *fb, dcu, nullptr, nullptr,
                    st.s);
@@ -386,7 +388,7 @@ void implicit_vy_(double* SVY, const int* ny, const double* dy, const double* dy
   double* f = st.up(SVY, L);
   double *ddy = st.up(dy, L), *ddy12 = st.up(dy12, L), *dcu = st.up(CVY, n);
   double* lsc = st.alloc(L);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   GridDev g{ddy, ddy, ddy, ddy12, ddy12, ddy12};
   launch_single_ul(f, lsc, 1, n, g, *Re, 1.0, *dt, *eta, *ft, *fb, dcu, nullptr, nullptr,
                    st.s);
@@ -408,7 +410,7 @@ void implicit_ty_(double* STY, const int* ny, const double* dy, const double* dy
   double *ddy = st.up(dy, L), *ddy12 = st.up(dy12, L);
   double *dcu = st.up(CUY, L), *dll = st.up(lly, L), *drr = st.up(rry, L);
   double* lsc = st.alloc(L);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   GridDev g{ddy, ddy, ddy, ddy12, ddy12, ddy12};
   launch_single_ul(f, lsc, 2, n, g, *Re, *Sc, *dt, *eta, *ft, *fb, dcu, dll, drr, st.s);
   st.down(STY + 1, f + 1, n);
@@ -429,7 +431,7 @@ void implicit_tx_(double* STX, const int* nx, const double* dx, const double* dx
   double *ddx = st.up(dx, L), *ddx12 = st.up(dx12, L);
   double *dcu = st.up(CUX, L), *dll = st.up(llx, L), *drr = st.up(rrx, L);
   double *g1 = st.alloc(L), *g2 = st.alloc(L);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   GridDev g{ddx, ddx, ddx, ddx12, ddx12, ddx12};
   launch_single_cyc(f, g1, g2, 1, n, g, *Re, *Sc, *dt, *eta, *ft, *fb, dcu, dll, drr, st.s);
   st.down(STX, f, L);
@@ -698,7 +700,7 @@ void set_bc_(double* u, double* v, double* w, double* p, const int* nx, const in
   Stage st;
   double *du = st.up(u, d.ntot), *dv = st.up(v, d.ntot), *dw = st.up(w, d.ntot);
   double *dp = st.up(p, d.ntot), *dT = st.up(T, d.ntot);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   launch_set_bc(d, du, dv, dw, dp, dT, 0.0, 0.0, 31, st.s);
   st.down(u, du, d.ntot); st.down(v, dv, d.ntot); st.down(w, dw, d.ntot);
   st.down(p, dp, d.ntot); st.down(T, dT, d.ntot);
@@ -707,8 +709,7 @@ void set_bc_(double* u, double* v, double* w, double* p, const int* nx, const in
 
 static bool down_interior(Stage& st, double* h, const double* dv, const Dims& d) {
   if (!st.ok) return false;
-  if (!copy_box_d2h(h, dv, d, 1, d.nx, 1, d.ny, 1, d.nz, st.s)) st.ok = false;
-  return st.ok;
+  return st.down_box(h, dv, d, 1, d.nx, 1, d.ny, 1, d.nz);
 }
 
 void set_convect_(double* u, double* u_v, double* v, double* v_v, double* w, double* w_v,
@@ -722,7 +723,7 @@ void set_convect_(double* u, double* u_v, double* v, double* v_v, double* w, dou
   if (!stage_grid(st, d.nx, d.ny, d.nz, dx, dy, dz, dx12, dy12, dz12, g)) return;
   double *du = st.up(u, d.ntot), *dv = st.up(v, d.ntot), *dw = st.up(w, d.ntot);
   double *duv = st.alloc(d.ntot), *dvv = st.alloc(d.ntot), *dwv = st.alloc(d.ntot);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   launch_convect(d, g, du, dv, dw, duv, dvv, dwv, *dt, 1.0, st.s);
   down_interior(st, u_v, duv, d);
   down_interior(st, v_v, dvv, d);
@@ -742,7 +743,7 @@ void set_convection_for_scalar_(double* u, double* v, double* w, const double* d
   if (!stage_grid(st, d.nx, d.ny, d.nz, dx, dy, dz, dx12, dy12, dz12, g)) return;
   double *du = st.up(u, d.ntot), *dv = st.up(v, d.ntot), *dw = st.up(w, d.ntot);
   double *dT = st.up(T, d.ntot), *dr = st.up(rhoCp, d.ntot), *dout = st.alloc(d.ntot);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   launch_convect_scalar(d, g, du, dv, dw, dT, dr, dout, *dt, 1.0, st.s);
   down_interior(st, u_vT, dout, d);
   st.finish();
@@ -759,7 +760,7 @@ void set_conduction_(double* u, double* u_d, double* v, double* v_d, double* w, 
   if (!stage_grid(st, d.nx, d.ny, d.nz, dx, dy, dz, dx12, dy12, dz12, g)) return;
   double *du = st.up(u, d.ntot), *dv = st.up(v, d.ntot), *dw = st.up(w, d.ntot);
   double *a = st.alloc(d.ntot), *b = st.alloc(d.ntot), *c = st.alloc(d.ntot);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   launch_conduction(d, g, du, dv, dw, a, b, c, *Re, *dt, st.s);
   down_interior(st, u_d, a, d);
   down_interior(st, v_d, b, d);
@@ -779,7 +780,7 @@ void set_diffusion_for_scalar_(const double* Re, const double* dt, const int* nx
   if (!stage_grid(st, d.nx, d.ny, d.nz, dx, dy, dz, dx12, dy12, dz12, g)) return;
   double *dT = st.up(T, d.ntot), *dl = st.up(thc, d.ntot), *dr = st.up(rhoCp, d.ntot);
   double* dout = st.alloc(d.ntot);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   launch_diffusion_scalar(d, g, dT, dl, dr, dout, *Re, *Sc, *dt, st.s);
   down_interior(st, u_dT, dout, d);
   st.finish();
@@ -801,7 +802,7 @@ void set_adj_convect_(double* u, double* u_v, double* v, double* v_v, double* w,
   double *duf = st.up(u_final, d.ntot), *dvf = st.up(v_final, d.ntot);
   double* dwf = st.up(w_final, d.ntot);
   double *duv = st.alloc(d.ntot), *dvv = st.alloc(d.ntot), *dwv = st.alloc(d.ntot);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   launch_set_adj_convect(d, adj_grid(g), du, dv, dw, duf, dvf, dwf, duv, dvv, dwv, *dt, st.s);
   down_interior(st, u_v, duv, d);
   down_interior(st, v_v, dvv, d);
@@ -825,7 +826,7 @@ void set_adj_convection_for_scalar_(double* u, double* v, double* w, const doubl
   double *dT = st.up(T, d.ntot), *dr = st.up(rhoCp, d.ntot);
   double *duf = st.up(u_final, d.ntot), *dvf = st.up(v_final, d.ntot);
   double *dwf = st.up(w_final, d.ntot), *dout = st.alloc(d.ntot);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   launch_set_adj_cscalar(d, adj_grid(g), dT, dr, duf, dvf, dwf, dout, *dt, st.s);
   down_interior(st, u_vT, dout, d);
   st.finish();
@@ -845,7 +846,7 @@ static void adj_ns_scalar(const double* dt, int nx, int ny, int nz, const double
   if (dTf && !Tf && !NSE_CUDA(cudaMemsetAsync(dTf, 0, d.ntot * sizeof(double), st.s)))
     st.ok = false;
   double *dus = st.alloc(d.ntot), *dvs = st.alloc(d.ntot), *dws = st.alloc(d.ntot);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   launch_set_adj_ns_scalar(d, adj_grid(g), dT, dTf, dus, dvs, dws, *dt, st.s);
   down_interior(st, u_s, dus, d);
   down_interior(st, v_s, dvs, d);
@@ -886,7 +887,7 @@ void set_immersed_boundary_(const double* eta, const int* nx, const int* ny, con
   double *a = st.up(u_ta, d.ntot), *b = st.up(v_ta, d.ntot), *c = st.up(w_ta, d.ntot);
   double *ul = st.alloc(d.ntot), *vl = st.alloc(d.ntot), *wl = st.alloc(d.ntot);
   double* tl = st.alloc(d.ntot);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   if (*l == 1) {
     launch_build_face_masks(d, dcv, st.s);
     st.down(cellvalue + d.ncell, dcv + d.ncell, 3 * (size_t)d.ncell);
@@ -912,7 +913,7 @@ void set_explicit_(double* u_v, double* u_pre, double* u_d, double* u_a, double*
   double *vv = st.up(v_v, n), *vp = st.up(v_pre, n), *vd = st.up(v_d, n), *va = st.up(v_a, n);
   double *wv = st.up(w_v, n), *wp = st.up(w_pre, n), *wd = st.up(w_d, n), *wa = st.up(w_a, n);
   double *ul = st.up(u_l, n), *vl = st.up(v_l, n), *wl = st.up(w_l, n);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   launch_explicit(d, uv, up, ud, ua, vv, vp, vd, va, wv, wp, wd, wa, ul, vl, wl, *l, st.s);
   st.down(u_a, ua, n); st.down(v_a, va, n); st.down(w_a, wa, n);
   down_interior(st, u_pre, up, d);
@@ -930,7 +931,7 @@ void set_explicit_for_tempreture_(double* u_vT, double* u_dT, double* u_T, doubl
   size_t n = d.ntot;
   double *vt = st.up(u_vT, n), *dtt = st.up(u_dT, n), *ut = st.up(u_T, n);
   double *tp = st.up(T_pre, n), *tl = st.up(T_l, n);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   launch_explicit_T(d, vt, dtt, ut, tp, tl, *l, st.s);
   st.down(u_T, ut, n);
   down_interior(st, T_pre, tp, d);
@@ -953,7 +954,7 @@ void solve_u_temp_(double* u_a, double* v_a, double* w_a, const int* nx, const i
   double *du = st.up(u, n), *dv = st.up(v, n), *dw = st.up(w, n);
   double* dcv = st.up(cellvalue, 4 * (size_t)d.ncell);
   LineScratch sc{st.alloc(n), st.alloc(n)};
-  if (!st.ok) return;
+  if (!st.flush()) return;
   double* fa[3] = {ua, va, wa};
   double* fo[3] = {du, dv, dw};
   for (int comp = 0; comp < 3; ++comp) {
@@ -980,7 +981,7 @@ void solve_t_(double* u_T, const int* nx, const int* ny, const int* nz, const do
   double *ut = st.up(u_T, n), *dr = st.up(rhoCp, n), *dl = st.up(thc, n);
   double* dcv = st.up(cellvalue, d.ncell);
   LineScratch sc{st.alloc(n), st.alloc(n)};
-  if (!st.ok) return;
+  if (!st.flush()) return;
   launch_ysolve_T(d, g, ut, dcv, dr, dl, 1.0, 1.0, *Re, *Sc, *dt, *eta, 0.0, 0.0, sc, st.s);
   launch_xsolve_T(d, g, ut, dcv, dr, dl, 1.0, 1.0, *Re, *Sc, *dt, *eta, sc, st.s);
   launch_zsolve_T(d, g, ut, dcv, dr, dl, 1.0, 1.0, *Re, *Sc, *dt, *eta, sc, st.s);
@@ -1094,15 +1095,13 @@ void p2s_(double* FP, double* FPT, const int* NX, const int* NY, const int* NZ) 
   int H = nx / 2 + 1;
   size_t nphit = 2 * (size_t)H * (ny + 2) * (nz + 2);
   double* dphit = st.alloc(nphit);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   GridDev g{};
   launch_fft_fwd_x(pb.pp, d, dfp, nullptr, nullptr, nullptr, g, 1.0, 0, st.s);
   launch_fft_z(pb.pp, false, st.s);
   launch_spec_to_phit(pb.pp, dphit, st.s);
   // written entries: J = 1..NY, K = 0..NZ-1, all kx
-  size_t row = (size_t)H * 2 * sizeof(double);
-  NSE_CUDA(cudaMemcpy2DAsync(FPT + 2 * (size_t)H, row * (ny + 2), dphit + 2 * (size_t)H,
-                             row * (ny + 2), row * ny, nz, cudaMemcpyDeviceToHost, st.s));
+  st.down_spec(FPT, dphit, H, ny, nz);
   st.finish();
 }
 
@@ -1119,12 +1118,12 @@ void s2p_(double* FPT, double* FP, const int* NX, const int* NY, const int* NZ) 
   size_t nphit = 2 * (size_t)H * (ny + 2) * (nz + 2);
   double* dphit = st.up(FPT, nphit);
   double* dfp = st.alloc(d.ntot);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   launch_phit_to_spec(pb.pp, dphit, st.s);
   launch_fft_z(pb.pp, true, st.s);
   launch_fft_inv_x(pb.pp, d, dfp, st.s);
   // written entries: FP(0:NX, J, 0:NZ) for J = 1..NY
-  copy_box_d2h(FP, dfp, d, 0, nx, 1, ny, 0, nz, st.s);
+  st.down_box(FP, dfp, d, 0, nx, 1, ny, 0, nz);
   st.finish();
 }
 
@@ -1142,16 +1141,14 @@ void spn_(const int* NX, const int* NY, const int* NZ, const double* AC, const d
   double* dK = st.up(KXZ, (size_t)H * (nz + 1));
   double* spec = st.alloc(2 * (size_t)Hp * ny * nz);
   double* scr = st.alloc((size_t)Hp * ny * nz);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   PoissonPlan pp{};
   pp.nx = nx; pp.ny = ny; pp.nz = nz; pp.H = H; pp.Hp = Hp;
   pp.spec = spec; pp.scr = scr; pp.AC = dAC; pp.KXZ = dK;
   launch_phit_to_spec(pp, dphit, st.s);
   launch_spn(pp, true, false, st.s);
   launch_spec_to_phit(pp, dphit, st.s);
-  size_t row = (size_t)H * 2 * sizeof(double);
-  NSE_CUDA(cudaMemcpy2DAsync(PHIT + 2 * (size_t)H, row * (ny + 2), dphit + 2 * (size_t)H,
-                             row * (ny + 2), row * ny, nz, cudaMemcpyDeviceToHost, st.s));
+  st.down_spec(PHIT, dphit, H, ny, nz);
   st.finish();
 }
 
@@ -1163,7 +1160,7 @@ void sp0b_(const int* NX, const int* NY, const int* NZ, const double* AC, double
   // the column PHIT(0, 0:NY+1, 0) (stride H complex)
   double* col = st.alloc(2 * (size_t)H * (ny + 2));
   double* dAC = st.up(AC, 3 * (size_t)ny);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   size_t row = (size_t)H * 2 * sizeof(double);
   NSE_CUDA(cudaMemcpy2DAsync(col, row, PHIT, row, 2 * sizeof(double), ny + 2,
                              cudaMemcpyHostToDevice, st.s));
@@ -1179,7 +1176,7 @@ void phibc_(const int* NX, const int* NY, const int* NZ, double* PHI) {
   Dims d = make_dims(*NX, *NY, *NZ);
   Stage st;
   double* dphi = st.up(PHI, d.ntot);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   launch_phibc(d, dphi, st.s);
   st.down(PHI, dphi, d.ntot);
   st.finish();
@@ -1206,7 +1203,7 @@ void mkp_(double* p, double* u_temp, double* v_temp, double* w_temp, const doubl
   double *du = st.alloc(n), *dv = st.alloc(n), *dw = st.alloc(n);
   double *e1 = st.alloc(n), *e2 = st.alloc(n), *e3 = st.alloc(n), *dd = st.alloc(n);
   double* phi = st.alloc(n);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   NSE_CUDA(cudaMemsetAsync(phi, 0, n * sizeof(double), st.s));
   launch_fft_fwd_x(pb.pp, d, nullptr, ut, vt, wt, g, *dt, 1, st.s);
   launch_fft_z(pb.pp, false, st.s);
@@ -1216,12 +1213,12 @@ void mkp_(double* p, double* u_temp, double* v_temp, double* w_temp, const doubl
   launch_phibc(d, phi, st.s);
   launch_correct(d, g, phi, ut, vt, wt, dp, du, dv, dw, a, b, c, e1, e2, e3, dd, *dt, st.s);
   int X = d.nx, Y = d.ny, Z = d.nz;
-  copy_box_d2h(u, du, d, 0, X, 0, Y, 0, Z, st.s);
-  copy_box_d2h(v, dv, d, 0, X, 0, Y, 0, Z, st.s);
-  copy_box_d2h(w, dw, d, 0, X, 0, Y, 0, Z, st.s);
-  copy_box_d2h(u_ta, a, d, 0, X, 0, Y, 0, Z, st.s);
-  copy_box_d2h(v_ta, b, d, 0, X, 0, Y, 0, Z, st.s);
-  copy_box_d2h(w_ta, c, d, 0, X, 0, Y, 0, Z, st.s);
+  st.down_box(u, du, d, 0, X, 0, Y, 0, Z);
+  st.down_box(v, dv, d, 0, X, 0, Y, 0, Z);
+  st.down_box(w, dw, d, 0, X, 0, Y, 0, Z);
+  st.down_box(u_ta, a, d, 0, X, 0, Y, 0, Z);
+  st.down_box(v_ta, b, d, 0, X, 0, Y, 0, Z);
+  st.down_box(w_ta, c, d, 0, X, 0, Y, 0, Z);
   down_interior(st, p, dp, d);
   down_interior(st, u_ep2, e1, d);
   down_interior(st, v_ep2, e2, d);
@@ -1353,7 +1350,7 @@ void set_levelset_(const int* nx, const int* ny, const int* nz, const double* dx
   g.dz = g.dz12;
   double* d0 = st.up(phi0, d.ntot);
   double *dphi = st.alloc(d.ntot), *dtmp = st.alloc(d.ntot), *dcv = st.alloc(d.ncell);
-  if (!st.ok) return;
+  if (!st.flush()) return;
   GridRcp rg{};
   const GridRcp* rgp = nullptr;
   std::vector<double> rcp[4];
@@ -1366,7 +1363,7 @@ void set_levelset_(const int* nx, const int* ny, const int* nz, const double* dx
       for (int i = 0; i < len[q]; ++i) rcp[q].push_back(1.0 / src[q][i]);
       dev[q] = st.up(rcp[q].data(), len[q]);
     }
-    if (!st.ok) return;
+    if (!st.flush()) return;
     rg.rdx = dev[0]; rg.rdx12 = dev[1]; rg.rdy12 = dev[2]; rg.rdz12 = dev[3];
     rgp = &rg;
   }
