@@ -125,3 +125,37 @@ def test_drop_ins_through_pinned_slots(n):
     G.spn(*n, *O.mkp_coeffs(go), Z)
     assert bit_equal(Z[:, [0, ny + 1]], Y[:, [0, ny + 1]]) and bit_equal(Z[..., nz:], Y[..., nz:])
     assert np.array_equal(Z[0, :, 0], Y[0, :, 0]) and not np.any(Z[1:, 1:-1, :nz] == Y[1:, 1:-1, :nz])
+
+
+# SPN by pipelined columns: one row, chunks of 16 rows with and without a
+# remainder, the lengths where 32, 16 and 8 systems share a CTA and past them, and
+# numbers of systems that leave lanes empty.  Same bits as the same systems
+# solved one thread each (an off-boundary array), 1e-13 to the oracle as test_zz_no_alloc.
+@pytest.mark.parametrize("n", [(4, 1, 5), (6, 2, 3), (10, 16, 9), (30, 17, 8), (64, 33, 12),
+                               (16, 109, 6), (16, 110, 6), (12, 212, 5), (12, 213, 5),
+                               (8, 800, 4), (8, 900, 3)])
+def test_spn_columns_match_oracle(n):
+    import ctypes as C
+
+    import torch
+    nx, ny, nz = n
+    AC, KXZ = O.mkp_coeffs(O.Grid(nx, ny, nz, 6.0, 2.0, 3.0, y0=-1.0, gamma=1.5))
+    rng = np.random.default_rng(ny)
+    Y = np.asfortranarray(rng.standard_normal((nx // 2 + 1, ny + 2, nz + 2)) +
+                          1j * rng.standard_normal((nx // 2 + 1, ny + 2, nz + 2)))
+    ref = Y.copy(order="F")
+    O.spn(nx, ny, nz, AC, KXZ, ref)
+    f = G.lib().nse_spn_noalloc
+    f.argtypes = [C.c_int] * 3 + [C.c_void_p] * 4
+    dev = [torch.from_numpy(a.ravel(order="F")).cuda() for a in (AC, KXZ)]
+    got = []
+    for off in (0, 1):
+        raw = torch.zeros(2 * Y.size + 1, dtype=torch.float64, device="cuda")
+        d = raw[off:off + 2 * Y.size]
+        d.copy_(torch.from_numpy(Y.ravel(order="F").view(np.float64)))
+        assert f(nx, ny, nz, dev[0].data_ptr(), dev[1].data_ptr(), d.data_ptr(),
+                 torch.cuda.current_stream().cuda_stream) == 0
+        got.append(d.cpu().numpy().view(np.complex128).reshape(Y.shape, order="F"))
+    assert np.array_equal(got[0], got[1])
+    assert rel_l2(got[0], ref) < 1e-13
+    assert np.array_equal(got[0][:, [0, ny + 1]], Y[:, [0, ny + 1]])

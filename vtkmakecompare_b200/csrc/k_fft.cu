@@ -18,6 +18,8 @@
 // is a different algorithm from FFTW's in any case).
 #include <math.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "fft_core.cuh"
 #include "tma.cuh"
@@ -620,6 +622,138 @@ __global__ void k_spn(int H, int ny, int nz, RT* base, long svj, long svk, doubl
       back(bb, ab, I0 - BB);
     }
   }
+}
+
+// SPN alone (no mean mode) with k_spn's arithmetic, operation for operation, on
+// columns staged in shared memory.  A thread of k_spn runs the pivot
+// recurrence, a division in every row of its serial chain, and the
+// elimination behind it, and its rows go through L2 twice.  Here the systems of
+// a CTA (S of them, consecutive in kx and then kz) are shared by three warps:
+// the first runs the pivots a chunk of rows ahead, the second and third
+// eliminate the real and the imaginary part.  Bound by the latency of the
+// serial chains (two CTAs per SM): 27 -> 15.6 us at 128x96x128, 42 -> 33 at
+// 160x130x128, 15 -> 13 at 64x48x64.
+template <int S>
+__global__ void __launch_bounds__(96) k_spn_pipe(int H, int ny, int nz, double2* base, long svj,
+                                                 long svk, const double* __restrict__ AC,
+                                                 const double* __restrict__ KXZ) {
+  constexpr int R = 8;  // rows of a chunk
+  extern __shared__ __align__(16) double psm[];
+  double2* vb = reinterpret_cast<double2*>(psm);  // [row][system]
+  double* rr = psm + 2 * (size_t)ny * S;          // reciprocal pivots
+  double* a3s = rr + (size_t)ny * S;              // eliminated super-diagonals
+  double* ac = a3s + (size_t)ny * S;              // AC1, AC2, AC3
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long ns = (long)H * nz, t0 = (long)blockIdx.x * S;
+  const int NN = ny;
+  // this thread copies column threadIdx.x mod S, rows threadIdx.x / S + ...
+  const int cl = threadIdx.x % S;
+  const long ct = t0 + cl;
+  const bool cok = ct > 0 && ct < ns;  // (0, 0) is the mean mode's
+  double2* col = base + ct % H + svk * (ct / H);
+  if (cok)
+    for (int I = threadIdx.x / S; I < NN; I += 96 / S) {
+      const unsigned sa = (unsigned)__cvta_generic_to_shared(vb + I * S + cl);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(col + svj * I)
+                   : "memory");
+    }
+  for (int I = threadIdx.x; I < 3 * NN; I += 96) ac[I] = AC[I];
+  const double *AC1 = ac, *AC2 = ac + NN, *AC3 = ac + 2 * NN;
+  const long t = t0 + lane;
+  const bool ok = lane < S && t > 0 && t < ns;
+  const double kxz = ok ? KXZ[t % H + (long)H * (t / H)] : 0.0;
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  __syncthreads();
+  double a2 = 0.0;
+  if (warp == 0 && ok) {
+    a2 = AC2[0] - kxz;
+    a2 = a2 + AC1[0];  // AA(1,2) += AA(1,1)
+    if (NN == 1) a2 = a2 + AC3[0];
+  }
+  const int nch = (NN + R - 1) / R;
+  double* part = psm + 2 * lane + (warp - 1);  // re or im of this column (warps 1, 2)
+  double* rl = rr + lane;
+  double* al = a3s + lane;
+  double b = 0.0;
+  // rows I0.. of a chunk, unrolled where it is whole and not the last: a
+  // chunk's operands are read before its chain (the stores would hold them back)
+  auto rows = [&](int I0, int n, auto f) {
+    if (n == R) f(I0, std::integral_constant<int, R>());
+    else
+      for (int q = 0; q < n; ++q) f(I0 + q, std::integral_constant<int, 1>());
+  };
+  for (int c = 0; c <= nch; ++c) {
+    if (warp == 0 && c < nch && ok) {
+      rows(c * R, min(R, NN - 1 - c * R), [&](int I, auto nr) {
+        constexpr int N = decltype(nr)::value;
+        double c1[N], c2[N], c3[N];
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+          c1[q] = AC1[I + q + 1];
+          c2[q] = AC2[I + q + 1] - kxz;
+          c3[q] = AC3[I + q];
+        }
+        if (I + N + 1 == NN) c2[N - 1] = c2[N - 1] + AC3[NN - 1];  // AA(NY,2) += AA(NY,3)
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+          const double r = 1.0 / a2;
+          const double a3 = c3[q] * r;
+          rl[(I + q) * S] = r;
+          al[(I + q) * S] = a3;
+          a2 = c2[q] - c1[q] * a3;
+        }
+      });
+      if (c == nch - 1) rl[(NN - 1) * S] = a2;  // the last row divides
+    }
+    if (warp > 0 && c > 0 && ok) {
+      rows((c - 1) * R, min(R, NN - 1 - (c - 1) * R), [&](int I, auto nr) {
+        constexpr int N = decltype(nr)::value;
+        double v[N], r[N], a1[N];
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+          v[q] = part[2 * (I + q) * S];
+          r[q] = rl[(I + q) * S];
+          a1[q] = AC1[I + q];
+        }
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+          b = I + q == 0 ? v[q] : v[q] - a1[q] * b;
+          b = b * r[q];
+          part[2 * (I + q) * S] = b;
+        }
+      });
+      if (c == nch) {
+        const int I = NN - 1;
+        b = I == 0 ? part[0] : part[2 * I * S] - AC1[I] * b;
+        b = b / rl[I * S];
+        part[2 * I * S] = b;
+      }
+    }
+    __syncthreads();
+  }
+  if (warp > 0 && ok)
+    for (int I1 = NN - 1; I1 > 0; I1 -= R)  // rows I1 - 1 down to I1 - R
+      if (I1 >= R) {
+        double v[R], a[R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+          v[q] = part[2 * (I1 - 1 - q) * S];
+          a[q] = al[(I1 - 1 - q) * S];
+        }
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+          b = v[q] - a[q] * b;
+          part[2 * (I1 - 1 - q) * S] = b;
+        }
+      } else {
+        for (int I = I1 - 1; I >= 0; --I) {
+          b = part[2 * I * S] - al[I * S] * b;
+          part[2 * I * S] = b;
+        }
+      }
+  __syncthreads();
+  if (cok)
+    for (int I = threadIdx.x / S; I < NN; I += 96 / S) col[svj * I] = vb[I * S + cl];
 }
 
 // ------------------------------------- SPN: two-ended Thomas (fast form) --
@@ -1336,7 +1470,32 @@ void launch_spn_fast_f32(const PoissonPlan& pp, cudaStream_t s) {
   launch_spn_f32(pp, s);
 }
 
+// SPN without the mean mode through k_spn_pipe; false where a column of 8 systems
+// does not fit shared memory or the spectrum is off the 16-byte boundary
+static bool spn_pipe(int H, int ny, int nz, double* base, long sj, long sk, const double* AC,
+                     const double* KXZ, cudaStream_t s) {
+  if (((uintptr_t)base & 15) != 0) return false;
+  auto smem = [&](int S) { return ((size_t)4 * ny * S + 3 * (size_t)ny) * sizeof(double); };
+  const long ns = (long)H * nz;
+  double2* b2 = reinterpret_cast<double2*>(base);
+  // 32 systems where two CTAs of them share an SM, fewer for longer columns
+  const int S = smem(32) <= 112 * 1024 ? 32 : (smem(16) <= 112 * 1024 ? 16 : 8);
+  if (smem(S) > 220 * 1024) return false;
+  count_launch();
+#define NSE_SPN_PIPE(S_)                                                                     \
+  {                                                                                          \
+    smem_optin((const void*)k_spn_pipe<S_>, smem(S_));                                       \
+    k_spn_pipe<S_><<<(unsigned)((ns + S_ - 1) / S_), 96, smem(S_), s>>>(H, ny, nz, b2, sj, sk, \
+                                                                        AC, KXZ);            \
+  }
+  if (S == 32) NSE_SPN_PIPE(32) else if (S == 16) NSE_SPN_PIPE(16) else NSE_SPN_PIPE(8)
+#undef NSE_SPN_PIPE
+  return true;
+}
 void launch_spn(const PoissonPlan& pp, bool do_spn, bool do_sp0b, cudaStream_t s) {
+  if (do_spn && !do_sp0b &&
+      spn_pipe(pp.H, pp.ny, pp.nz, pp.spec, pp.Hp, (long)pp.Hp * pp.ny, pp.AC, pp.KXZ, s))
+    return;
   dim3 grid((2 * pp.H + 63) / 64, pp.nz);
   count_launch();
   k_spn<double><<<grid, 64, 0, s>>>(pp.H, pp.ny, pp.nz, pp.spec, pp.Hp, (long)pp.Hp * pp.ny,
@@ -1349,6 +1508,7 @@ void launch_spn(const PoissonPlan& pp, bool do_spn, bool do_sp0b, cudaStream_t s
 void launch_spn_view(int H, int ny, int nz, double* base, long sj, long sk, double* sc,
                      long scj, long sck, const double* AC, const double* KXZ, bool do_spn,
                      bool do_sp0b, cudaStream_t s) {
+  if (do_spn && !do_sp0b && spn_pipe(H, ny, nz, base, sj, sk, AC, KXZ, s)) return;
   dim3 grid((2 * H + 63) / 64, nz);
   count_launch();
   k_spn<double><<<grid, 64, 0, s>>>(H, ny, nz, base, sj, sk, sc, scj, sck, AC, KXZ,
