@@ -23,10 +23,11 @@ namespace nse {
 
 namespace {
 
+// A padded cell by its indices
 struct Pos {
   int c[3];
+  __device__ __forceinline__ int ix(int ax) const { return c[ax]; }
 };
-
 __device__ __forceinline__ bool inside(const Dims& D, const Pos& p) {
   return p.c[0] >= 1 && p.c[0] <= D.nx && p.c[1] >= 1 && p.c[1] <= D.ny && p.c[2] >= 1 &&
          p.c[2] <= D.nz;
@@ -38,10 +39,30 @@ __device__ __forceinline__ Pos sh(Pos p, int axis, int s) {
   p.c[axis] += s;
   return p;
 }
-__device__ __forceinline__ Pos sh2(Pos p, int a1, int s1, int a2, int s2) {
-  p.c[a1] += s1;
-  p.c[a2] += s2;
+
+// A cell next to the thread's own, which lies off the y and z boundaries: one
+// step at most in each direction, so every neighbour is an output cell
+// (x wraps, as the periodic ghosts do) and the shifts are known to the
+// compiler, which then loads and forms each shared value once
+struct Near {
+  int i, j, k;
+  long c, xm, xp;  // the own cell and the steps to its x neighbours
+  int s[3];
+  __device__ __forceinline__ int ix(int ax) const {
+    return (ax == 0 ? i : ax == 1 ? j : k) + s[ax];
+  }
+};
+__device__ __forceinline__ bool inside(const Dims&, const Near&) { return true; }
+__device__ __forceinline__ long at(const Dims& D, const Near& p) {
+  return p.c + (p.s[0] > 0 ? p.xp : p.s[0] < 0 ? p.xm : 0) + p.s[1] * D.sx + p.s[2] * D.sy;
+}
+__device__ __forceinline__ Near sh(Near p, int axis, int s) {
+  p.s[axis] += s;
   return p;
+}
+template <class Q>
+__device__ __forceinline__ Q sh2(const Q& p, int a1, int s1, int a2, int s2) {
+  return sh(sh(p, a1, s1), a2, s2);
 }
 
 // ----------------------------------------------- explicit-term transposes --
@@ -58,56 +79,58 @@ struct XArgs {
   double cfac, dfac, qfac;  // dt/Re/2, dt/(2 Re Sc R), -dt/R
 };
 
-__device__ __forceinline__ double val(const XArgs& a, const double* f, const Pos& p) {
+template <class Q>
+__device__ __forceinline__ double val(const XArgs& a, const double* f, const Q& p) {
   return f[at(a.D, p)];
 }
 // momentum convection output of component AC at o: -0.25 dt * adjoint
-__device__ __forceinline__ double qmom(const XArgs& a, int AC, const Pos& o) {
+template <class Q>
+__device__ __forceinline__ double qmom(const XArgs& a, int AC, const Q& o) {
   return -0.25 * a.dt * a.B[AC][at(a.D, o)];
 }
 
 // square term ((f + f+)^2 - (f + f-)^2) / d12 of output AC; adjoint w.r.t. f = vel[AC] at q
-template <int AC>
-__device__ double sq_f(const XArgs& a, const Pos& q) {
+template <int AC, class Q>
+__device__ __forceinline__ double sq_f(const XArgs& a, const Q& q) {
   const double* f = a.vel[AC];
   const double* d12 = a.g.d12[AC];
   double s = 0.0;
   if (inside(a.D, q)) {
-    const double m = qmom(a, AC, q) * a.g.r12[AC][q.c[AC]];
+    const double m = qmom(a, AC, q) * a.g.r12[AC][q.ix(AC)];
     s += 2.0 * m * ((val(a, f, q) + val(a, f, sh(q, AC, 1))) - (val(a, f, q) + val(a, f, sh(q, AC, -1))));
   }
-  Pos o = sh(q, AC, -1);
-  if (inside(a.D, o)) s += 2.0 * qmom(a, AC, o) * a.g.r12[AC][o.c[AC]] * (val(a, f, o) + val(a, f, q));
+  Q o = sh(q, AC, -1);
+  if (inside(a.D, o)) s += 2.0 * qmom(a, AC, o) * a.g.r12[AC][o.ix(AC)] * (val(a, f, o) + val(a, f, q));
   o = sh(q, AC, 1);
-  if (inside(a.D, o)) s -= 2.0 * qmom(a, AC, o) * a.g.r12[AC][o.c[AC]] * (val(a, f, o) + val(a, f, q));
+  if (inside(a.D, o)) s -= 2.0 * qmom(a, AC, o) * a.g.r12[AC][o.ix(AC)] * (val(a, f, o) + val(a, f, q));
   return s;
 }
 
 // cross term of output AC along AF: scale (Gp (f(o+eF) + f(o)) - Gm (f(o) + f(o-eF)))
 // with f = vel[AC], g = vel[AF], scale = 1/(d12_AC(o) d_AF(o)),
 // Gp = g(o+eC) dC(o+1) + g(o) dC(o), Gm = g(o+eC-eF) dC(o+1) + g(o-eF) dC(o)
-template <int AC, int AF>
-__device__ __forceinline__ double cross_m(const XArgs& a, const Pos& o) {
-  return qmom(a, AC, o) * a.g.r12[AC][o.c[AC]] * a.g.r[AF][o.c[AF]];
+template <int AC, int AF, class Q>
+__device__ __forceinline__ double cross_m(const XArgs& a, const Q& o) {
+  return qmom(a, AC, o) * a.g.r12[AC][o.ix(AC)] * a.g.r[AF][o.ix(AF)];
 }
-template <int AC, int AF>
-__device__ __forceinline__ double cross_gp(const XArgs& a, const Pos& o) {
+template <int AC, int AF, class Q>
+__device__ __forceinline__ double cross_gp(const XArgs& a, const Q& o) {
   const double* gg = a.vel[AF];
   const double* dC = a.g.d[AC];
-  return val(a, gg, sh(o, AC, 1)) * dC[o.c[AC] + 1] + val(a, gg, o) * dC[o.c[AC]];
+  return val(a, gg, sh(o, AC, 1)) * dC[o.ix(AC) + 1] + val(a, gg, o) * dC[o.ix(AC)];
 }
-template <int AC, int AF>
-__device__ __forceinline__ double cross_gm(const XArgs& a, const Pos& o) {
+template <int AC, int AF, class Q>
+__device__ __forceinline__ double cross_gm(const XArgs& a, const Q& o) {
   const double* gg = a.vel[AF];
   const double* dC = a.g.d[AC];
-  return val(a, gg, sh2(o, AC, 1, AF, -1)) * dC[o.c[AC] + 1] +
-         val(a, gg, sh(o, AF, -1)) * dC[o.c[AC]];
+  return val(a, gg, sh2(o, AC, 1, AF, -1)) * dC[o.ix(AC) + 1] +
+         val(a, gg, sh(o, AF, -1)) * dC[o.ix(AC)];
 }
 // adjoint w.r.t. f = vel[AC] at q
-template <int AC, int AF>
-__device__ double cross_f(const XArgs& a, const Pos& q) {
+template <int AC, int AF, class Q>
+__device__ __forceinline__ double cross_f(const XArgs& a, const Q& q) {
   double s = 0.0;
-  Pos o = sh(q, AF, -1);
+  Q o = sh(q, AF, -1);
   if (inside(a.D, o)) s += cross_m<AC, AF>(a, o) * cross_gp<AC, AF>(a, o);
   if (inside(a.D, q))
     s += cross_m<AC, AF>(a, q) * (cross_gp<AC, AF>(a, q) - cross_gm<AC, AF>(a, q));
@@ -116,27 +139,27 @@ __device__ double cross_f(const XArgs& a, const Pos& q) {
   return s;
 }
 // adjoint w.r.t. g = vel[AF] at q
-template <int AC, int AF>
-__device__ double cross_g(const XArgs& a, const Pos& q) {
+template <int AC, int AF, class Q>
+__device__ __forceinline__ double cross_g(const XArgs& a, const Q& q) {
   const double* f = a.vel[AC];
   const double* dC = a.g.d[AC];
   double s = 0.0;
-  Pos o = sh(q, AC, -1);  // q = o + eC: weight dC(o+1)
+  Q o = sh(q, AC, -1);  // q = o + eC: weight dC(o+1)
   if (inside(a.D, o))
-    s += cross_m<AC, AF>(a, o) * dC[o.c[AC] + 1] * (val(a, f, sh(o, AF, 1)) + val(a, f, o));
+    s += cross_m<AC, AF>(a, o) * dC[o.ix(AC) + 1] * (val(a, f, sh(o, AF, 1)) + val(a, f, o));
   if (inside(a.D, q))  // q = o: weight dC(o)
-    s += cross_m<AC, AF>(a, q) * dC[q.c[AC]] * (val(a, f, sh(q, AF, 1)) + val(a, f, q));
+    s += cross_m<AC, AF>(a, q) * dC[q.ix(AC)] * (val(a, f, sh(q, AF, 1)) + val(a, f, q));
   o = sh2(q, AC, -1, AF, 1);  // q = o + eC - eF: weight dC(o+1)
   if (inside(a.D, o))
-    s -= cross_m<AC, AF>(a, o) * dC[o.c[AC] + 1] * (val(a, f, o) + val(a, f, sh(o, AF, -1)));
+    s -= cross_m<AC, AF>(a, o) * dC[o.ix(AC) + 1] * (val(a, f, o) + val(a, f, sh(o, AF, -1)));
   o = sh(q, AF, 1);  // q = o - eF: weight dC(o)
   if (inside(a.D, o))
-    s -= cross_m<AC, AF>(a, o) * dC[o.c[AC]] * (val(a, f, o) + val(a, f, sh(o, AF, -1)));
+    s -= cross_m<AC, AF>(a, o) * dC[o.ix(AC)] * (val(a, f, o) + val(a, f, sh(o, AF, -1)));
   return s;
 }
 
-template <int X>
-__device__ double conv_adj(const XArgs& a, const Pos& q) {
+template <int X, class Q>
+__device__ __forceinline__ double conv_adj(const XArgs& a, const Q& q) {
   constexpr int Y1 = (X + 1) % 3, Y2 = (X + 2) % 3;
   return sq_f<X>(a, q) + cross_f<X, Y1>(a, q) + cross_f<X, Y2>(a, q) + cross_g<Y1, X>(a, q) +
          cross_g<Y2, X>(a, q);
@@ -158,25 +181,25 @@ __device__ __forceinline__ void lap_coef(const AdjGrid& g, int comp, int ax, int
   }
 }
 
-template <int C>
-__device__ double cond_adj(const XArgs& a, const Pos& q) {
+template <int C, class Q>
+__device__ __forceinline__ double cond_adj(const XArgs& a, const Q& q) {
   const double* A = a.A[C];
   double s = 0.0;
 #pragma unroll
   for (int ax = 0; ax < 3; ++ax) {
     double cp, cm;
     if (inside(a.D, q)) {
-      lap_coef(a.g, C, ax, q.c[ax], cp, cm);
+      lap_coef(a.g, C, ax, q.ix(ax), cp, cm);
       s -= (cp + cm) * val(a, A, q);
     }
-    Pos o = sh(q, ax, -1);
+    Q o = sh(q, ax, -1);
     if (inside(a.D, o)) {
-      lap_coef(a.g, C, ax, o.c[ax], cp, cm);
+      lap_coef(a.g, C, ax, o.ix(ax), cp, cm);
       s += cp * val(a, A, o);
     }
     o = sh(q, ax, 1);
     if (inside(a.D, o)) {
-      lap_coef(a.g, C, ax, o.c[ax], cp, cm);
+      lap_coef(a.g, C, ax, o.ix(ax), cp, cm);
       s += cm * val(a, A, o);
     }
   }
@@ -192,23 +215,24 @@ __device__ __forceinline__ void diffT_coef(const AdjGrid& g, int ax, int o, doub
   cm = L * r12[o - 1] * r[o];
 }
 
-__device__ double diffT_adj(const XArgs& a, const Pos& q) {
+template <class Q>
+__device__ __forceinline__ double diffT_adj(const XArgs& a, const Q& q) {
   double s = 0.0;
 #pragma unroll
   for (int ax = 0; ax < 3; ++ax) {
     double cp, cm;
     if (inside(a.D, q)) {
-      diffT_coef(a.g, ax, q.c[ax], a.L, cp, cm);
+      diffT_coef(a.g, ax, q.ix(ax), a.L, cp, cm);
       s -= (cp + cm) * val(a, a.At, q);
     }
-    Pos o = sh(q, ax, -1);
+    Q o = sh(q, ax, -1);
     if (inside(a.D, o)) {
-      diffT_coef(a.g, ax, o.c[ax], a.L, cp, cm);
+      diffT_coef(a.g, ax, o.ix(ax), a.L, cp, cm);
       s += cp * val(a, a.At, o);
     }
     o = sh(q, ax, 1);
     if (inside(a.D, o)) {
-      diffT_coef(a.g, ax, o.c[ax], a.L, cp, cm);
+      diffT_coef(a.g, ax, o.ix(ax), a.L, cp, cm);
       s += cm * val(a, a.At, o);
     }
   }
@@ -220,50 +244,53 @@ __device__ double diffT_adj(const XArgs& a, const Pos& q) {
 //   m1(o) = qT(o) / (2 d12(o-1) d(o));
 //   term2(o) = (R T(o) d(o+1) + R T(o+e) d(o)) f(o) m2(o),
 //   m2(o) = qT(o) / (2 d12(o) d(o)),  qT = -dt/R * adjoint of u_vT
-__device__ __forceinline__ double m1T(const XArgs& a, int ax, const Pos& o) {
+template <class Q>
+__device__ __forceinline__ double m1T(const XArgs& a, int ax, const Q& o) {
   const double qT = a.qfac * val(a, a.Bt, o);
-  return 0.5 * qT * a.g.r12[ax][o.c[ax] - 1] * a.g.r[ax][o.c[ax]];
+  return 0.5 * qT * a.g.r12[ax][o.ix(ax) - 1] * a.g.r[ax][o.ix(ax)];
 }
-__device__ __forceinline__ double m2T(const XArgs& a, int ax, const Pos& o) {
+template <class Q>
+__device__ __forceinline__ double m2T(const XArgs& a, int ax, const Q& o) {
   const double qT = a.qfac * val(a, a.Bt, o);
-  return 0.5 * qT * a.g.r12[ax][o.c[ax]] * a.g.r[ax][o.c[ax]];
+  return 0.5 * qT * a.g.r12[ax][o.ix(ax)] * a.g.r[ax][o.ix(ax)];
 }
 // adjoint w.r.t. vel[AX] at q
-template <int AX>
-__device__ double cscal_vel_adj(const XArgs& a, const Pos& q) {
+template <int AX, class Q>
+__device__ __forceinline__ double cscal_vel_adj(const XArgs& a, const Q& q) {
   const double* d = a.g.d[AX];
   const double R = a.R;
   double s = 0.0;
-  Pos o = sh(q, AX, 1);
+  Q o = sh(q, AX, 1);
   if (inside(a.D, o))
-    s -= m1T(a, AX, o) * (R * val(a, a.T, q) * d[o.c[AX]] + R * val(a, a.T, o) * d[q.c[AX]]);
+    s -= m1T(a, AX, o) * (R * val(a, a.T, q) * d[o.ix(AX)] + R * val(a, a.T, o) * d[q.ix(AX)]);
   if (inside(a.D, q))
     s += m2T(a, AX, q) *
-         (R * val(a, a.T, q) * d[q.c[AX] + 1] + R * val(a, a.T, sh(q, AX, 1)) * d[q.c[AX]]);
+         (R * val(a, a.T, q) * d[q.ix(AX) + 1] + R * val(a, a.T, sh(q, AX, 1)) * d[q.ix(AX)]);
   return s;
 }
 // adjoint w.r.t. T at q
-__device__ double cscal_T_adj(const XArgs& a, const Pos& q) {
+template <class Q>
+__device__ __forceinline__ double cscal_T_adj(const XArgs& a, const Q& q) {
   const double R = a.R;
   double s = 0.0;
 #pragma unroll
   for (int ax = 0; ax < 3; ++ax) {
     const double* d = a.g.d[ax];
     const double* f = a.vel[ax];
-    Pos o = sh(q, ax, 1);
-    if (inside(a.D, o)) s -= m1T(a, ax, o) * R * d[o.c[ax]] * val(a, f, q);
+    Q o = sh(q, ax, 1);
+    if (inside(a.D, o)) s -= m1T(a, ax, o) * R * d[o.ix(ax)] * val(a, f, q);
     if (inside(a.D, q)) {
-      s -= m1T(a, ax, q) * R * d[q.c[ax] - 1] * val(a, f, sh(q, ax, -1));
-      s += m2T(a, ax, q) * R * d[q.c[ax] + 1] * val(a, f, q);
+      s -= m1T(a, ax, q) * R * d[q.ix(ax) - 1] * val(a, f, sh(q, ax, -1));
+      s += m2T(a, ax, q) * R * d[q.ix(ax) + 1] * val(a, f, q);
     }
     o = sh(q, ax, -1);
-    if (inside(a.D, o)) s += m2T(a, ax, o) * R * d[o.c[ax]] * val(a, f, o);
+    if (inside(a.D, o)) s += m2T(a, ax, o) * R * d[o.ix(ax)] * val(a, f, o);
   }
   return s;
 }
 
-template <int F>
-__device__ double raw_adj(const XArgs& a, const Pos& q) {
+template <int F, class Q>
+__device__ __forceinline__ double raw_adj(const XArgs& a, const Q& q) {
   if constexpr (F < 3) {
     double s = inside(a.D, q) ? val(a, a.A[F], q) : 0.0;
     return s + cond_adj<F>(a, q) + conv_adj<F>(a, q) + cscal_vel_adj<F>(a, q);
@@ -297,6 +324,11 @@ __global__ void k_adj_explicit(XArgs a, double* __restrict__ out) {
   const long c = D.P(i, j, k);
   if (F == 1 && j == D.ny) {  // v(ny) is set to zero by SET_BC
     out[c] = 0.0;
+    return;
+  }
+  if (j > 1 && j < D.ny && k > 1 && k < D.nz) {  // (the same for a whole warp)
+    const Near q = {i, j, k, c, i > 1 ? -1L : (long)D.nx - 1, i < D.nx ? 1L : 1L - D.nx, {0, 0, 0}};
+    out[c] = raw_adj<F>(a, q);
     return;
   }
   int qi[3], qk[3], qj[3];
