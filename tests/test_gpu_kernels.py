@@ -159,3 +159,48 @@ def test_spn_columns_match_oracle(n):
     assert np.array_equal(got[0], got[1])
     assert rel_l2(got[0], ref) < 1e-13
     assert np.array_equal(got[0][:, [0, ny + 1]], Y[:, [0, ny + 1]])
+
+
+# The adjoint on recorded steps in place (the lean form) against the one that copies
+# (everything on one stream): grids with remainders of the 32 x 4 blocks, segments
+# of one, some and all steps, a weight on a field behind the upper wall's row.
+# Both are held to 1e-8 of the numpy adjoint (test_gpu_adjoint); to each other, a tenth.
+@pytest.mark.parametrize("n,every", [((50, 15, 20), 1), ((64, 13, 18), 4), ((90, 14, 25), 9),
+                                     ((33 * 2 - 2, 20, 12), 2)])
+def test_adjoint_in_place_matches_copied(n, every):
+    g, f, c1, par = make_case(*n, seed=8)
+    out = []
+    fields = ("u", "v", "w", "T", "u_ta", "v_ta", "w_ta", "u_pre", "v_pre", "w_pre", "T_pre")
+    for flags in (0, S.FLAG_ONE_STREAM):
+        cfg = S.Config(*n, par["dt"], par["Re"], par["Sc"], 50.0, g["xl"], g["yl"], g["zl"],
+                       y0=-1.0, ystretch=2.0, body_force=par["force"], t_bot=1.0,
+                       t_solid=par["tsolid"], flags=flags)
+        with S.Context(cfg) as ctx:
+            for k in ("u", "v", "w", "T"):
+                ctx.upload(k, f[k])
+            ctx.upload("cellvalue", c1)
+            ctx.project()
+            ctx.start()
+            ctx.step(2)
+            with S.Adjoint(ctx, 9, checkpoint_every=every, avg_from=5) as adj:
+                rng = np.random.default_rng(3)
+                for k in ("v", "u_ta", "T_pre"):
+                    adj.set_weight(k, rng.standard_normal(ctx.shape))
+                J, grad = adj.gradient()
+                init = [adj.initial_adjoint(k)[1:-1, 1:-1, 1:-1]
+                        for k in ("u", "v", "w", "T", "u_ta", "w_pre", "T_pre")]
+            out.append([np.array(J), grad] + init + [ctx.download(k) for k in fields])
+            if not flags:  # the context is left at the state after the steps
+                got = [ctx.download(k) for k in STATE]
+                for k in ("u", "v", "w", "T"):
+                    ctx.upload(k, f[k])
+                ctx.project()
+                ctx.step_index = 1
+                ctx.start()
+                ctx.step(2)
+                ctx.step(9)
+                for k, a in zip(STATE, got):
+                    assert np.array_equal(a, ctx.download(k)), k
+    for k, (a, b) in enumerate(zip(*out)):
+        assert np.linalg.norm(b) > 0
+        assert rel_l2(a, b) < 1e-9, k

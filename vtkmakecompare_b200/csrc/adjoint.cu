@@ -10,7 +10,7 @@
 // then its steps are reversed one by one with the transposed kernels of
 // k_adjoint.cu; the transposed line solves are the step's own line solves
 // between diagonal scalings.  Device memory: (ceil(nsteps/ckpt) * 11 +
-// ckpt * 23 + 36) padded fields.
+// ckpt * 23 + 32) padded fields.
 #include <algorithm>
 #include <vector>
 
@@ -28,7 +28,7 @@ enum { S_U = 0, S_V, S_W, S_T, S_UTA, S_VTA, S_WTA, S_UP, S_VP, S_WP, S_TP, NS }
 const int kSeg = 7;   // u, v, w, T, u_ta, v_ta, w_ta at the start of a recorded step
 const int kRec = 16;  // line-pass inputs and outputs of a recorded step
 // work fields
-enum { W_B = 0, W_O = 4, W_XS = 8, W_RB = 9, W_ST = 10, NW = 14 };
+enum { W_B = 0, W_O = 4, W_XS = 8, W_RB = 9, NW = 10 };
 
 int state_index(int field) {
   for (int q = 0; q < NS; ++q)
@@ -104,8 +104,9 @@ bool run_forward(nse_adjoint* a) {
 }
 
 // one step reversed: a->barp holds the adjoint of the state after the step
-// on entry and of the state before it on return
-void adjoint_step(nse_adjoint* a, double* sg, double* const* rc, int l) {
+// on entry and of the state before it on return.  sg: u, v, w, T and u_ta, v_ta,
+// w_ta the step started from (bc: their ghosts are set)
+void adjoint_step(nse_adjoint* a, double* const* sg, bool bc, double* const* rc, int l) {
   const CtxInfo& ci = a->ci;
   const nse_config& c = *ci.cfg;
   const Dims& D = ci.d;
@@ -117,7 +118,6 @@ void adjoint_step(nse_adjoint* a, double* sg, double* const* rc, int l) {
   for (int q = 0; q < 4; ++q) cb[q] = a->cbar.as<double>() + (size_t)q * D.ncell;
   double* wk[NW];
   for (int q = 0; q < NW; ++q) wk[q] = a->field(a->work, q);
-  auto SG = [&](int q) { return sg + (size_t)q * a->F; };
   // MKP (mkp.f:88-217) transposed
   double* ub[3] = {bar[S_U], bar[S_V], bar[S_W]};
   const double* ubc[3] = {bar[S_U], bar[S_V], bar[S_W]};
@@ -128,7 +128,7 @@ void adjoint_step(nse_adjoint* a, double* sg, double* const* rc, int l) {
   if (!launch_spn_transposed(*ci.pp, ci.rg.rdy, ci.g.dy, s)) launch_adj_spn(*ci.pp, s);
   launch_fft_z(*ci.pp, true, s);
   launch_fft_inv_x(*ci.pp, D, wk[W_RB], s);
-  launch_adj_div(D, g, ub, wk[W_RB], c.dt, s);
+  launch_adj_div(D, g, ub, wk[W_RB], c1, c.dt, c.eta, s);
   // line passes in reverse (velocity y, z, x; temperature y, x, z forward);
   // the four components are independent: component 0 on the context's
   // stream, 1..3 on side streams forked from it and joined back
@@ -139,15 +139,17 @@ void adjoint_step(nse_adjoint* a, double* sg, double* const* rc, int l) {
     const int vdirs[3] = {1, 2, 0}, tdirs[3] = {1, 0, 2};
     const int* dirs = comp == 3 ? tdirs : vdirs;
     double* cbar = comp == 3 ? cb[0] : cb[comp + 1];
-    // scale for the last pass, then each solve's output scaling also
-    // prepares the input of the pass before it (one kernel between solves)
-    launch_adj_line_scale(D, g, dirs[2], comp, false, bar[comp], nullptr, nullptr, c1, nullptr,
-                          c.dt, c.eta, cs);
+    // scale for the last pass (u, v, w: launch_adj_div did), then each
+    // solve's output scaling also prepares the input of the pass before it (one
+    // kernel between solves; the first pass's is launch_adj_point's)
+    if (comp == 3)
+      launch_adj_line_scale(D, g, dirs[2], comp, false, bar[comp], nullptr, nullptr, c1, nullptr,
+                            c.dt, c.eta, cs);
     for (int p = 2; p >= 0; --p) {
       ctx_line_solve(a->x, dirs[p], comp, bar[comp], cs);
-      launch_adj_line_scale(D, g, dirs[p], comp, true, bar[comp], rc[4 * comp + p],
-                            rc[4 * comp + p + 1], c1, cbar, c.dt, c.eta, cs,
-                            p > 0 ? dirs[p - 1] : -1);
+      if (p > 0)
+        launch_adj_line_scale(D, g, dirs[p], comp, true, bar[comp], rc[4 * comp + p],
+                              rc[4 * comp + p + 1], c1, cbar, c.dt, c.eta, cs, dirs[p - 1]);
     }
     if (comp > 0) NSE_CUDA(cudaEventRecord(a->join[comp - 1], cs));
   }
@@ -157,19 +159,17 @@ void adjoint_step(nse_adjoint* a, double* sg, double* const* rc, int l) {
   double* B[4] = {wk[W_B], wk[W_B + 1], wk[W_B + 2], wk[W_B + 3]};
   double* pre[4] = {bar[S_UP], bar[S_VP], bar[S_WP], bar[S_TP]};
   double* bta[3] = {bar[S_UTA], bar[S_VTA], bar[S_WTA]};
-  const double* ta[3] = {SG(4), SG(5), SG(6)};
+  const double* ta[3] = {sg[4], sg[5], sg[6]};
   const double* rin[4] = {rc[0], rc[4], rc[8], rc[12]};
-  launch_adj_point(D, A, B, pre, bta, ta, rin, c1, cb, c.eta, c.dt, c.t_solid, l, s);
-  // explicit terms at the start state (SET_BC applied to a copy)
-  const size_t fb = a->F * sizeof(double);
-  for (int q = 0; q < 4; ++q)
-    NSE_CUDA(cudaMemcpyAsync(wk[W_ST + q], SG(q), fb, cudaMemcpyDeviceToDevice, s));
-  launch_set_bc(D, wk[W_ST], wk[W_ST + 1], wk[W_ST + 2], nullptr, wk[W_ST + 3], c.t_bot,
-                c.t_top, 1 | 2 | 4 | 16, s);
-  const double* vel[3] = {wk[W_ST], wk[W_ST + 1], wk[W_ST + 2]};
+  const double* xout[4] = {rc[1], rc[5], rc[9], rc[13]};
+  launch_adj_point(D, A, B, pre, bta, ta, rin, xout, g, c1, cb, c.eta, c.dt, c.t_solid, l, s);
+  // explicit terms at the start state with its ghosts
+  if (!bc)
+    launch_set_bc(D, sg[0], sg[1], sg[2], nullptr, sg[3], c.t_bot, c.t_top, 1 | 2 | 4 | 16, s);
+  const double* vel[3] = {sg[0], sg[1], sg[2]};
   NSE_CUDA(cudaEventRecord(a->fork, s));
   for (int q = 0; q < 3; ++q) NSE_CUDA(cudaStreamWaitEvent(a->side[q], a->fork, 0));
-  launch_adj_explicit(D, g, vel, wk[W_ST + 3], A, B, c.dt, c.Re, c.Sc, c.rho_cp, c.thc,
+  launch_adj_explicit(D, g, vel, sg[3], A, B, c.dt, c.Re, c.Sc, c.rho_cp, c.thc,
                       a->outp, s, a->side);
   for (int q = 0; q < 3; ++q) {
     NSE_CUDA(cudaEventRecord(a->join[q], a->side[q]));
@@ -306,21 +306,40 @@ int nse_adjoint_gradient(nse_adjoint* a, double* J, double* grad_c1) {
     const int first = m * K + 1, last = std::min(N, first + K - 1);
     if (!copy_fields(a, a->field(a->ck, (size_t)m * NS), kState, NS, true)) return NSE_ERR_CUDA;
     ctx_set_l(a->x, a->ck_l[m]);
-    int in = END_FULL;
+    const bool lean = ctx_lean_ok(a->x);
+    auto seg = [&](int r, int q) { return a->field(a->seg, (size_t)r * kSeg + q); };
+    // the start state of step r; a recorded step's T is the last output of
+    // the step before it
+    auto state = [&](int r, int q) {
+      return lean && q == 3 && r > 0 ? recp[(size_t)(r - 1) * kRec + 15] : seg(r, q);
+    };
     for (int n = first; n <= last; ++n) {
       const int r = n - first;
-      if (!copy_fields(a, a->field(a->seg, (size_t)r * kSeg), segIds, kSeg, false))
-        return NSE_ERR_CUDA;
-      // the reverse sweep reads u_ta of every step, but no p, u_ep2 or divu
-      const int out = ctx_lean_ok(a->x) ? END_TA : END_FULL;
-      ctx_step_rec(a->x, recp.data() + (size_t)r * kRec, in, out);
-      in = out;
+      if (!lean || r == 0)
+        if (!copy_fields(a, seg(r, 0), segIds, kSeg, false)) return NSE_ERR_CUDA;
+      if (!lean) {
+        ctx_step_rec(a->x, recp.data() + (size_t)r * kRec, END_FULL, END_FULL);
+        continue;
+      }
+      RecordedStep io;
+      for (int q = 0; q < 3; ++q) {
+        io.u[q] = state(r, q);
+        io.ta[q] = state(r, 4 + q);
+        // (nothing follows the segment's last step)
+        io.un[q] = n < last ? seg(r + 1, q) : nullptr;
+        io.tan[q] = n < last ? seg(r + 1, 4 + q) : nullptr;
+      }
+      io.T = state(r, 3);
+      io.rec = recp.data() + (size_t)r * kRec;
+      io.bc = r == 0;
+      ctx_step_record(a->x, io);
     }
     for (int n = last; n >= first; --n) {
       const int r = n - first;
       if (n >= n0) launch_adj_wall_flux(D, g, a->barp[S_T], c.thc, c.xl, c.zl, w, s);
-      adjoint_step(a, a->field(a->seg, (size_t)r * kSeg), recp.data() + (size_t)r * kRec,
-                   a->ck_l[m] + r);
+      double* sg[kSeg];
+      for (int q = 0; q < kSeg; ++q) sg[q] = state(r, q);
+      adjoint_step(a, sg, lean, recp.data() + (size_t)r * kRec, a->ck_l[m] + r);
     }
     if (!NSE_CUDA(cudaGetLastError())) return NSE_ERR_CUDA;
   }

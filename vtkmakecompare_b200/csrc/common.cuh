@@ -351,6 +351,18 @@ void ctx_step_rec(nse_ctx* x, double* const* rec, int in, int out);
 // the histories (phi holds the pressure); END_TA: u_ta, v_ta, w_ta as well.
 enum StepEnd { END_FULL = 0, END_LEAN, END_TA };
 bool ctx_lean_ok(nse_ctx* x);
+// A step of a context of the lean form on fields of the caller: u, v, w, T (bc:
+// their ghosts are set first) and u_ta, v_ta, w_ta it starts from, the line
+// passes' inputs and outputs rec (T's last, rec[15], with ghosts: the next step's
+// T), and where the next step's u, v, w and u_ta, v_ta, w_ta go (un[0] null:
+// the step ends after the line passes)
+struct RecordedStep {
+  double *u[3], *T, *ta[3];
+  double *un[3], *tan[3];
+  double* const* rec;
+  bool bc;
+};
+void ctx_step_record(nse_ctx* x, const RecordedStep& io);
 // the line solve of (dir, comp) of the step on the field f (ft = fb = 0)
 void ctx_line_solve(nse_ctx* x, int dir, int comp, double* f, cudaStream_t s);
 

@@ -313,9 +313,12 @@ __device__ __forceinline__ int periodic_pre(int p, int n, int* q) {
 // adjoint of the state field F (0 u, 1 v, 2 w, 3 T) at the start of the
 // step, interior cells: the explicit terms transposed and SET_BC folded.
 // A CTA covers an (x, y) tile of one plane, so the y neighbours every cell
-// gathers are mostly the tile's own rows (L1 hits).
+// gathers are mostly the tile's own rows (L1 hits).  Bound by the latency of
+// those loads (1.5 TB/s of HBM, 1.2 instructions a cycle): 740 us for the four
+// fields at 128^3 with every neighbour checked, 460 through Near, 390 with 128
+// threads at 64 registers, eight CTAs to an SM.
 template <int F>
-__global__ void k_adj_explicit(XArgs a, double* __restrict__ out) {
+__global__ void __launch_bounds__(128, 8) k_adj_explicit(XArgs a, double* __restrict__ out) {
   const Dims& D = a.D;
   const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
   const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
@@ -353,11 +356,15 @@ __global__ void k_adj_explicit(XArgs a, double* __restrict__ out) {
 }
 
 // ------------------------------------------------- pointwise transposes --
-// penalised updates, AB2 and immersed-boundary forcing (interior cells):
-//   A[X]: adjoint of the penalised u_a (in) -> adjoint of the explicit u_a (out)
+// the last scaling of the y passes (see k_adj_line_scale), then the penalised
+// updates, AB2 and immersed-boundary forcing (interior cells):
+//   A[X]: the y pass's transposed solution (in) -> adjoint of the explicit u_a (out)
+//   a0 = alpha w A[X], A[X] <- a0 / den = w A[X] (den = alpha)
 //   B[X] = a1 A[X] + adjoint of the new history u_pre
 //   bar_pre[X] <- a2 A[X], bar_ta[X] <- eta c dt A[X]
-//   cbar_X += -a0 u_a0 eta dt / den + eta dt u_ta A[X]
+//   cbar_X += a0 dt eta / alpha (rin - xout) - a0 rin eta dt / den + eta dt u_ta A[X]
+// Bound by HBM: 42 fields, 121 us at 128^3 (5.6 TB/s), where it and the four
+// scalings took 152 + 4 x 23 as passes of their own, with sixteen divisions.
 struct PArgs {
   Dims D;
   double* A[4];          // u, v, w, T
@@ -365,11 +372,23 @@ struct PArgs {
   double* bar_pre[4];
   double* bar_ta[3];
   const double* ta[3];   // u_ta, v_ta, w_ta at the start of the step
-  const double* rin[4];  // penalised u_a, v_a, w_a, u_T (input of the y pass)
+  const double* rin[4];   // penalised u_a, v_a, w_a, u_T (input of the y pass)
+  const double* xout[4];  // output of the y pass
   const double* c1;
+  AdjGrid g;
   double* cbar[4];       // c1, c2, c3, c4 (nx*ny*nz each)
   double eta, dt, tsolid, a1, a2;
 };
+
+// 1 / w and w of line direction `dir` for component `comp` at index idx
+__device__ __forceinline__ double line_rw(const AdjGrid& g, int dir, int comp, int idx) {
+  const bool wd = comp == 3 || (dir == 1 && comp != 1);
+  return wd ? g.r[dir][idx] : g.r12[dir][idx];
+}
+__device__ __forceinline__ double line_w(const AdjGrid& g, int dir, int comp, int idx) {
+  const bool wd = comp == 3 || (dir == 1 && comp != 1);
+  return wd ? g.d[dir][idx] : g.d12[dir][idx];
+}
 
 __device__ __forceinline__ double face_mask(const Dims& D, const double* c1, int comp, int i,
                                             int j, int k) {
@@ -391,20 +410,24 @@ __global__ void k_adj_point(PArgs a) {
 #pragma unroll
   for (int X = 0; X < 3; ++X) {
     const double cm = face_mask(D, a.c1, X, i, j, k);
-    const double den = 1.0 + a.eta * cm * a.dt;
-    const double a0 = a.A[X][c];
-    const double ab = a0 / den;
-    a.cbar[X + 1][m] += -a0 * a.rin[X][c] * a.eta * a.dt / den + a.eta * a.dt * a.ta[X][c] * ab;
+    const double x0 = a.A[X][c], rin = a.rin[X][c];
+    // a0 / (1 + eta c dt), where the solve's scaling by the same factor cancels
+    // but on v's wall row, which is on no line
+    const bool line = X != 1 || j < D.ny;
+    double ab = x0;
+    if (line) ab = x0 * line_w(a.g, 1, X, j);
+    else if (cm != 0.0) ab = x0 / (1.0 + a.eta * cm * a.dt);
+    double cb = a.ta[X][c] - rin;
+    if (line) cb += rin - a.xout[X][c];
+    a.cbar[X + 1][m] += a.eta * a.dt * ab * cb;
     a.B[X][c] = a.a1 * ab + a.bar_pre[X][c];
     a.bar_pre[X][c] = a.a2 * ab;
     a.bar_ta[X][c] = a.eta * cm * a.dt * ab;
     a.A[X][c] = ab;
   }
-  const double c1 = a.c1[m];
-  const double den = 1.0 + a.eta * c1 * a.dt;
-  const double t0 = a.A[3][c];
-  const double tb = t0 / den;
-  a.cbar[0][m] += t0 * a.eta * a.dt * (a.tsolid - a.rin[3][c]) / den;
+  const double rin = a.rin[3][c];
+  const double tb = a.A[3][c] * line_w(a.g, 1, 3, j);
+  a.cbar[0][m] += a.eta * a.dt * tb * ((a.tsolid - rin) + (rin - a.xout[3][c]));
   a.B[3][c] = a.a1 * tb + a.bar_pre[3][c];
   a.bar_pre[3][c] = a.a2 * tb;
   a.A[3][c] = tb;
@@ -434,12 +457,6 @@ struct SArgs {
   double dte;  // dt * eta
 };
 
-// 1 / w of line direction `dir` for component `comp` at index idx
-__device__ __forceinline__ double line_rw(const AdjGrid& g, int dir, int comp, int idx) {
-  const bool wd = comp == 3 || (dir == 1 && comp != 1);
-  return wd ? g.r[dir][idx] : g.r12[dir][idx];
-}
-
 __global__ void k_adj_line_scale(SArgs a) {
   const Dims& D = a.D;
   const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
@@ -447,29 +464,27 @@ __global__ void k_adj_line_scale(SArgs a) {
   const int k = 1 + blockIdx.z;
   if (i > D.nx || (a.comp == 1 && j == D.ny)) return;
   const int ijk[3] = {i, j, k};
-  const double rw = line_rw(a.g, a.dir, a.comp, ijk[a.dir]);  // 1 / w
   const double cm = face_mask(D, a.c1, a.comp, i, j, k);
-  const double alpha = a.dte * cm + 1.0;
   const long c = D.P(i, j, k);
+  const double x = a.xb[c];
   if (!a.out) {
-    a.xb[c] = cm == 0.0 ? a.xb[c] * rw : a.xb[c] * rw / alpha;
+    const double v = x * line_rw(a.g, a.dir, a.comp, ijk[a.dir]);
+    a.xb[c] = cm == 0.0 ? v : v / (a.dte * cm + 1.0);
     return;
   }
-  const double rb = cm == 0.0 ? a.xb[c] / rw : alpha * a.xb[c] / rw;
-  a.cbar[D.C(i, j, k)] += rb * (cm == 0.0 ? a.dte : a.dte / alpha) * (a.rin[c] - a.xout[c]);
-  if (a.next < 0) {
-    a.xb[c] = rb;
-    return;
-  }
-  const double rn = line_rw(a.g, a.next, a.comp, ijk[a.next]);
-  a.xb[c] = cm == 0.0 ? rb * rn : rb * rn / alpha;
+  // (rbar / alpha: alpha cancels in both results but the last pass's)
+  const double ra = x * line_w(a.g, a.dir, a.comp, ijk[a.dir]);
+  a.cbar[D.C(i, j, k)] += ra * a.dte * (a.rin[c] - a.xout[c]);
+  if (a.next < 0) a.xb[c] = cm == 0.0 ? ra : (a.dte * cm + 1.0) * ra;
+  else a.xb[c] = ra * line_rw(a.g, a.next, a.comp, ijk[a.next]);
 }
 
 // -------------------------------------------------------- MKP transposes --
 // adjoint of phi at the P2S sample positions (i = 0..nx-1, J = 1..ny,
-// k = 0..nz-1): the correction u = u* - dt G, u_ta = dt G transposed
-// (G_bar = dt (u_ta_bar - u_bar) on interior cells), then every padded
-// cell that S2P's wrap fill and PHIBC copy from this sample folded back
+// k = 0..nz-1, sample 0 being cell n): the correction u = u* - dt G, u_ta = dt G
+// transposed (G_bar = dt (u_ta_bar - u_bar) on interior cells), the padded
+// cells that S2P's wrap fill and PHIBC copy from a sample folded back: x and z
+// differences wrap, and no gradient crosses a wall
 struct GArgs {
   Dims D;
   AdjGrid g;
@@ -479,38 +494,21 @@ struct GArgs {
   double* xs;
 };
 
-__device__ __forceinline__ double gbar(const GArgs& a, int ax, const Pos& q) {
-  if (!inside(a.D, q)) return 0.0;
-  const long c = at(a.D, q);
-  return a.dt * (a.tab[ax][c] - a.ub[ax][c]) * a.g.r12[ax][q.c[ax]];
-}
-
 __global__ void k_adj_phibar(GArgs a) {
   const Dims& D = a.D;
   const int si = blockIdx.x * blockDim.x + threadIdx.x;
-  const int J = 1 + blockIdx.y;
+  const int J = 1 + blockIdx.y * blockDim.y + threadIdx.y;
   const int sk = blockIdx.z;
-  if (si >= D.nx) return;
-  int qi[2], qk[2], qj[3];
-  int ni = 0, nk = 0, nj = 0;
-  qi[ni++] = si;
-  if (si == 0) qi[ni++] = D.nx;
-  if (si == 1) qi[ni++] = D.nx + 1;
-  qk[nk++] = sk;
-  if (sk == 0) qk[nk++] = D.nz;
-  if (sk == 1) qk[nk++] = D.nz + 1;
-  qj[nj++] = J;
-  if (J == 1) qj[nj++] = 0;
-  if (J == D.ny) qj[nj++] = D.ny + 1;
-  double s = 0.0;
-  for (int b = 0; b < nj; ++b)
-    for (int e = 0; e < nk; ++e)
-      for (int t = 0; t < ni; ++t) {
-        Pos q;
-        q.c[0] = qi[t]; q.c[1] = qj[b]; q.c[2] = qk[e];
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) s += gbar(a, ax, sh(q, ax, -1)) - gbar(a, ax, q);
-      }
+  if (si >= D.nx || J > D.ny) return;
+  const int I = si == 0 ? D.nx : si, K = sk == 0 ? D.nz : sk;
+  const int im = I == 1 ? D.nx : I - 1, km = K == 1 ? D.nz : K - 1;
+  auto gbar = [&](int ax, int i, int j, int k) {
+    const long c = D.P(i, j, k);
+    return a.dt * (a.tab[ax][c] - a.ub[ax][c]) * a.g.r12[ax][ax == 0 ? i : ax == 1 ? j : k];
+  };
+  double s = gbar(0, im, J, K) - gbar(0, I, J, K);
+  s += (J > 1 ? gbar(1, I, J - 1, K) : 0.0) - (J < D.ny ? gbar(1, I, J, K) : 0.0);
+  s += gbar(2, I, J, km) - gbar(2, I, J, K);
   a.xs[D.P(si, J, sk)] = s;
 }
 
@@ -590,8 +588,11 @@ struct DArgs {
   double* ub[3];  // in: adjoint of the corrected u, v, w; out: adjoint of u*, v*, w*
   const double* rb;
   double rdt;     // 1 / dt
+  const double* c1;
+  double dte;     // dt * eta
 };
 
+// and the scaling before the x passes' transposed solves (k_adj_line_scale)
 __global__ void k_adj_div(DArgs a) {
   const Dims& D = a.D;
   const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x;
@@ -600,17 +601,20 @@ __global__ void k_adj_div(DArgs a) {
   if (i > D.nx) return;
   const long c = D.P(i, j, k);
   const double r0 = a.rb[c];
-  {
-    const int ip = i == D.nx ? 1 : i + 1;
-    a.ub[0][c] += (r0 * a.g.r[0][i] - a.rb[D.P(ip, j, k)] * a.g.r[0][ip]) * a.rdt;
-  }
-  if (j < D.ny)
-    a.ub[1][c] += (r0 * a.g.r[1][j] - a.rb[D.P(i, j + 1, k)] * a.g.r[1][j + 1]) * a.rdt;
-  else
-    a.ub[1][c] = 0.0;
-  {
-    const int kp = k == D.nz ? 1 : k + 1;
-    a.ub[2][c] += (r0 * a.g.r[2][k] - a.rb[D.P(i, j, kp)] * a.g.r[2][kp]) * a.rdt;
+  const int ip = i == D.nx ? 1 : i + 1, kp = k == D.nz ? 1 : k + 1;
+  double f[3];
+  f[0] = r0 * a.g.r[0][i] - a.rb[D.P(ip, j, k)] * a.g.r[0][ip];
+  f[1] = r0 * a.g.r[1][j] - a.rb[D.P(i, j + 1, k)] * a.g.r[1][j + 1];
+  f[2] = r0 * a.g.r[2][k] - a.rb[D.P(i, j, kp)] * a.g.r[2][kp];
+#pragma unroll
+  for (int X = 0; X < 3; ++X) {
+    if (X == 1 && j == D.ny) {
+      a.ub[X][c] = 0.0;
+      continue;
+    }
+    const double v = (a.ub[X][c] + f[X] * a.rdt) * line_rw(a.g, 0, X, i);
+    const double cm = face_mask(D, a.c1, X, i, j, k);
+    a.ub[X][c] = cm == 0.0 ? v : v / (a.dte * cm + 1.0);
   }
 }
 
@@ -840,8 +844,8 @@ void launch_adj_explicit(const Dims& D, const AdjGrid& g, const double* const ve
   a.cfac = dt / Re / 2.0;
   a.dfac = dt / (2.0 * Re * Sc * R);
   a.qfac = -dt / R;
-  const dim3 block(32, 8, 1);
-  const dim3 grid((D.nx + 31) / 32, (D.ny + 7) / 8, D.nz);
+  const dim3 block(32, 4, 1);
+  const dim3 grid((D.nx + 31) / 32, (D.ny + 3) / 4, D.nz);
   const cudaStream_t* ss = side ? side : nullptr;
   count_launch();
   k_adj_explicit<0><<<grid, block, 0, s>>>(a, out[0]);
@@ -855,14 +859,15 @@ void launch_adj_explicit(const Dims& D, const AdjGrid& g, const double* const ve
 
 void launch_adj_point(const Dims& D, double* const A[4], double* const B[4],
                       double* const bar_pre[4], double* const bar_ta[3],
-                      const double* const ta[3], const double* const rin[4], const double* c1,
+                      const double* const ta[3], const double* const rin[4],
+                      const double* const xout[4], const AdjGrid& g, const double* c1,
                       double* const cbar[4], double eta, double dt, double tsolid, int l,
                       cudaStream_t s) {
   PArgs a;
-  a.D = D;
+  a.D = D; a.g = g;
   for (int c = 0; c < 4; ++c) {
     a.A[c] = A[c]; a.B[c] = B[c]; a.bar_pre[c] = bar_pre[c]; a.rin[c] = rin[c];
-    a.cbar[c] = cbar[c];
+    a.cbar[c] = cbar[c]; a.xout[c] = xout[c];
   }
   for (int c = 0; c < 3; ++c) { a.bar_ta[c] = bar_ta[c]; a.ta[c] = ta[c]; }
   a.c1 = c1; a.eta = eta; a.dt = dt; a.tsolid = tsolid;
@@ -888,9 +893,8 @@ void launch_adj_phibar(const Dims& D, const AdjGrid& g, const double* const ub[3
   GArgs a;
   a.D = D; a.g = g; a.dt = dt; a.xs = xs;
   for (int c = 0; c < 3; ++c) { a.ub[c] = ub[c]; a.tab[c] = tab[c]; }
-  const int bx = 64;
   count_launch();
-  k_adj_phibar<<<dim3((D.nx + bx - 1) / bx, D.ny, D.nz), bx, 0, s>>>(a);
+  k_adj_phibar<<<dim3((D.nx + 31) / 32, (D.ny + 7) / 8, D.nz), dim3(32, 8), 0, s>>>(a);
 }
 
 void launch_adj_spn(const PoissonPlan& pp, cudaStream_t s) {
@@ -901,9 +905,9 @@ void launch_adj_spn(const PoissonPlan& pp, cudaStream_t s) {
 }
 
 void launch_adj_div(const Dims& D, const AdjGrid& g, double* const ub[3], const double* rb,
-                    double dt, cudaStream_t s) {
+                    const double* c1, double dt, double eta, cudaStream_t s) {
   DArgs a;
-  a.D = D; a.g = g; a.rb = rb; a.rdt = 1.0 / dt;
+  a.D = D; a.g = g; a.rb = rb; a.rdt = 1.0 / dt; a.c1 = c1; a.dte = dt * eta;
   for (int c = 0; c < 3; ++c) a.ub[c] = ub[c];
   count_launch();
   k_adj_div<<<cell_grid(D, 128), 128, 0, s>>>(a);

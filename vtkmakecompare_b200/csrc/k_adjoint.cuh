@@ -33,10 +33,12 @@ void launch_adj_explicit(const Dims& D, const AdjGrid& g, const double* const ve
                          const double* T, double* const A[4], double* const B[4], double dt,
                          double Re, double Sc, double R, double L, double* const out[4],
                          cudaStream_t s, const cudaStream_t* side = nullptr);
+// last scaling of the y passes (rin, xout: their inputs and outputs), then the
 // penalised updates, AB2 and immersed-boundary forcing transposed
 void launch_adj_point(const Dims& D, double* const A[4], double* const B[4],
                       double* const bar_pre[4], double* const bar_ta[3],
-                      const double* const ta[3], const double* const rin[4], const double* c1,
+                      const double* const ta[3], const double* const rin[4],
+                      const double* const xout[4], const AdjGrid& g, const double* c1,
                       double* const cbar[4], double eta, double dt, double tsolid, int l,
                       cudaStream_t s);
 // diagonal scalings around the step's own line solve that make it the
@@ -46,12 +48,12 @@ void launch_adj_line_scale(const Dims& D, const AdjGrid& g, int dir, int comp, b
                            double* xb, const double* rin, const double* xout, const double* c1,
                            double* cbar, double dt, double eta, cudaStream_t s, int next = -1);
 // MKP transposed: phi_bar at the P2S samples, transposed SPN/SP0B on the
-// spectrum, divergence transposed
+// spectrum, divergence transposed with the scaling before the x passes
 void launch_adj_phibar(const Dims& D, const AdjGrid& g, const double* const ub[3],
                        const double* const tab[3], double dt, double* xs, cudaStream_t s);
 void launch_adj_spn(const PoissonPlan& pp, cudaStream_t s);
 void launch_adj_div(const Dims& D, const AdjGrid& g, double* const ub[3], const double* rb,
-                    double dt, cudaStream_t s);
+                    const double* c1, double dt, double eta, cudaStream_t s);
 // objective: area-weighted wall heat flux at the y = y0 wall and its adjoint
 void launch_wall_flux(const Dims& D, const AdjGrid& g, const double* T, double tb, double thc,
                       double xl, double zl, double w, double* J, cudaStream_t s);

@@ -1321,12 +1321,12 @@ static void lines_part(int dir, int kind, const Dims& d, S* f, RO* out, const Li
   // for the uniform storage/arithmetic types
   constexpr bool uni = sizeof(S) == sizeof(R) && sizeof(R) == sizeof(RO);
   if constexpr (uni) {
-    if (a.yzshape == 1 && !out) {
+    if (a.yzshape == 1) {
       yz_launch<8>(dir, d, f, out, nu, P, MM, nother, tab, slots, mtab, (R)a.ft, (R)a.fb,
                    kind >= LK_CYC_VEL, s);
       return;
     }
-    if (a.yzshape == 3 && !out) {
+    if (a.yzshape == 3) {
       yz_launch<32>(dir, d, f, out, nu, P, MM, nother, tab, slots, mtab, (R)a.ft, (R)a.fb,
                     kind >= LK_CYC_VEL, s);
       return;
@@ -1336,10 +1336,11 @@ static void lines_part(int dir, int kind, const Dims& d, S* f, RO* out, const Li
                         kind >= LK_CYC_VEL, s);
 }
 
+// (out given: a y or z solve writes its solution there and leaves f)
 void launch_lines_part(int dir, int kind, const Dims& d, double* f, const LineArgs& a,
                        const double* tab, const int* slots, const int* ids, int nmasked,
-                       const double* mtab, cudaStream_t s) {
-  lines_part<double, double, double>(dir, kind, d, f, nullptr, a, tab, slots, ids, nmasked,
+                       const double* mtab, cudaStream_t s, double* out) {
+  lines_part<double, double, double>(dir, kind, d, f, out, a, tab, slots, ids, nmasked,
                                      mtab, s);
 }
 

@@ -44,7 +44,7 @@ void launch_part_tables(int dir, int kind, const Dims& d, const GridDev& g, cons
                         cudaStream_t s);
 void launch_lines_part(int dir, int kind, const Dims& d, double* f, const LineArgs& a,
                        const double* tab, const int* slots, const int* ids, int nmasked,
-                       const double* mtab, cudaStream_t s);
+                       const double* mtab, cudaStream_t s, double* out = nullptr);
 void launch_lines_part_f32(int dir, int kind, const Dims& d, float* f, double* out,
                            const LineArgs& a, const float* tab, const int* slots,
                            const int* ids, int nmasked, const float* mtab,
@@ -1493,7 +1493,7 @@ struct nse_ctx {
     void* t = nullptr;
     DBuf T, uT;
     long long nk = 0;  // kernels in the graph
-  } sg[8];
+  } sg[18];
   unsigned long long sg_sig = 0;  // launch shapes the graphs were captured with
   void* hpin = nullptr;           // pinned staging of the masked line lists
   size_t hpin_n = 0;              // its capacity (ints)
@@ -2869,6 +2869,10 @@ static void ctx_step(nse_ctx* x, int in = END_FULL, int out = END_FULL) {
 
 }  // extern "C"
 
+extern "C" {
+static int step_replay(nse_ctx* x, int in, int out);
+}
+
 // internal hooks of the adjoint driver (adjoint.cu)
 namespace nse {
 bool ctx_info(nse_ctx* x, CtxInfo& out) {
@@ -2887,9 +2891,75 @@ int ctx_get_l(nse_ctx* x) { return x->l; }
 void ctx_set_l(nse_ctx* x, int l) { x->l = l; }
 bool ctx_lean_ok(nse_ctx* x) { return lean_ok(x); }
 void ctx_step_rec(nse_ctx* x, double* const* rec, int in, int out) {
+  if (!rec && step_replay(x, in, out) == 1) return;
   x->rec = rec;
   ctx_step(x, in, out);
   x->rec = nullptr;
+}
+// A step of the lean form (ctx_lean_ok) whose fields live where its record is
+// kept, so that nothing is copied but the x passes' inputs: the right-hand side
+// writes the first line inputs, the y and z passes solve from one record field
+// into the next, and the correction writes the next step's start state.
+void ctx_step_record(nse_ctx* x, const RecordedStep& io) {
+  const Dims& d = x->d;
+  const nse_config& c = x->cfg;
+  cudaStream_t s = x->stream;
+  StepParams sp;
+  sp.dt = c.dt; sp.Re = c.Re; sp.Sc = c.Sc; sp.eta = c.eta;
+  sp.force = c.body_force; sp.source = c.heat_source;
+  sp.tbot = c.t_bot; sp.ttop = c.t_top; sp.tsolid = c.t_solid;
+  sp.rho_cp = c.rho_cp; sp.thc = c.thc; sp.l = x->l;
+  double* const* r = io.rec;
+  const size_t fb = d.ntot * sizeof(double);
+  if (io.bc)
+    launch_set_bc(d, io.u[0], io.u[1], io.u[2], nullptr, io.T, c.t_bot, c.t_top, 1 | 2 | 4 | 16,
+                  s);
+  launch_rhs_fast(d, x->g, x->rg, sp, io.u[0], io.u[1], io.u[2], io.T, io.ta[0], io.ta[1],
+                  io.ta[2], F(x, NSE_U_PRE), F(x, NSE_V_PRE), F(x, NSE_W_PRE), F(x, NSE_T_PRE),
+                  F(x, NSE_CELLVALUE), r[0], r[4], r[8], r[12], s, x->rhs_shape);
+  NSE_CUDA(cudaEventRecord(x->lfork, s));
+  for (int q = 0; q < 3; ++q) NSE_CUDA(cudaStreamWaitEvent(x->side[q], x->lfork, 0));
+  for (int comp = 0; comp < 4; ++comp) {
+    cudaStream_t st = comp == 0 ? s : x->side[comp - 1];
+    for (int p = 0; p < 3; ++p) {
+      const int dir = p == 0 ? 1 : ((p == 1) == (comp == 3) ? 0 : 2);
+      double *in = r[4 * comp + p], *out = r[4 * comp + p + 1];
+      LineArgs la = line_args(x, comp);
+      line_shape(x, dir, comp, la);
+      if (comp == 3 && dir == 1) {
+        la.ft = 2.0 * c.t_bot;
+        la.fb = 2.0 * c.t_top;
+      }
+      if (dir == 0) {
+        NSE_CUDA(cudaMemcpyAsync(out, in, fb, cudaMemcpyDeviceToDevice, st));
+        in = out;
+        out = nullptr;
+      }
+      launch_lines_part(dir, line_kind(dir, comp), d, in, la, x->ptab[dir][comp].as<double>(),
+                        x->slots[dir][comp].as<int>(), x->ids[dir][comp].as<int>(),
+                        x->nmasked[dir][comp], x->pmtab[dir][comp].as<double>(), st, out);
+    }
+    if (comp == 3)
+      launch_set_bc(d, nullptr, nullptr, nullptr, nullptr, r[15], c.t_bot, c.t_top, 16, st);
+    if (comp > 0) NSE_CUDA(cudaEventRecord(x->ljoin[comp - 1], st));
+  }
+  for (int q = 0; q < 2; ++q) NSE_CUDA(cudaStreamWaitEvent(s, x->ljoin[q], 0));
+  if (io.un[0]) {
+    const PoissonPlan& pp = x->pb.pp;
+    double* phi = F(x, NSE_PHI);
+    launch_div_src(d, x->rg, r[3], r[7], r[11], c.dt, phi, true, s);
+    launch_fft_fwd_x(pp, d, phi, nullptr, nullptr, nullptr, x->g, 1.0, 0, s);
+    ctx_poisson_mid(x, false);
+    launch_fft_inv_x(pp, d, phi, s);
+    launch_correct_step(d, x->rg, phi, r[3], r[7], r[11], io.un[0], io.un[1], io.un[2],
+                        io.tan[0], io.tan[1], io.tan[2], c.dt, s);
+    // v behind the upper wall keeps its value from step to step
+    const size_t row = (size_t)d.sx * sizeof(double), plane = (size_t)d.sy * sizeof(double);
+    NSE_CUDA(cudaMemcpy2DAsync(io.un[1] + d.P(0, d.ny + 1, 0), plane, io.u[1] + d.P(0, d.ny + 1, 0),
+                               plane, row, d.nz + 2, cudaMemcpyDeviceToDevice, s));
+  }
+  NSE_CUDA(cudaStreamWaitEvent(s, x->ljoin[2], 0));
+  x->l += 1;
 }
 // the step's line solve of (dir, comp) applied to the field f with zero wall
 // values (the linear part of the pass), on stream s; FP64 contexts
@@ -2936,13 +3006,13 @@ static int step_replay(nse_ctx* x, int in, int out) {
   if (cudaStreamIsCapturing(x->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
     return 0;
   void* t0 = x->f[NSE_T].p;
-  const int kind = 2 * (in != END_FULL) + (out != END_FULL);
+  const int kind = 3 * in + out;
   nse_ctx::StepGraph* g = nullptr;
   for (auto& q : x->sg)
     if (q.kind == kind && q.t == t0) g = &q;
   for (auto& q : x->sg)
     if (!g && q.kind < 0) g = &q;
-  if (!g) return 0;  // (four kinds and two buffers: never)
+  if (!g) return 0;  // (nine kinds and two buffers: never)
   g->kind = kind;
   g->t = t0;
   if (++g->uses < 2 || x->l < 2) return 0;
