@@ -204,3 +204,25 @@ def test_adjoint_in_place_matches_copied(n, every):
     for k, (a, b) in enumerate(zip(*out)):
         assert np.linalg.norm(b) > 0
         assert rel_l2(a, b) < 1e-9, k
+
+
+# The explicit terms with the tuned number of z planes per CTA (2 to 16), bit for
+# bit those of 16: every cell is computed alone.  nz below, at and past multiples.
+@pytest.mark.parametrize("prec,n", [(S.FP64, (36, 9, 5)), (S.FP64, (50, 15, 20)),
+                                    (S.FP64, (64, 62, 64)), (S.FP64, (90, 14, 25)),
+                                    (S.MIXED, (64, 24, 18)), (S.MIXED, (96, 17, 15))])
+def test_explicit_terms_with_tuned_planes(prec, n):
+    g, f, _, par = make_case(*n, seed=5)
+    out = []
+    for flags in (S.FLAG_NO_AUTOTUNE, 0):
+        cfg = S.Config(*n, par["dt"], par["Re"], par["Sc"], 50.0, g["xl"], g["yl"], g["zl"],
+                       y0=-1.0, ystretch=2.0, body_force=par["force"], t_bot=par["tbot"],
+                       t_solid=par["tsolid"], precision=prec, flags=flags)
+        with S.Context(cfg) as ctx:
+            for k in ("u", "v", "w", "T"):
+                ctx.upload(k, f[k])
+            ctx.start()
+            ctx.step(1)
+            out.append([ctx.download(k) for k in ("u_pre", "v_pre", "w_pre", "T_pre")])
+    for a, b in zip(*out):
+        assert a.any() and np.array_equal(a, b)

@@ -17,13 +17,13 @@ void launch_rhs_f32(const Dims& d, const GridDev& g, const GridRcp& rg, const St
                     const float* u_ta, const float* v_ta, const float* w_ta, float* u_pre,
                     float* v_pre, float* w_pre, float* T_pre, const double* c1, float* u_a,
                     float* v_a, float* w_a, float* u_T, bool math64, cudaStream_t s,
-                    int shape, const double* phi) {
+                    int shape, const double* phi, int kc) {
   if (math64)
     rhs_fast<float, double>(d, g, rg, sp, u, v, w, T, u_ta, v_ta, w_ta, u_pre, v_pre, w_pre,
-                            T_pre, c1, u_a, v_a, w_a, u_T, phi, s, shape);
+                            T_pre, c1, u_a, v_a, w_a, u_T, phi, s, shape, kc);
   else
     rhs_fast<float, float>(d, g, rg, sp, u, v, w, T, u_ta, v_ta, w_ta, u_pre, v_pre, w_pre,
-                           T_pre, c1, u_a, v_a, w_a, u_T, phi, s, shape);
+                           T_pre, c1, u_a, v_a, w_a, u_T, phi, s, shape, kc);
 }
 
 }  // namespace nse

@@ -15,9 +15,9 @@ void launch_rhs_fast(const Dims& d, const GridDev& g, const GridRcp& rg, const S
                      const double* u_ta, const double* v_ta, const double* w_ta,
                      double* u_pre, double* v_pre, double* w_pre, double* T_pre,
                      const double* c1, double* u_a, double* v_a, double* w_a, double* u_T,
-                     cudaStream_t s, int shape, const double* phi) {
+                     cudaStream_t s, int shape, const double* phi, int kc) {
   rhs_fast<double, double>(d, g, rg, sp, u, v, w, T, u_ta, v_ta, w_ta, u_pre, v_pre, w_pre,
-                           T_pre, c1, u_a, v_a, w_a, u_T, phi, s, shape);
+                           T_pre, c1, u_a, v_a, w_a, u_T, phi, s, shape, kc);
 }
 
 }  // namespace nse

@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(TXW * TY, MINB) k_rhs_fast(
     const H* __restrict__ U_TA, const H* __restrict__ V_TA, const H* __restrict__ W_TA,
     H* __restrict__ U_PRE, H* __restrict__ V_PRE, H* __restrict__ W_PRE, H* __restrict__ T_PRE,
     const double* __restrict__ C1, H* __restrict__ U_A, H* __restrict__ V_A,
-    H* __restrict__ W_A, H* __restrict__ U_T, const double* __restrict__ PHI,
+    H* __restrict__ W_A, H* __restrict__ U_T, const double* __restrict__ PHI, int kc,
     const __grid_constant__ RhsMaps tm) {
   extern __shared__ __align__(128) char smc[];
   char* sm = smc;
@@ -241,8 +241,8 @@ __global__ void __launch_bounds__(TXW * TY, MINB) k_rhs_fast(
   const int i0 = 1 + blockIdx.x * TXW, j0 = 1 + blockIdx.y * TY;
   const int I = i0 + threadIdx.x, J = j0 + threadIdx.y;
   const bool valid = (I <= d.nx) && (J <= d.ny);
-  const int k0 = 1 + blockIdx.z * KCHUNK;
-  const int k1 = min(d.nz, k0 + KCHUNK - 1);
+  const int k0 = 1 + blockIdx.z * kc;  // (kc <= KCHUNK planes per CTA)
+  const int k1 = min(d.nz, k0 + kc - 1);
   const int kmax = k1 + 1;  // last plane any iteration reads
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + NS * Lay::SLOT);
   const bool lead = threadIdx.x == 0 && threadIdx.y == 0;
@@ -495,7 +495,8 @@ static bool rhs_go(const Dims& d, const GridDev& g, const GridRcp& rg, const Ste
                    const double* u, const double* v, const double* w, const double* T,
                    const H* u_ta, const H* v_ta, const H* w_ta, H* u_pre, H* v_pre, H* w_pre,
                    H* T_pre, const double* c1, H* u_a, H* v_a, H* w_a, H* u_T, const double* phi,
-                   cudaStream_t s) {
+                   int kc, cudaStream_t s) {
+  if (kc < 1 || kc > KCHUNK) kc = KCHUNK;
   RhsMaps tm;
   memset(&tm, 0, sizeof(tm));
   size_t smem = (size_t)NS * RhsLay<H, TY, TM>::SLOT;
@@ -511,12 +512,12 @@ static bool rhs_go(const Dims& d, const GridDev& g, const GridRcp& rg, const Ste
     smem += NS * sizeof(uint64_t);
   }
   dim3 block(TXW, TY, 1);
-  dim3 grid((d.nx + TXW - 1) / TXW, (d.ny + TY - 1) / TY, (d.nz + KCHUNK - 1) / KCHUNK);
+  dim3 grid((d.nx + TXW - 1) / TXW, (d.ny + TY - 1) / TY, (d.nz + kc - 1) / kc);
   auto kern = k_rhs_fast<H, CT, TY, NS, MINB, TM>;
   cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   count_launch();
   kern<<<grid, block, smem, s>>>(d, g, rg, sp, u, v, w, T, u_ta, v_ta, w_ta, u_pre, v_pre, w_pre,
-                                 T_pre, c1, u_a, v_a, w_a, u_T, phi, tm);
+                                 T_pre, c1, u_a, v_a, w_a, u_T, phi, kc, tm);
   return true;
 }
 
@@ -533,15 +534,15 @@ static void rhs_fast(const Dims& d, const GridDev& g, const GridRcp& rg, const S
                      const double* u, const double* v, const double* w, const double* T,
                      const H* u_ta, const H* v_ta, const H* w_ta, H* u_pre, H* v_pre, H* w_pre,
                      H* T_pre, const double* c1, H* u_a, H* v_a, H* w_a, H* u_T,
-                     const double* phi, cudaStream_t s, int shape) {
+                     const double* phi, cudaStream_t s, int shape, int kc) {
   using Sh = RhsShape<H, CT>;
 #define NSE_RHS_GO(TY_, NS_, MB_)                                                           \
   rhs_go<H, CT, TY_, NS_, MB_>(d, g, rg, sp, u, v, w, T, u_ta, v_ta, w_ta, u_pre, v_pre,    \
-                               w_pre, T_pre, c1, u_a, v_a, w_a, u_T, phi, s)
+                               w_pre, T_pre, c1, u_a, v_a, w_a, u_T, phi, kc, s)
   constexpr int TM = sizeof(H) == 8 ? 1 : 2;
 #define NSE_RHS_TMA(TY_, NS_, MB_)                                                              \
   done = rhs_go<H, CT, TY_, NS_, MB_, TM>(d, g, rg, sp, u, v, w, T, u_ta, v_ta, w_ta, u_pre,    \
-                                          v_pre, w_pre, T_pre, c1, u_a, v_a, w_a, u_T, phi, s)
+                                          v_pre, w_pre, T_pre, c1, u_a, v_a, w_a, u_T, phi, kc, s)
   {
     bool done = false;
     if (shape == 4) NSE_RHS_TMA(4, 5, 3);

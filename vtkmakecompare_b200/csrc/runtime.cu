@@ -60,7 +60,7 @@ void launch_rhs_f32(const Dims& d, const GridDev& g, const GridRcp& rg, const St
                     const float* u_ta, const float* v_ta, const float* w_ta, float* u_pre,
                     float* v_pre, float* w_pre, float* T_pre, const double* c1, float* u_a,
                     float* v_a, float* w_a, float* u_T, bool math64, cudaStream_t s,
-                    int shape = 0, const double* phi = nullptr);
+                    int shape = 0, const double* phi = nullptr, int kc = 0);
 void launch_correct_f32(const Dims& d, const GridRcp& rg, const double* PHI, const float* ut,
                         const float* vt, const float* wt, double* p, double* u, double* v,
                         double* w, float* u_ta, float* v_ta, float* w_ta, float* u_ep2,
@@ -1474,6 +1474,7 @@ struct nse_ctx {
   bool tuned = false;
   // launch shape of the fast right-hand-side kernel (autotune_rhs)
   int rhs_shape = 0;
+  int rhs_kc = 0;  // z planes per CTA (0: the kernel's 16)
   bool rhs_tuned = false;
   // launch shape of the pipelined correction (autotune_correct)
   int corr_shape = 0;
@@ -1509,6 +1510,7 @@ unsigned long long shape_sig(const nse_ctx* x) {
     for (int comp = 0; comp < 4; ++comp) mix(x->yzshape[dir][comp]);
   for (int comp = 0; comp < 4; ++comp) mix(x->xnl[comp]);
   mix(x->rhs_shape);
+  mix(x->rhs_kc);
   mix(x->corr_shape);
   mix(x->mid_chunks);
   mix(x->pb.pp.spn_cp);
@@ -2553,7 +2555,8 @@ static void autotune_rhs(nse_ctx* x, const StepParams& sp) {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);
     if (it != g_tune.end()) {
-      x->rhs_shape = it->second;
+      x->rhs_shape = it->second % 16;
+      x->rhs_kc = it->second / 16;
       x->rhs_tuned = true;
       return;
     }
@@ -2584,21 +2587,31 @@ static void autotune_rhs(nse_ctx* x, const StepParams& sp) {
     cudaMemcpyAsync(hist[q], x->f[hid[q]].p, hb, cudaMemcpyDeviceToDevice, s);
   const double *u = F(x, NSE_U), *v = F(x, NSE_V), *w = F(x, NSE_W), *T = F(x, NSE_T);
   const double* c1 = F(x, NSE_CELLVALUE);
-  int best = 0;
+  int best = 0, best_kc = 0;
   float best_ms = 1e30f;
   const int nshape = 7;  // shapes 4-6: the TMA rings
-  for (int shape = 0; shape < nshape; ++shape) {
+  // the shapes with the kernel's 16 z planes per CTA, then the fastest with
+  // fewer.  A CTA loads its first three planes before it computes one and
+  // marches the rest serially, so many planes cost the least traffic, and
+  // few give a small grid more CTAs than the 2 x 2 x 4 .. of 16 planes and a
+  // shorter march.  Measured per launch, 16 planes against the fastest:
+  // 64^3 29.7 -> 17.4 us (4), 100x75x90 38.6 -> 29.7 (8), 128x96x128 65.2 ->
+  // 57.7 (8), 160x92x135 78.8 -> 68.6, 128^3 75.4 -> 72.0, 256x192x256 323
+  // either way (16 stays)
+  const int fewer[4] = {12, 8, 4, 2};
+  for (int cand = 0; cand < nshape + 4; ++cand) {
+    const int shape = cand < nshape ? cand : best, kc = cand < nshape ? 0 : fewer[cand - nshape];
     auto run = [&]() {
       if (x->mixed)
         launch_rhs_f32(d, x->g, x->rg, sp, u, v, w, T, F32(x, NSE_U_TA), F32(x, NSE_V_TA),
                        F32(x, NSE_W_TA), (float*)hist[0], (float*)hist[1], (float*)hist[2],
                        (float*)hist[3], c1, x->ua.as<float>(), x->va.as<float>(),
-                       x->wa.as<float>(), x->uT.as<float>(), x->math64, s, shape);
+                       x->wa.as<float>(), x->uT.as<float>(), x->math64, s, shape, nullptr, kc);
       else
         launch_rhs_fast(d, x->g, x->rg, sp, u, v, w, T, F(x, NSE_U_TA), F(x, NSE_V_TA),
                         F(x, NSE_W_TA), (double*)hist[0], (double*)hist[1], (double*)hist[2],
                         (double*)hist[3], c1, x->ua.as<double>(), x->va.as<double>(),
-                        x->wa.as<double>(), x->uT.as<double>(), s, shape);
+                        x->wa.as<double>(), x->uT.as<double>(), s, shape, nullptr, kc);
     };
     run();
     cudaEventRecord(e0, s);
@@ -2609,16 +2622,18 @@ static void autotune_rhs(nse_ctx* x, const StepParams& sp) {
         cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess && ms < best_ms) {
       best_ms = ms;
       best = shape;
+      best_kc = kc;
     }
-    tune_log(key, shape, ms);
+    tune_log(key, kc * 16 + shape, ms);
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   extra.release();
   x->rhs_shape = best;
+  x->rhs_kc = best_kc;
   x->rhs_tuned = true;
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  g_tune[key] = best;
+  g_tune[key] = best + 16 * best_kc;
 }
 
 // one time step in the mixed-precision form: FP64 state u, v, w, T, p;
@@ -2644,7 +2659,7 @@ static void ctx_step_f32(nse_ctx* x, int in, int out) {
   launch_rhs_f32(d, x->g, x->rg, sp, u, v, w, T, F32(x, NSE_U_TA), F32(x, NSE_V_TA),
                  F32(x, NSE_W_TA), F32(x, NSE_U_PRE), F32(x, NSE_V_PRE), F32(x, NSE_W_PRE),
                  F32(x, NSE_T_PRE), c1, ua, va, wa, uT, x->math64, s, x->rhs_shape,
-                 in == END_LEAN ? F(x, NSE_PHI) : nullptr);
+                 in == END_LEAN ? F(x, NSE_PHI) : nullptr, x->rhs_kc);
   refresh_line_flags(x, s);
   autotune_lines(x);
   float* fa[3] = {ua, va, wa};
@@ -2765,7 +2780,7 @@ static void ctx_step(nse_ctx* x, int in = END_FULL, int out = END_FULL) {
     launch_rhs_fast(d, x->g, x->rg, sp, u, v, w, T, F(x, NSE_U_TA), F(x, NSE_V_TA),
                     F(x, NSE_W_TA), F(x, NSE_U_PRE), F(x, NSE_V_PRE), F(x, NSE_W_PRE),
                     F(x, NSE_T_PRE), c1, ua, va, wa, uT, s, x->rhs_shape,
-                    in == END_LEAN ? F(x, NSE_PHI) : nullptr);
+                    in == END_LEAN ? F(x, NSE_PHI) : nullptr, x->rhs_kc);
   // :397 solve_u_temp: per component y, z, x line solves
   // (timed per direction: all y solves, then z, then x of the three fields;
   // the fields are independent, so this order gives the same values as
@@ -2916,7 +2931,8 @@ void ctx_step_record(nse_ctx* x, const RecordedStep& io) {
                   s);
   launch_rhs_fast(d, x->g, x->rg, sp, io.u[0], io.u[1], io.u[2], io.T, io.ta[0], io.ta[1],
                   io.ta[2], F(x, NSE_U_PRE), F(x, NSE_V_PRE), F(x, NSE_W_PRE), F(x, NSE_T_PRE),
-                  F(x, NSE_CELLVALUE), r[0], r[4], r[8], r[12], s, x->rhs_shape);
+                  F(x, NSE_CELLVALUE), r[0], r[4], r[8], r[12], s, x->rhs_shape, nullptr,
+                  x->rhs_kc);
   NSE_CUDA(cudaEventRecord(x->lfork, s));
   for (int q = 0; q < 3; ++q) NSE_CUDA(cudaStreamWaitEvent(x->side[q], x->lfork, 0));
   for (int comp = 0; comp < 4; ++comp) {
@@ -3274,6 +3290,7 @@ int nse_ctx_set_shapes(nse_ctx* x, int rhs_shape, int corr_shape) {
     return NSE_ERR_ARG;
   if (rhs_shape >= 0) {
     x->rhs_shape = rhs_shape;
+    x->rhs_kc = 0;  // a fixed shape runs with the kernel's 16 planes
     x->rhs_tuned = true;
   }
   if (corr_shape >= 0) {
