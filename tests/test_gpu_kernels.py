@@ -226,3 +226,47 @@ def test_explicit_terms_with_tuned_planes(prec, n):
             out.append([ctx.download(k) for k in ("u_pre", "v_pre", "w_pre", "T_pre")])
     for a, b in zip(*out):
         assert a.any() and np.array_equal(a, b)
+
+
+# Transforms of two register stages: every radix in either place, odd counts of
+# rows and columns off the tiles of 8, and lengths of three stages (250, 216).
+# Tolerance: that of the other transforms (test_gpu_dropin).
+@pytest.mark.parametrize("n", [(4, 1, 9), (6, 2, 10), (12, 3, 15), (20, 2, 25), (36, 3, 40),
+                               (45, 2, 54), (64, 3, 72), (80, 2, 81), (90, 3, 100),
+                               (96, 2, 108), (120, 2, 120), (128, 2, 135), (144, 2, 150),
+                               (160, 3, 160), (180, 1, 192), (192, 2, 225), (240, 2, 240),
+                               (250, 2, 216)])
+def test_transforms_of_two_stages(n):
+    nx, ny, nz = n
+    FP = rand_field(np.random.default_rng(nx), nx, ny, nz)
+    F1 = np.full((nx // 2 + 1, ny + 2, nz + 2), 7.0 + 3.0j, order="F")
+    F2 = F1.copy(order="F")
+    O.p2s(FP, nx, ny, nz, F1)
+    G.p2s(FP, F2, nx, ny, nz)
+    sl = (slice(None), slice(1, ny + 1), slice(0, nz))
+    assert rel_l2(F2[sl], F1[sl]) < 1e-14
+    F2[sl] = F1[sl]
+    assert np.array_equal(F1, F2)  # nothing else written
+    P1 = O.field(nx, ny, nz, -9.0)
+    P2 = P1.copy(order="F")
+    O.s2p(F1, nx, ny, nz, P1)
+    G.s2p(F1, P2, nx, ny, nz)
+    box = (slice(0, nx + 1), slice(1, ny + 1), slice(0, nz + 1))
+    assert rel_l2(P2[box], P1[box]) < 1e-14
+    P2[box] = P1[box]
+    assert np.array_equal(P1, P2)
+
+
+# The forward transform's division by NX NZ, a reciprocal with a correction, gives
+# the bits of the division: an impulse at the origin has the one value everywhere.
+@pytest.mark.parametrize("nx,nz", [(20, 25), (81, 9), (90, 100), (225, 240), (96, 256),
+                                   (64, 128)])
+def test_transform_divides_exactly(nx, nz):
+    v = np.random.default_rng(nx + nz).standard_normal(400) * 10.0 ** np.arange(-200, 200)
+    v[:8] = [0.0, -0.0, 5e-324, -1e-310, 3e-290, 1e290, -8e307, 2.2250738585072014e-308]
+    FP = np.zeros((nx + 2, v.size + 2, nz + 2), order="F")
+    FP[0, 1:-1, 0] = v
+    F = np.zeros((nx // 2 + 1, v.size + 2, nz + 2), complex, order="F")
+    G.p2s(FP, F, nx, v.size, nz)
+    want = np.broadcast_to((v / (nx * nz))[None, :, None], (nx // 2 + 1, v.size, nz))
+    assert np.array_equal(F[:, 1:-1, :nz].real, want)

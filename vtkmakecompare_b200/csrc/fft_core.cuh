@@ -90,6 +90,90 @@ struct DftSmall<5, CT> {
   }
 };
 
+// DFTs of length 6, 8, 9, 10, 12, 15 out of the ones above.
+// A and B coprime (the prime-factor map of Good, J. R. Stat. Soc. B 20, 1958):
+// n = (B a + A b) mod N, k = the number below N with k mod A = ka, k mod B = kb,
+// and no multiplications between the two.
+template <int A, int B, class CT>
+struct DftCoprime {
+  __device__ static void run(CT* v, bool inv) {
+    constexpr int N = A * B;
+    CT t[N];  // t[b A + ka]
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+      CT q[A];
+#pragma unroll
+      for (int a = 0; a < A; ++a) q[a] = v[(B * a + A * b) % N];
+      DftSmall<A, CT>::run(q, inv);
+#pragma unroll
+      for (int a = 0; a < A; ++a) t[b * A + a] = q[a];
+    }
+#pragma unroll
+    for (int ka = 0; ka < A; ++ka) {
+      CT q[B];
+#pragma unroll
+      for (int b = 0; b < B; ++b) q[b] = t[b * A + ka];
+      DftSmall<B, CT>::run(q, inv);
+#pragma unroll
+      for (int k = 0; k < N; ++k)
+        if (k % A == ka) v[k] = q[k % B];
+    }
+  }
+};
+template <class CT> struct DftSmall<6, CT> : DftCoprime<2, 3, CT> {};
+template <class CT> struct DftSmall<10, CT> : DftCoprime<2, 5, CT> {};
+template <class CT> struct DftSmall<12, CT> : DftCoprime<4, 3, CT> {};
+template <class CT> struct DftSmall<15, CT> : DftCoprime<3, 5, CT> {};
+template <class CT>
+struct DftSmall<8, CT> {  // n = 2a + b, k = c + 4e
+  __device__ static void run(CT* v, bool inv) {
+    using RT = typename CReal<CT>::T;
+    const RT r = (RT)0.70710678118654752440;
+    CT e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+    DftSmall<4, CT>::run(e, inv);
+    DftSmall<4, CT>::run(o, inv);
+    const CT m1 = mul_mi(o[1], inv), m3 = mul_mi(o[3], inv);
+    o[1] = mkc<CT>((o[1].x + m1.x) * r, (o[1].y + m1.y) * r);  // W8 = (1 -+ i) / sqrt 2
+    o[2] = mul_mi(o[2], inv);
+    o[3] = mkc<CT>((m3.x - o[3].x) * r, (m3.y - o[3].y) * r);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      v[c] = cadd(e[c], o[c]);
+      v[c + 4] = csub(e[c], o[c]);
+    }
+  }
+};
+template <class CT>
+struct DftSmall<9, CT> {  // n = 3a + b, k = c + 3e
+  __device__ static void run(CT* v, bool inv) {
+    using RT = typename CReal<CT>::T;
+    const RT c1 = (RT)0.76604444311897803520, s1 = (RT)0.64278760968653932632;
+    const RT c2 = (RT)0.17364817766693034885, s2 = (RT)0.98480775301220805937;
+    const RT c4 = (RT)-0.93969262078590838405, s4 = (RT)0.34202014332566873304;
+    const CT w1 = mkc<CT>(c1, inv ? s1 : -s1), w2 = mkc<CT>(c2, inv ? s2 : -s2),
+             w4 = mkc<CT>(c4, inv ? s4 : -s4);
+    CT q[3][3];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      q[b][0] = v[b];
+      q[b][1] = v[b + 3];
+      q[b][2] = v[b + 6];
+      DftSmall<3, CT>::run(q[b], inv);
+    }
+    q[1][1] = cmul(q[1][1], w1);
+    q[1][2] = cmul(q[1][2], w2);
+    q[2][1] = cmul(q[2][1], w2);
+    q[2][2] = cmul(q[2][2], w4);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      CT t[3] = {q[0][c], q[1][c], q[2][c]};
+      DftSmall<3, CT>::run(t, inv);
+#pragma unroll
+      for (int e = 0; e < 3; ++e) v[c + 3 * e] = t[e];
+    }
+  }
+};
+
 // ------------------------------------------- register FFT of length 256 --
 // N = 256 = 16 x 16: with n = 16a + b and k = c + 16e,
 //   X[c + 16e] = sum_b W256^(bc) W16^(be) [ sum_a x[16a + b] W16^(ac) ].
@@ -138,6 +222,11 @@ __device__ __forceinline__ void dft16(CT (&v)[16], bool inv) {
     for (int e1 = 0; e1 < 4; ++e1) v[e0 + 4 * e1] = q[e1];
   }
 }
+
+template <class CT>
+struct DftSmall<16, CT> {
+  __device__ static void run(CT* v, bool inv) { dft16(*reinterpret_cast<CT(*)[16]>(v), inv); }
+};
 
 // the inner half of the transform on thread b: DFT over a, then W256^(bc)
 template <class CT>

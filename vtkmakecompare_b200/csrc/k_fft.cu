@@ -162,6 +162,26 @@ __global__ void __launch_bounds__(128) k_div_src(Dims d, FwdSrc<S> q, double* __
   out[d.P(i, J, k)] = div_rhs<WRAP>(d, q, I, J, K);
 }
 
+// source modes 1 and 2 at the periodic image of sample (i, k)
+template <class S>
+__device__ __forceinline__ double rhs_sample(const Dims& d, const FwdSrc<S>& q, int src_mode,
+                                             int i, int J, int k) {
+  const int I = (i == 0) ? d.nx : i, K = (k == 0) ? d.nz : k;
+  const double val = div_rhs(d, q, I, J, K);
+  if (src_mode != 2) return val;
+  // minus the operator the spectral solve inverts (mkp.f:56-84): periodic
+  // second differences in x and z, AC rows in y with the Neumann ghosts of PHIBC
+  const double* ph = q.phi;
+  const long c = d.P(I, J, K);
+  const int ny = d.ny;
+  const double p0 = ph[c];
+  const double lx = (ph[c + 1] - 2.0 * p0 + ph[c - 1]) * q.rdx2;
+  const double lz = (ph[c + d.sy] - 2.0 * p0 + ph[c - d.sy]) * q.rdz2;
+  const double ly = q.AC[J - 1] * ph[c - d.sx] + q.AC[J - 1 + ny] * p0 +
+                    q.AC[J - 1 + 2 * ny] * ph[c + d.sx];
+  return val - (lx + ly + lz);
+}
+
 // ------------------------------------------------------------- x forward --
 // CTA: plane J (1..ny) and `npair` row pairs starting at row 2*npair*blockIdx.y
 template <class CT, class S>
@@ -175,7 +195,7 @@ __global__ void k_fft_fwd_x(FFTShape sh, int npair, Dims d, SpecViewT<CT> sv, Fw
   CT* b = smem + (long)npair * N;
   const int J = 1 + sv.j0 + blockIdx.x;
   const int kk0 = 2 * npair * blockIdx.y;
-  const int nx = d.nx, ny = d.ny, nz = d.nz;
+  const int nz = d.nz;
   for (int t = threadIdx.x; t < npair * N; t += blockDim.x) {
     int pr = t / N, i = t - pr * N;
     int ka = kk0 + 2 * pr, kb = ka + 1;
@@ -184,28 +204,8 @@ __global__ void k_fft_fwd_x(FFTShape sh, int npair, Dims d, SpecViewT<CT> sv, Fw
       if (ka < nz) va = (double)q.FP[d.P(i, J, ka)];
       if (kb < nz) vb = (double)q.FP[d.P(i, J, kb)];
     } else {
-      // right-hand side at the periodic image of sample (i,k)
-      int I = (i == 0) ? nx : i;
-      for (int h = 0; h < 2; ++h) {
-        int kq = h ? kb : ka;
-        if (kq >= nz) continue;
-        int K = (kq == 0) ? nz : kq;
-        double val = div_rhs(d, q, I, J, K);
-        if (src_mode == 2) {
-          // minus the operator the spectral solve inverts (mkp.f:56-84):
-          // periodic second differences in x and z, AC rows in y with the
-          // Neumann ghosts of PHIBC
-          const double* ph = q.phi;
-          long c = d.P(I, J, K);
-          const double p0 = ph[c];
-          const double lx = (ph[c + 1] - 2.0 * p0 + ph[c - 1]) * q.rdx2;
-          const double lz = (ph[c + d.sy] - 2.0 * p0 + ph[c - d.sy]) * q.rdz2;
-          const double ly = q.AC[J - 1] * ph[c - d.sx] + q.AC[J - 1 + ny] * p0 +
-                            q.AC[J - 1 + 2 * ny] * ph[c + d.sx];
-          val = val - (lx + ly + lz);
-        }
-        if (h) vb = val; else va = val;
-      }
+      if (ka < nz) va = rhs_sample(d, q, src_mode, i, J, ka);
+      if (kb < nz) vb = rhs_sample(d, q, src_mode, i, J, kb);
     }
     a[t] = mkc<CT>((RT)va, (RT)vb);
   }
@@ -302,6 +302,253 @@ __global__ void k_fft_inv_x(FFTShape sh, int npair, Dims d, SpecViewT<CT> sv, do
       FP[c] = accumulate ? FP[c] + (double)z.y : (double)z.y;
     }
   }
+}
+
+// ------------------------------------------------- two register stages --
+// N = R1 x R2, both at most 16: two Stockham stages with a whole DFT of R1 (then
+// R2) values in a thread's registers, the first reading and the last writing
+// global memory (the z pass) and one exchange through shared memory between
+// them.  On the small and middle grids, whose spectrum stays in L2, a pass is
+// bound by the length of its chain of barriers, exchanges and index divisions:
+// the radix-4/2/3/5 stages above have four or five of each for N = 64 .. 135.
+// One pass, stages above -> here (us, events around each): 64^3 z 9 -> 5, x back
+// 8 -> 8; 100x75x90 z 16 -> 8, x back 11 -> 9; a whole lean step of 64^3 83 ->
+// 71 us, 100x75x90 160 -> 147, 128x96x128 255 -> 225.  Lengths without two such
+// factors (125, 200, 216, 243, 250 and the powers above 256) keep the stages.
+template <class F>
+__device__ __forceinline__ void with_radix(int R, F f) {
+  switch (R) {
+    case 2: f(std::integral_constant<int, 2>{}); break;
+    case 3: f(std::integral_constant<int, 3>{}); break;
+    case 4: f(std::integral_constant<int, 4>{}); break;
+    case 5: f(std::integral_constant<int, 5>{}); break;
+    case 6: f(std::integral_constant<int, 6>{}); break;
+    case 8: f(std::integral_constant<int, 8>{}); break;
+    case 9: f(std::integral_constant<int, 9>{}); break;
+    case 10: f(std::integral_constant<int, 10>{}); break;
+    case 12: f(std::integral_constant<int, 12>{}); break;
+    case 15: f(std::integral_constant<int, 15>{}); break;
+    default: f(std::integral_constant<int, 16>{}); break;
+  }
+}
+
+// v *= W_N^(r j) of the second stage (table tw of N), then the DFT
+template <int R, bool INV, class CT>
+__device__ __forceinline__ void second_dft(CT* v, int j, const CT* __restrict__ tw) {
+#pragma unroll
+  for (int r = 1; r < R; ++r) {
+    CT w = __ldg(tw + r * j);
+    if (INV) w.y = -w.y;
+    v[r] = cmul(v[r], w);
+  }
+  DftSmall<R, CT>::run(v, INV);
+}
+
+// x / d for a whole number d > 0 with r = 1/d rounded: x r corrected by its
+// remainder is the rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990: r is
+// rounded and d's significand is not all ones), the same bits without a division
+// sequence per value; `apart` when it is tiny, huge or not a number (the
+// exponent field of q outside 2^-900 .. 2^900)
+__device__ __forceinline__ double quotient(double x, double d, double r, bool& apart) {
+  const double q = x * r;
+  const bool zero = x == 0.0;
+  const unsigned e = (unsigned)(__double2hiint(q) >> 20) & 0x7ffu;
+  apart |= !zero && e - 123u > 1800u;
+  return zero ? q : __fma_rn(__fma_rn(-q, d, x), r, q);
+}
+__device__ __forceinline__ float quotient(float x, float d, float, bool&) { return x / d; }
+
+// z pass: a CTA holds F2_W adjacent kx columns of plane jj; thread (c, j) runs
+// the butterfly j of column c in both stages.  NORM as in k_fft256_z; the values
+// that need a division after all are divided apart, out of the common path.
+constexpr int F2_W = 8;
+template <class CT, int NORM>
+__global__ void __launch_bounds__(F2_W * 16) k_fft2_z(int R1, int R2, int H, SpecViewT<CT> sv,
+                                                      const CT* __restrict__ tw, double nrm,
+                                                      double rnrm) {
+  constexpr bool INV = NORM == 0;
+  using RT = typename CReal<CT>::T;
+  extern __shared__ __align__(16) char fsm[];
+  CT* sm = reinterpret_cast<CT*>(fsm);  // [N][F2_W]
+  const int c = threadIdx.x % F2_W, j = threadIdx.x / F2_W;
+  const int kx = blockIdx.x * F2_W + c;
+  const bool ok = kx < H;
+  CT* col = sv.base + kx + sv.sj * (sv.j0 + (int)blockIdx.y);
+  if (ok && j < R2)
+    with_radix(R1, [&](auto rc) {
+      constexpr int R = rc();
+      CT v[R];
+      const CT* p = col + sv.sk * j;
+      const long st = sv.sk * R2;
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = p[st * r];
+      DftSmall<R, CT>::run(v, INV);
+#pragma unroll
+      for (int r = 0; r < R; ++r) sm[(j * R + r) * F2_W + c] = v[r];
+    });
+  __syncthreads();
+  if (ok && j < R1)
+    with_radix(R2, [&](auto rc) {
+      constexpr int R = rc();
+      CT v[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = sm[(j + r * R1) * F2_W + c];
+      second_dft<R, INV>(v, j, tw);
+      CT* p = col + sv.sk * j;
+      const long st = sv.sk * R1;
+      const RT rn = (RT)nrm, rq = (RT)rnrm;
+      bool apart = false;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        CT w = v[r];
+        if (NORM == 1) w = mkc<CT>(w.x * rq, w.y * rq);
+        if (NORM == 2) w = mkc<CT>(quotient(w.x, rn, rq, apart), quotient(w.y, rn, rq, apart));
+        p[st * r] = w;
+      }
+      if (NORM == 2 && apart) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) p[st * r] = mkc<CT>(v[r].x / rn, v[r].y / rn);
+      }
+    });
+}
+
+// x passes: T = max(R1, R2) threads per row pair (packed as a + i b), npair
+// pairs of plane J per CTA; stage one leaves row j of R1 values at pitch R1 | 1,
+// so neither side of the exchange meets a bank twice
+constexpr int F2_XT = 64;  // threads a CTA holds at most
+struct Fft2X {
+  int R1, R2, T, npair, pitch;  // pitch: complex values of shared memory per pair
+};
+template <class CT, class S, bool SAMPLES>
+__global__ void __launch_bounds__(F2_XT) k_fft2_fwd_x(Fft2X x, Dims d, SpecViewT<CT> sv,
+                                                      FwdSrc<S> q, int src_mode,
+                                                      const CT* __restrict__ tw) {
+  using RT = typename CReal<CT>::T;
+  extern __shared__ __align__(16) char fsm[];
+  const int R1 = x.R1, R2 = x.R2, N = R1 * R2, H = N / 2 + 1, Q1 = R1 | 1;
+  const int pr = threadIdx.x / x.T, j = threadIdx.x - pr * x.T;
+  CT* sm = reinterpret_cast<CT*>(fsm) + pr * x.pitch;
+  const int J = 1 + sv.j0 + blockIdx.x;
+  const int ka = 2 * (x.npair * blockIdx.y + pr), kb = ka + 1;
+  const bool ok = pr < x.npair && ka < d.nz;
+  const bool two = kb < d.nz;
+  if (ok && j < R2)
+    with_radix(R1, [&](auto rc) {
+      constexpr int R = rc();
+      CT v[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int i = j + r * R2;
+        double va, vb = 0.0;
+        if (SAMPLES) {
+          va = (double)q.FP[d.P(i, J, ka)];
+          if (two) vb = (double)q.FP[d.P(i, J, kb)];
+        } else {
+          va = rhs_sample(d, q, src_mode, i, J, ka);
+          if (two) vb = rhs_sample(d, q, src_mode, i, J, kb);
+        }
+        v[r] = mkc<CT>((RT)va, (RT)vb);
+      }
+      DftSmall<R, CT>::run(v, false);
+#pragma unroll
+      for (int r = 0; r < R; ++r) sm[j * Q1 + r] = v[r];
+    });
+  __syncthreads();
+  // the barrier between the reads and the natural order written over them is
+  // reached by every thread: the values wait in w
+  CT w[16];
+  if (ok && j < R1)
+    with_radix(R2, [&](auto rc) {
+      constexpr int R = rc();
+#pragma unroll
+      for (int r = 0; r < R; ++r) w[r] = sm[r * Q1 + j];
+      second_dft<R, false>(w, j, tw);
+    });
+  __syncthreads();
+  if (ok && j < R1) {
+#pragma unroll
+    for (int r = 0; r < 16; ++r)
+      if (r < R2) sm[j + r * R1] = w[r];
+  }
+  __syncthreads();
+  if (!ok) return;
+  CT* oa = sv.base + sv.sj * (J - 1) + sv.sk * ka;
+#pragma unroll
+  for (int e = 0; e <= 8; ++e) {
+    const int kx = j + e * x.T;
+    if (kx >= H) break;
+    const CT Z = sm[kx], Zr = sm[kx == 0 ? 0 : N - kx];
+    oa[kx] = mkc<CT>((Z.x + Zr.x) * RT(0.5), (Z.y - Zr.y) * RT(0.5));
+    if (two) oa[sv.sk + kx] = mkc<CT>((Z.y + Zr.y) * RT(0.5), (Zr.x - Z.x) * RT(0.5));
+  }
+}
+
+template <class CT, bool ACC>
+__global__ void __launch_bounds__(F2_XT) k_fft2_inv_x(Fft2X x, Dims d, SpecViewT<CT> sv,
+                                                      double* FP, const CT* __restrict__ tw) {
+  using RT = typename CReal<CT>::T;
+  extern __shared__ __align__(16) char fsm[];
+  const int R1 = x.R1, R2 = x.R2, N = R1 * R2, H = N / 2 + 1, Q1 = R1 | 1;
+  const int pr = threadIdx.x / x.T, j = threadIdx.x - pr * x.T;
+  CT* sm = reinterpret_cast<CT*>(fsm) + pr * x.pitch;
+  const int J = 1 + sv.j0 + blockIdx.x;
+  const int ka = 2 * (x.npair * blockIdx.y + pr), kb = ka + 1;
+  const bool ok = pr < x.npair && ka < d.nz;
+  const bool two = kb < d.nz;
+  if (ok) {
+    const CT* ia = sv.base + sv.sj * (J - 1) + sv.sk * ka;
+#pragma unroll
+    for (int e = 0; e <= 8; ++e) {
+      const int kx = j + e * x.T;
+      if (kx >= H) break;
+      CT A = ia[kx], B = mkc<CT>(RT(0), RT(0));
+      if (two) B = ia[sv.sk + kx];
+      if (kx == 0 || 2 * kx == N) { A.y = RT(0); B.y = RT(0); }
+      // Z = A + iB at kx, conj(A) + i conj(B) at N - kx
+      sm[kx] = mkc<CT>(A.x - B.y, A.y + B.x);
+      if (kx > 0 && 2 * kx < N) sm[N - kx] = mkc<CT>(A.x + B.y, B.x - A.y);
+    }
+  }
+  __syncthreads();
+  CT w[16];
+  if (ok && j < R2)
+    with_radix(R1, [&](auto rc) {
+      constexpr int R = rc();
+#pragma unroll
+      for (int r = 0; r < R; ++r) w[r] = sm[j + r * R2];
+      DftSmall<R, CT>::run(w, true);
+    });
+  __syncthreads();
+  if (ok && j < R2) {
+#pragma unroll
+    for (int r = 0; r < 16; ++r)
+      if (r < R1) sm[j * Q1 + r] = w[r];
+  }
+  __syncthreads();
+  if (ok && j < R1)
+    with_radix(R2, [&](auto rc) {
+      constexpr int R = rc();
+      CT v[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = sm[r * Q1 + j];
+      second_dft<R, true>(v, j, tw);
+      double* oa = FP + d.P(j, J, ka);
+      double* ob = oa + d.sy;
+      double* oz = oa + d.nz * d.sy;  // the S2P wrap (k_fft_inv_x)
+      auto put = [&](int i, CT z) {
+        double a = (double)z.x, b = (double)z.y;
+        if (ACC) a = oa[i] + a;
+        oa[i] = a;
+        if (ka == 0) oz[i] = a;
+        if (two) {
+          if (ACC) b = ob[i] + b;
+          ob[i] = b;
+        }
+      };
+#pragma unroll
+      for (int r = 0; r < R; ++r) put(r * R1, v[r]);
+      if (j == 0) put(N, v[0]);
+    });
 }
 
 // x forward, N = 256: a half-warp transforms one row pair (two real rows
@@ -1226,6 +1473,27 @@ template <> const float2* twz_of<float2>(const PoissonPlan& pp) {
   return reinterpret_cast<const float2*>(pp.twz_f);
 }
 
+// N = R1 x R2 of the two-stage transforms, the two as equal as they come; false
+// when N has no such factors (then the radix-4/2/3/5 stages)
+static bool two_factors(int N, int* R1, int* R2) {
+  *R1 = 0;
+  for (int a : {2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16})
+    for (int b : {2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16})
+      if (a * b == N && a <= b) { *R1 = a; *R2 = b; }
+  return *R1 != 0;
+}
+// (the threads of a pair touch R2 adjacent samples on the way in and R1 on the
+// way out, so the longer factor goes where the samples are)
+static bool fft2_x(const PoissonPlan& pp, Fft2X* x, dim3* grid, int nj, bool inverse) {
+  if (!two_factors(pp.nx, &x->R1, &x->R2)) return false;
+  x->T = x->R2;
+  if (inverse) std::swap(x->R1, x->R2);
+  x->npair = F2_XT / x->T;
+  x->pitch = x->R2 * (x->R1 | 1);
+  *grid = dim3(nj, ((pp.nz + 1) / 2 + x->npair - 1) / x->npair);
+  return true;
+}
+
 static int row_pairs(const PoissonPlan& pp) {
   int npair = 1024 / pp.nx;
   if (npair < 1) npair = 1;
@@ -1250,9 +1518,21 @@ static void fwd_x(const PoissonPlan& pp, const Dims& d, const FwdSrc<S>& q, int 
       k_fft256_fwd_x<CT, S, 2><<<grid, 128, 0, s>>>(d, sv, q, twx_of<CT>(pp));
     return;
   }
+  Fft2X x2;
+  dim3 grid;
+  if (fft2_x(pp, &x2, &grid, nj, false)) {
+    const size_t sm2 = (size_t)x2.npair * x2.pitch * sizeof(CT);
+    count_launch();
+    if (src_mode == 0)
+      k_fft2_fwd_x<CT, S, true><<<grid, F2_XT, sm2, s>>>(x2, d, sv, q, 0, twx_of<CT>(pp));
+    else
+      k_fft2_fwd_x<CT, S, false><<<grid, F2_XT, sm2, s>>>(x2, d, sv, q, src_mode,
+                                                          twx_of<CT>(pp));
+    return;
+  }
   FFTShape sh = make_shape(pp.nx);
   int npair = row_pairs(pp);
-  dim3 grid(nj, (pp.nz + 2 * npair - 1) / (2 * npair));
+  grid = dim3(nj, (pp.nz + 2 * npair - 1) / (2 * npair));
   size_t sm = 2 * (size_t)npair * pp.nx * sizeof(CT);
   smem_optin((const void*)k_fft_fwd_x<CT, S>, sm);
   count_launch();
@@ -1317,6 +1597,18 @@ static void fft_z(const PoissonPlan& pp, bool inverse, cudaStream_t s, int j0 = 
     }
     return;
   }
+  const double nrm = (double)pp.nx * (double)pp.nz;
+  int e2 = 0, R1, R2;
+  const bool pow2 = !inverse && frexp(nrm, &e2) == 0.5;
+  if (two_factors(pp.nz, &R1, &R2)) {
+    dim3 grid((pp.H + F2_W - 1) / F2_W, nj);
+    const int nt = F2_W * R2;
+    const size_t sm = (size_t)F2_W * pp.nz * sizeof(CT);
+    count_launch();
+    auto kern = inverse ? k_fft2_z<CT, 0> : pow2 ? k_fft2_z<CT, 1> : k_fft2_z<CT, 2>;
+    kern<<<grid, nt, sm, s>>>(R1, R2, pp.H, sv, twz_of<CT>(pp), nrm, 1.0 / nrm);
+    return;
+  }
   FFTShape sh = make_shape(pp.nz);
   int W = 2048 / pp.nz;
   if (W < 1) W = 1;
@@ -1325,9 +1617,6 @@ static void fft_z(const PoissonPlan& pp, bool inverse, cudaStream_t s, int j0 = 
   size_t sm = 2 * (size_t)W * (pp.nz + 1) * sizeof(CT);
   smem_optin((const void*)k_fft_z<CT>, sm);
   count_launch();
-  const double nrm = (double)pp.nx * (double)pp.nz;
-  int e2 = 0;
-  const bool pow2 = !inverse && frexp(nrm, &e2) == 0.5;
   k_fft_z<CT><<<grid, fft_threads(W * pp.nz), sm, s>>>(sh, W, pp.H, sv, twz_of<CT>(pp),
                                                        inverse ? 1 : 0, pow2 ? 1.0 / nrm : nrm,
                                                        pow2 ? 1 : 0);
@@ -1527,9 +1816,18 @@ static void inv_x(const PoissonPlan& pp, const Dims& d, double* FP, bool accumul
     k_fft256_inv_x<CT><<<grid, 128, 0, s>>>(d, sv, FP, twx_of<CT>(pp), accumulate ? 1 : 0);
     return;
   }
+  Fft2X x2;
+  dim3 grid;
+  if (fft2_x(pp, &x2, &grid, nj, true)) {
+    count_launch();
+    auto kern = accumulate ? k_fft2_inv_x<CT, true> : k_fft2_inv_x<CT, false>;
+    kern<<<grid, F2_XT, (size_t)x2.npair * x2.pitch * sizeof(CT), s>>>(x2, d, sv, FP,
+                                                                       twx_of<CT>(pp));
+    return;
+  }
   FFTShape sh = make_shape(pp.nx);
   int npair = row_pairs(pp);
-  dim3 grid(nj, (pp.nz + 2 * npair - 1) / (2 * npair));
+  grid = dim3(nj, (pp.nz + 2 * npair - 1) / (2 * npair));
   size_t sm = 2 * (size_t)npair * pp.nx * sizeof(CT);
   smem_optin((const void*)k_fft_inv_x<CT>, sm);
   count_launch();
