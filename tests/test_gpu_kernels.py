@@ -270,3 +270,21 @@ def test_transform_divides_exactly(nx, nz):
     G.p2s(FP, F, nx, v.size, nz)
     want = np.broadcast_to((v / (nx * nz))[None, :, None], (nx // 2 + 1, v.size, nz))
     assert np.array_equal(F[:, 1:-1, :nz].real, want)
+
+
+# SPN on tiles: every remainder of the rows its sweeps and the mean mode's march run
+# ahead (from the least number of rows that split, 4), against the form that loads
+# each row as it needs it: same bits.  Tiles of 12 columns, whole and partial.
+@pytest.mark.parametrize("ny", [4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 17, 18, 19, 20, 27, 256])
+def test_spn_tiles_of_any_height(ny):
+    nx, nz = (45, 5) if ny % 2 else (64, 6)
+    rhs = rand_field(np.random.default_rng(ny), nx, ny, nz)
+    out = []
+    for form in (0, S.FLAG_SPN_CPASYNC):
+        cfg = S.Config(nx, ny, nz, 1.0, 1.0, 1.0, 0.0, 2.0, 2.0, 3.0, y0=-1.0, ystretch=2.0,
+                       flags=S.FLAG_NO_AUTOTUNE | form)
+        with S.Context(cfg) as ctx:
+            ctx.upload("phi", rhs)
+            ctx.poisson()
+            out.append(ctx.download("phi"))
+    assert out[0].any() and np.array_equal(out[0], out[1])

@@ -1218,70 +1218,123 @@ __global__ void __launch_bounds__(64) k_spn_babe(int H, int ny, int nz, int m, R
 // leave by one TMA store.  Lane = 16 half + kxl (kxl < 12): each lane runs the
 // re and im recurrences of its half (half 0: rows 0..m-1 downwards, half 1:
 // rows ny-1..m upwards), which share the pivots; a half-warp's accesses to a
-// row are contiguous (no bank conflicts).  The row loads run one block of
-// SPN_U rows ahead of the recurrence (register double buffering), so the
-// shared-memory and L1 latencies overlap the dependent FMA chain.  Four
-// 54 KB tiles fit an SM at ny = 192.  Columns kx >= H are outside both tensor
+// row are contiguous (no bank conflicts).  The row loads run SPN_U rows ahead of
+// the recurrence, so the shared-memory latencies overlap the dependent FMA chain.
+// The coefficients are copied beside the tile while it is under way: from L1 each
+// row waited for them, and each line of 16 rows for L2.  Columns kx >= H are outside both tensor
 // maps (zero-filled on load, not stored); columns kx0 + ... >= kx1 (the end of
-// a kx slice) are not solved and go back unchanged.  The mean mode's lane
-// marches SP0B on the tile's kx = 0 column.  Forward solve only (the
+// a kx slice) are not solved and go back unchanged.  The mean mode's two lanes
+// march SP0B on the tile's kx = 0 column.  Forward solve only (the
 // transposed solve keeps k_spn_babe).  Bounded waits: a TMA copy that does
 // not arrive sets g_spn2_wait_err and the tile is not stored.
-constexpr int SPN_KT = 12, SPN_U = 8;
+constexpr int SPN_KT = 12, SPN_U = 4;
 // One sweep of the two-ended recurrence over n rows of a lane's half: row j
 // of the sweep is v[j sv], w[j sv], c[j sc].  DOWN: elimination y(j) =
 // (d(j) - c(j) y(j-1)) w(j); else back substitution x(j) = y(j) - c(j) w(j)
-// x(j-1); each result replaces the row's value.  Loads run one block of
-// SPN_U rows ahead of the recurrence (two register buffers), so their
-// shared-memory and L1 latencies overlap the dependent chain.
+// x(j-1); each result replaces the row's value.  A row's registers take the
+// row SPN_U further on as soon as they are used, and the addresses step by
+// additions: 44 cycles a row of one warp alone, 56 with two buffers of 8 rows
+// filled in turn and their last rows loaded as they are needed.
 template <bool DOWN>
 __device__ __forceinline__ void spn_sweep(double2* v, const double* w, const double* c, int sv,
                                           int sc, int n, double2& y) {
   constexpr int U = SPN_U;
-  double2 dA[U], dB[U];
-  double wA[U], wB[U], cA[U], cB[U];
-  const int nb = n / U;
-  auto load = [&](int b, double2* dd, double* ww, double* cc) {
-    const double2* pv = v + b * U * sv;
-    const double* pw = w + b * U * sv;
-    const double* pc = c + b * U * sc;
-#pragma unroll
-    for (int k = 0; k < U; ++k) {
-      dd[k] = pv[k * sv];
-      ww[k] = pw[k * sv];
-      cc[k] = __ldg(pc + k * sc);
-    }
+  double2 d[U];
+  double wr[U], cr[U];
+  double2* o = v;
+  auto load = [&](int k) {
+    d[k] = *v;
+    wr[k] = *w;
+    cr[k] = *c;
+    v += sv;
+    w += sv;
+    c += sc;
   };
-  auto row = [&](double2 d, double cf, double wr) {
+  auto row = [&](int k) {
     if (DOWN) {
-      y.x = spn_down(false, d.x, cf, y.x, wr);
-      y.y = spn_down(false, d.y, cf, y.y, wr);
+      y.x = spn_down(false, d[k].x, cr[k], y.x, wr[k]);
+      y.y = spn_down(false, d[k].y, cr[k], y.y, wr[k]);
     } else {
-      y.x = spn_up(d.x, cf, wr, y.x);
-      y.y = spn_up(d.y, cf, wr, y.y);
+      y.x = spn_up(d[k].x, cr[k], wr[k], y.x);
+      y.y = spn_up(d[k].y, cr[k], wr[k], y.y);
     }
+    *o = y;
+    o += sv;
   };
-  auto step = [&](int b, const double2* dd, const double* ww, const double* cc) {
-    double2* pv = v + b * U * sv;
+#pragma unroll
+  for (int k = 0; k < U; ++k)
+    if (k < n) load(k);
+  int j = 0;
+  for (; j + 2 * U <= n; j += U) {
 #pragma unroll
     for (int k = 0; k < U; ++k) {
-      row(dd[k], cc[k], ww[k]);
-      pv[k * sv] = y;
+      row(k);
+      load(k);
     }
+  }
+  const int rest = n - j;  // below 2 U
+#pragma unroll
+  for (int k = 0; k < U; ++k)
+    if (k < rest) {
+      row(k);
+      if (k + U < rest) load(k);
+    }
+#pragma unroll
+  for (int k = 0; k < U; ++k)
+    if (k + U < rest) row(k);
+}
+
+// SP0B's forward march (mkp.f:271-288; phi(1) = 0) on one component of the tile's
+// kx = 0 column, row r at v[S r], each solved value over its right-hand side.
+// One lane marches all ny rows while the others take half as many each, so on
+// small grids this chain sets the length of the launch: the rows run U ahead of
+// it as in spn_sweep, re and im on two lanes and the coefficients in shared
+// memory (31 cycles a row alone; 168 with both components on a lane, the
+// coefficients from L2 and the reciprocal's presence tested in each row).
+template <int S>
+__device__ __forceinline__ void sp0b_march(double* v, const double* AC1, const double* AC2,
+                                           const double* rAC3, int ny) {
+  constexpr int U = 4;
+  const int n = ny - 1;  // row j = 0 .. n-1: the right-hand side at j, the value at j + 1
+  double d[U], a1[U], a2[U], a3[U], pm = 0.0, pc = 0.0;
+  auto load = [&](int k, int r) {
+    d[k] = v[S * r];
+    a1[k] = AC1[r];
+    a2[k] = AC2[r];
+    a3[k] = rAC3[r];
   };
-  if (nb > 0) load(0, dA, wA, cA);
-  int b = 0;
-  for (; b + 2 <= nb; b += 2) {
-    load(b + 1, dB, wB, cB);
-    step(b, dA, wA, cA);
-    if (b + 2 < nb) load(b + 2, dA, wA, cA);
-    step(b + 1, dB, wB, cB);
+  auto row = [&](int k, int r) {
+    const double pn = sp0b_row(d[k], pm, pc, a1[k], a2[k], a3[k]);
+    v[S * (r + 1)] = pn;
+    pm = pc;
+    pc = pn;
+  };
+#pragma unroll
+  for (int k = 0; k < U; ++k)
+    if (k < n) load(k, k);
+  v[0] = 0.0;
+  int j = 0;
+  for (; j + 2 * U <= n; j += U) {
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      row(k, k);
+      load(k, k + U);
+    }
+    v += S * U;
+    AC1 += U;
+    AC2 += U;
+    rAC3 += U;
   }
-  if (b < nb) step(b, dA, wA, cA);
-  for (int j = nb * U; j < n; ++j) {
-    row(v[j * sv], __ldg(c + j * sc), w[j * sv]);
-    v[j * sv] = y;
-  }
+  const int rest = n - j;
+#pragma unroll
+  for (int k = 0; k < U; ++k)
+    if (k < rest) {
+      row(k, k);
+      if (k + U < rest) load(k, k + U);
+    }
+#pragma unroll
+  for (int k = 0; k < U; ++k)
+    if (k + U < rest) row(k, k + U);
 }
 
 __device__ int g_spn2_wait_err = 0;
@@ -1290,7 +1343,7 @@ __host__ __device__ inline size_t spn_tile_piv_off(int ny) {
   return ((size_t)ny * 2 * SPN_KT * sizeof(double) + 127) & ~(size_t)127;
 }
 __host__ __device__ inline size_t spn_tile_smem(int ny) {
-  return spn_tile_piv_off(ny) + (size_t)ny * SPN_KT * sizeof(double) + 16;
+  return spn_tile_piv_off(ny) + (size_t)ny * (SPN_KT + 4) * sizeof(double) + 16;
 }
 
 __global__ void __launch_bounds__(32) k_spn_babe_tma(const __grid_constant__ CUtensorMap tv,
@@ -1303,7 +1356,8 @@ __global__ void __launch_bounds__(32) k_spn_babe_tma(const __grid_constant__ CUt
   extern __shared__ __align__(128) unsigned char sbt_sm[];
   double* vs = reinterpret_cast<double*>(sbt_sm);                        // [ny][2 KT]
   double* ws = reinterpret_cast<double*>(sbt_sm + spn_tile_piv_off(ny));  // [ny][KT]
-  uint64_t* bar = reinterpret_cast<uint64_t*>(ws + (size_t)ny * KT);
+  double* cs = ws + (size_t)ny * KT;  // AC1, AC2, AC3, 1/AC3
+  uint64_t* bar = reinterpret_cast<uint64_t*>(cs + 4 * (size_t)ny);
   const int lane = threadIdx.x;
   const int kb = kx0 + KT * blockIdx.x, kz = blockIdx.y;
   const bool aligned = ((reinterpret_cast<uintptr_t>(&tv) & 63) == 0) &&
@@ -1320,6 +1374,8 @@ __global__ void __launch_bounds__(32) k_spn_babe_tma(const __grid_constant__ CUt
     tma_load_3d(vs, &tv, 2 * kb, 0, kz, bar);
     tma_load_3d(ws, &tp, kb, 0, kz, bar);
   }
+  for (int r = lane; r < 3 * ny; r += 32) cs[r] = __ldg(AC + r);
+  for (int r = lane; r < ny; r += 32) cs[3 * ny + r] = __ldg(rAC3 + r);
   __syncwarp();
   if (!tma_wait(bar, 0)) {
     // the copies of this tile did not arrive: record it, give them one more
@@ -1332,28 +1388,12 @@ __global__ void __launch_bounds__(32) k_spn_babe_tma(const __grid_constant__ CUt
   const int kx = kb + kxl;
   const bool mean = (kx == 0 && kz == 0);
   const bool valid = kxl < KT && kx < kx1 && kx < H && !mean;
-  const double* AC1 = AC;
-  const double* AC2 = AC + ny;
-  const double* AC3 = AC + 2 * ny;
+  const double* AC1 = cs;
+  const double* AC3 = cs + 2 * ny;
   double2* v2 = reinterpret_cast<double2*>(vs) + (kxl < KT ? kxl : 0);  // row r at v2[KT r]
   const double* w = ws + (kxl < KT ? kxl : 0);                           // row r at w[KT r]
-  if (mean && part == 0) {
-    // SP0B (mkp.f:271-288) on the re and im columns of kx = 0
-    double2 pm = make_double2(0.0, 0.0), pc = pm, Dj = v2[0];
-    v2[0] = make_double2(0.0, 0.0);
-#pragma unroll 4
-    for (int J = 1; J <= ny - 1; ++J) {
-      const double2 Dn = v2[KT * J];
-      const double a1 = __ldg(AC1 + J - 1), a2 = __ldg(AC2 + J - 1);
-      const double a3 = rAC3 ? __ldg(rAC3 + J - 1) : 1.0 / __ldg(AC3 + J - 1);
-      const double2 pn = make_double2(sp0b_row(Dj.x, pm.x, pc.x, a1, a2, a3),
-                                      sp0b_row(Dj.y, pm.y, pc.y, a1, a2, a3));
-      v2[KT * J] = pn;
-      pm = pc;
-      pc = pn;
-      Dj = Dn;
-    }
-  }
+  // (the two lanes of the mean column: part 0 its real part, part 1 its imaginary)
+  if (mean) sp0b_march<2 * KT>(vs + part, AC1, cs + ny, cs + 3 * ny, ny);
   // this lane's rows: q = 0 .. cnt-1 is row r0 + dr q
   const int cnt = part ? ny - m : m;
   const int r0 = part ? ny - 1 : 0, dr = part ? -1 : 1;
@@ -1377,8 +1417,8 @@ __global__ void __launch_bounds__(32) k_spn_babe_tma(const __grid_constant__ CUt
   o.y = __shfl_xor_sync(0xffffffffu, y.y, 16);
   if (valid) {
     const double2 ytop = part ? o : y, zbot = part ? y : o;
-    const double cT = __dmul_rn(__ldg(AC3 + m - 1), w[KT * (m - 1)]);
-    const double cBm = __dmul_rn(__ldg(AC1 + m), w[KT * m]);
+    const double cT = __dmul_rn(AC3[m - 1], w[KT * (m - 1)]);
+    const double cBm = __dmul_rn(AC1[m], w[KT * m]);
     const double2 xm = make_double2(spn_meet(ytop.x, zbot.x, cT, cBm),
                                     spn_meet(ytop.y, zbot.y, cT, cBm));
     double2 x = part ? xm : make_double2(__fma_rn(-cT, xm.x, ytop.x),
