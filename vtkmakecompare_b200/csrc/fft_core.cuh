@@ -182,7 +182,7 @@ struct DftSmall<9, CT> {  // n = 3a + b, k = c + 3e
 // values are exchanged through shared memory so that thread c holds the 16
 // partial sums of its c; the outer 16-point DFT leaves X[c + 16e] in its
 // register e.  One exchange and no block-wide barrier per transform (the
-// x kernels synchronise a warp, the z kernel its CTA).
+// x kernels synchronise a warp).
 // W16^m = exp(-2 pi i m/16) for the products m = a1*e0 of the 4 x 4 split
 template <class CT>
 __device__ __forceinline__ CT w16(int m, bool inv) {

@@ -9,9 +9,10 @@
 //    spectra are separated with the Hermitian identities;
 //  * z pass: a CTA holds W adjacent kx columns of one plane (W x NZ complex)
 //    and runs W complex FFTs of length NZ;
-//  * both use a Stockham autosort FFT (radix 4, 2, 3, 5 stages; Govindaraju
-//    et al., SC'08 formulation) with twiddles exp(-2 pi i k/N) taken from a
-//    table computed on the host in extended precision.
+//  * both use a Stockham autosort FFT (Govindaraju et al., SC'08 formulation)
+//    with twiddles exp(-2 pi i k/N) taken from a table computed on the host in
+//    extended precision: two stages in registers where N = R1 x R2 with both
+//    at most 16, radix 4, 2, 3, 5 stages through shared memory otherwise.
 // Spectral solve (SPN/SP0B): one thread per (kx,kz) wavenumber runs CTRIDIAG
 // (tridiag.f:43-58) along y, coalesced over kx; the mean mode runs SP0B's
 // forward marching.  This file keeps FMA contraction enabled (the transform
@@ -313,7 +314,9 @@ __global__ void k_fft_inv_x(FFTShape sh, int npair, Dims d, SpecViewT<CT> sv, do
 // the radix-4/2/3/5 stages above have four or five of each for N = 64 .. 135.
 // One pass, stages above -> here (us, events around each): 64^3 z 9 -> 5, x back
 // 8 -> 8; 100x75x90 z 16 -> 8, x back 11 -> 9; a whole lean step of 64^3 83 ->
-// 71 us, 100x75x90 160 -> 147, 128x96x128 255 -> 225.  Lengths without two such
+// 71 us, 100x75x90 160 -> 147, 128x96x128 255 -> 225.  At 256x192x256 the z passes
+// (107 MB each way) take 42 and 40 us, where one CTA of 256 threads and 128
+// registers for 16 columns took 47 and 47.  Lengths without two such
 // factors (125, 200, 216, 243, 250 and the powers above 256) keep the stages.
 template <class F>
 __device__ __forceinline__ void with_radix(int R, F f) {
@@ -358,12 +361,17 @@ __device__ __forceinline__ double quotient(double x, double d, double r, bool& a
 }
 __device__ __forceinline__ float quotient(float x, float d, float, bool&) { return x / d; }
 
-// z pass: a CTA holds F2_W adjacent kx columns of plane jj; thread (c, j) runs
-// the butterfly j of column c in both stages.  NORM as in k_fft256_z; the values
-// that need a division after all are divided apart, out of the common path.
+// z pass: a CTA holds F2_W adjacent kx columns (kx0 + 8 blockIdx.x, below kx1) of
+// one plane; thread (c, j) runs the butterfly j of column c in both stages.  NORM,
+// the forward pass's division by NX NZ: 2 divides (`quotient`; the values that need
+// a division after all are divided apart, out of the common path); 1 multiplies by
+// the reciprocal, where NX NZ is a power of two and the product is the quotient;
+// 0 none (the inverse pass).  Five CTAs an SM: uncapped the forward pass takes
+// four (45 us at 256x192x256 against 42), and at six it spills (53).
 constexpr int F2_W = 8;
 template <class CT, int NORM>
-__global__ void __launch_bounds__(F2_W * 16) k_fft2_z(int R1, int R2, int H, SpecViewT<CT> sv,
+__global__ void __launch_bounds__(F2_W * 16, 5) k_fft2_z(int R1, int R2, int kx0, int kx1,
+                                                      SpecViewT<CT> sv,
                                                       const CT* __restrict__ tw, double nrm,
                                                       double rnrm) {
   constexpr bool INV = NORM == 0;
@@ -371,8 +379,8 @@ __global__ void __launch_bounds__(F2_W * 16) k_fft2_z(int R1, int R2, int H, Spe
   extern __shared__ __align__(16) char fsm[];
   CT* sm = reinterpret_cast<CT*>(fsm);  // [N][F2_W]
   const int c = threadIdx.x % F2_W, j = threadIdx.x / F2_W;
-  const int kx = blockIdx.x * F2_W + c;
-  const bool ok = kx < H;
+  const int kx = kx0 + blockIdx.x * F2_W + c;
+  const bool ok = kx < kx1;
   CT* col = sv.base + kx + sv.sj * (sv.j0 + (int)blockIdx.y);
   if (ok && j < R2)
     with_radix(R1, [&](auto rc) {
@@ -683,49 +691,6 @@ __global__ void __launch_bounds__(128, 5) k_fft256_inv_x(Dims d, SpecViewT<CT> s
       FP[c] = val;
       if (i == 0) FP[d.P(N, J, kb)] = val;
     }
-  }
-}
-
-// z pass, N = 256: a CTA transforms 16 adjacent kx columns of one plane
-// (column group g0 + blockIdx.x); thread (col, b) holds x[16a + b] of its
-// column (loads coalesced over col).  NORM, the forward pass's division by
-// NX*NZ: 2 divides; 1 multiplies by the reciprocal, which the host passes
-// only when NX*NZ is a power of two (then the product is the correctly
-// rounded quotient, the same bits without a division sequence per value);
-// 0 none (the inverse pass).
-template <class CT, int NORM>
-__global__ void __launch_bounds__(256) k_fft256_z(int H, SpecViewT<CT> sv,
-                                                  const CT* __restrict__ tw, double nrm,
-                                                  int g0) {
-  constexpr bool inv = NORM == 0;
-  using RT = typename CReal<CT>::T;
-  constexpr int FS = 17;
-  extern __shared__ __align__(16) char fsm[];
-  CT* S_ = reinterpret_cast<CT*>(fsm);  // [c][b][col], col stride 1, b stride 17
-  const int col = threadIdx.x & 15, b = threadIdx.x >> 4;
-  const int jj = sv.j0 + blockIdx.y;
-  const int kx = (g0 + blockIdx.x) * 16 + col;
-  const bool ok = kx < H;
-  CT* base = sv.base + kx + sv.sj * jj;
-  CT v[16];
-#pragma unroll
-  for (int a = 0; a < 16; ++a) v[a] = ok ? base[sv.sk * (16 * a + b)] : mkc<CT>(RT(0), RT(0));
-  fft256_inner(v, b, tw, inv != 0);
-#pragma unroll
-  for (int c = 0; c < 16; ++c) S_[(c * 16 + b) * FS + col] = v[c];
-  __syncthreads();
-  const int c = b;  // this thread now runs the outer DFT of index c
-#pragma unroll
-  for (int bb = 0; bb < 16; ++bb) v[bb] = S_[(c * 16 + bb) * FS + col];
-  dft16(v, inv != 0);
-  if (!ok) return;
-  const RT rn = (RT)nrm;
-#pragma unroll
-  for (int e = 0; e < 16; ++e) {
-    CT w = v[e];
-    if (NORM == 2) { w.x = w.x / rn; w.y = w.y / rn; }
-    if (NORM == 1) { w.x = w.x * rn; w.y = w.y * rn; }
-    base[sv.sk * (c + 16 * e)] = w;
   }
 }
 
@@ -1609,44 +1574,25 @@ void launch_div_src32(const Dims& d, const GridRcp& rg, const float* ut, const f
   div_src<float>(d, rg, ut, vt, wt, dt, out, wrap, s);
 }
 
-// g0, ng: the groups of 16 kx columns to transform (ng = 0: all; only the
-// NZ = 256 kernel takes a subset)
+// g0, ng: the groups of 16 kx columns to transform (ng = 0: all; only lengths of
+// two stages take a subset)
 template <class CT>
 static void fft_z(const PoissonPlan& pp, bool inverse, cudaStream_t s, int j0 = 0, int nj = 0,
                   int g0 = 0, int ng = 0) {
   if (nj <= 0) { j0 = 0; nj = pp.ny; }
   SpecViewT<CT> sv = spec_internal_t<CT>(pp);
   sv.j0 = j0;
-  if (pp.nz == 256) {
-    if (ng <= 0) { g0 = 0; ng = (pp.H + 15) / 16; }
-    dim3 grid(ng, nj);
-    size_t sm = 16 * 16 * 17 * sizeof(CT);
-    const double nrm = (double)pp.nx * (double)pp.nz;
-    int e2 = 0;
-    const bool pow2 = frexp(nrm, &e2) == 0.5;  // nrm = 2^(e2-1)
-    count_launch();
-    if (inverse) {
-      smem_optin((const void*)k_fft256_z<CT, 0>, sm);
-      k_fft256_z<CT, 0><<<grid, 256, sm, s>>>(pp.H, sv, twz_of<CT>(pp), nrm, g0);
-    } else if (pow2) {
-      smem_optin((const void*)k_fft256_z<CT, 1>, sm);
-      k_fft256_z<CT, 1><<<grid, 256, sm, s>>>(pp.H, sv, twz_of<CT>(pp), 1.0 / nrm, g0);
-    } else {
-      smem_optin((const void*)k_fft256_z<CT, 2>, sm);
-      k_fft256_z<CT, 2><<<grid, 256, sm, s>>>(pp.H, sv, twz_of<CT>(pp), nrm, g0);
-    }
-    return;
-  }
   const double nrm = (double)pp.nx * (double)pp.nz;
   int e2 = 0, R1, R2;
   const bool pow2 = !inverse && frexp(nrm, &e2) == 0.5;
   if (two_factors(pp.nz, &R1, &R2)) {
-    dim3 grid((pp.H + F2_W - 1) / F2_W, nj);
+    const int kx0 = 16 * g0, kx1 = ng > 0 ? std::min(pp.H, 16 * (g0 + ng)) : pp.H;
+    dim3 grid((kx1 - kx0 + F2_W - 1) / F2_W, nj);
     const int nt = F2_W * R2;
     const size_t sm = (size_t)F2_W * pp.nz * sizeof(CT);
     count_launch();
     auto kern = inverse ? k_fft2_z<CT, 0> : pow2 ? k_fft2_z<CT, 1> : k_fft2_z<CT, 2>;
-    kern<<<grid, nt, sm, s>>>(R1, R2, pp.H, sv, twz_of<CT>(pp), nrm, 1.0 / nrm);
+    kern<<<grid, nt, sm, s>>>(R1, R2, kx0, kx1, sv, twz_of<CT>(pp), nrm, 1.0 / nrm);
     return;
   }
   FFTShape sh = make_shape(pp.nz);
@@ -1770,8 +1716,8 @@ void launch_spn_fast(const PoissonPlan& pp, cudaStream_t s) {
 // so the slice's spectrum (107 MB / nchunk at 256x192x256) is re-read from
 // L2 instead of HBM by the second and third pass.  Every column sees the
 // same operations as in the unsliced order (the passes act on disjoint
-// columns), so the result is bit-identical.  Slicing needs the N = 256 z
-// kernel and the tabulated SPN; otherwise the three passes run whole.
+// columns), so the result is bit-identical.  Slicing needs NZ = 256
+// and the tabulated SPN; otherwise the three passes run whole.
 int poisson_mid_groups(const PoissonPlan& pp) {
   return (pp.nz == 256 && pp.spn_im) ? (pp.H + 15) / 16 : 0;
 }
