@@ -431,35 +431,37 @@ __global__ void __launch_bounds__(256, (M >= 16 ? 2 : 4)) k_xlines(Dims d, S* __
   constexpr int HW = 32 / PL;  // lines per warp at a time
   __shared__ R stab[MASKED ? 1 : NVC * PL];
   const int lane = threadIdx.x & (PL - 1), half = (threadIdx.x & 31) / PL;
-  const long warp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int n = d.nx;
   const unsigned FULL = 0xffffffffu;
   if (!MASKED) {
     for (int t = threadIdx.x; t < NVC * PL; t += blockDim.x) stab[t] = __ldg(tab + t);
     __syncthreads();
   }
-  const long nlines = MASKED ? count : (long)jtop * d.nz;
-  const long ngroups = (nlines + NL * HW - 1) / (NL * HW);
-  for (long gi = warp; gi < ngroups; gi += nwarps) {
+  // (32-bit line numbers: at most 512 x 512, and a 64-bit quotient per line and
+  // lane was a tenth of a pass of 128x96x128, 18.6 -> 16.5 us)
+  const int nlines = MASKED ? count : jtop * d.nz;
+  const int ngroups = (nlines + NL * HW - 1) / (NL * HW);
+  for (int gi = warp; gi < ngroups; gi += nwarps) {
     XTab<R, PL> tb;
     tb.lane = lane;
     // (masked pass: NL = 1, table of line gi*HW + half)
-    tb.p = MASKED ? tab + (size_t)min(gi * HW + half, (long)count - 1) * (size_t)(NVC * PL)
+    tb.p = MASKED ? tab + (size_t)min(gi * HW + half, count - 1) * (size_t)(NVC * PL)
                   : stab;
     S* line[NL];
     bool ok[NL];
     R x[NL][M];
 #pragma unroll
     for (int q = 0; q < NL; ++q) {
-      const long l = (gi * NL + q) * HW + half;
-      long id = 0;
+      const int l = (gi * NL + q) * HW + half;
+      int id = 0;
       ok[q] = l < nlines;
       if (ok[q]) {
         if (MASKED) id = ids[l];
         else { id = l; ok[q] = slots[l] < 0; }  // masked lines: their own pass
       }
-      const int j = 1 + (int)(id % jtop), k = 1 + (int)(id / jtop);
+      const int k0 = id / jtop, j = 1 + id - k0 * jtop, k = 1 + k0;
       line[q] = f + d.P(0, j, k);
       if constexpr (STG) continue;
       // unknowns t = lane*M + r at positions t (t = 0 stands for x(n))
@@ -652,9 +654,11 @@ __global__ void __launch_bounds__(256, (M >= 16 ? 2 : 4)) k_xlines(Dims d, S* __
 // while these are solved) and the lanes pick their partitions from there; the
 // solution leaves the same way.  Lines that touch the mask read their own
 // table in the same pass.  The arithmetic is k_xlines'.
-// What bounds it: shared-memory and shuffle latency, not DRAM.  Before it,
-// these lengths ran one thread per line (k_lines, in all three directions):
-// 20 steps of 100x75x90 with their copies took 13.4 ms, now 5.5 ms.
+// What bounds it: shared-memory and shuffle latency, not DRAM: a pass of
+// 100x75x90 takes 14.7 us (16.6 with 64-bit line numbers and the table copied
+// before the first lines are asked for).  Before it, these lengths ran one thread
+// per line (k_lines, in all three directions): 20 steps of 100x75x90 with their
+// copies took 13.4 ms, 5.5 ms with it.
 template <int MM, int PL>
 __global__ void __launch_bounds__(256, MM > 8 ? 2 : 4)
     k_xlines_any(Dims d, double* __restrict__ f, int jtop, const double* __restrict__ tab,
@@ -665,14 +669,15 @@ __global__ void __launch_bounds__(256, MM > 8 ? 2 : 4)
   const int n = d.nx, t32 = threadIdx.x & 31;
   const int k = t32 & (PL - 1), h = t32 / PL;
   double* buf = xsm + NV * PL + (size_t)(threadIdx.x >> 5) * 2 * HW * n;
-  for (int t = threadIdx.x; t < NV * PL; t += blockDim.x) xsm[t] = __ldg(tab + t);
-  __syncthreads();
-  const long nlines = (long)jtop * d.nz, ngroups = (nlines + HW - 1) / HW;
-  const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
-  auto line_at = [&](long l) { return f + d.P(1, 1 + (int)(l % jtop), 1 + (int)(l / jtop)); };
-  auto fetch = [&](long gi, double* b) {
+  const int nlines = jtop * d.nz, ngroups = (nlines + HW - 1) / HW;
+  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  auto line_at = [&](int l) {
+    const int k0 = l / jtop;
+    return f + d.P(1, 1 + l - k0 * jtop, 1 + k0);
+  };
+  auto fetch = [&](int gi, double* b) {
     for (int q = 0; q < HW; ++q) {
-      const long l = gi * HW + q;
+      const int l = gi * HW + q;
       if (l >= nlines) break;
       const double* src = line_at(l);
       for (int t = t32; t < n; t += 32) cp_async8(b + q * n + t, src + t);
@@ -680,13 +685,16 @@ __global__ void __launch_bounds__(256, MM > 8 ? 2 : 4)
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
   const int s = k * n / PL, m = (k + 1) * n / PL - s;
-  long gi = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  // (the first lines are under way while the table is copied)
+  int gi = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (gi < ngroups) fetch(gi, buf);
+  for (int t = threadIdx.x; t < NV * PL; t += blockDim.x) xsm[t] = __ldg(tab + t);
+  __syncthreads();
   for (int it = 0; gi < ngroups; gi += nwarps, ++it) {
     double* cur = buf + (it & 1) * HW * n;
     if (gi + nwarps < ngroups) fetch(gi + nwarps, buf + ((it & 1) ^ 1) * HW * n);
     else asm volatile("cp.async.commit_group;\n" ::: "memory");
-    const long l = gi * HW + h;
+    const int l = gi * HW + h;
     const bool ok = l < nlines;
     const int slot = ok ? slots[l] : -1;
     XTab<double, PL> tb;
