@@ -226,6 +226,7 @@ struct PoissonPlan {
   const float* twx_f;         // the same twiddles rounded to FP32
   const float* twz_f;
   const double* spn_im;       // SPN pivot reciprocals [nz][ny][Hp] (null: none)
+  bool stages = false;        // transforms keep the radix-4/2/3/5 stages (mixed form)
   int spn_cp = 0;             // 1: the two-ended SPN stages by cp.async, not TMA tiles
   const double* rAC3 = nullptr;  // 1/AC3 [ny] for SP0B's marching (null: computed inline)
 };

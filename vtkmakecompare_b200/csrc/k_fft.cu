@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(F2_XT) k_fft2_fwd_x(Fft2X x, Dims d, SpecViewT
   }
 }
 
-template <class CT, bool ACC>
+template <class CT>
 __global__ void __launch_bounds__(F2_XT) k_fft2_inv_x(Fft2X x, Dims d, SpecViewT<CT> sv,
                                                       double* FP, const CT* __restrict__ tw) {
   using RT = typename CReal<CT>::T;
@@ -544,14 +544,9 @@ __global__ void __launch_bounds__(F2_XT) k_fft2_inv_x(Fft2X x, Dims d, SpecViewT
       double* ob = oa + d.sy;
       double* oz = oa + d.nz * d.sy;  // the S2P wrap (k_fft_inv_x)
       auto put = [&](int i, CT z) {
-        double a = (double)z.x, b = (double)z.y;
-        if (ACC) a = oa[i] + a;
-        oa[i] = a;
-        if (ka == 0) oz[i] = a;
-        if (two) {
-          if (ACC) b = ob[i] + b;
-          ob[i] = b;
-        }
+        oa[i] = (double)z.x;
+        if (ka == 0) oz[i] = (double)z.x;
+        if (two) ob[i] = (double)z.y;
       };
 #pragma unroll
       for (int r = 0; r < R; ++r) put(r * R1, v[r]);
@@ -1479,7 +1474,10 @@ template <> const float2* twz_of<float2>(const PoissonPlan& pp) {
 }
 
 // N = R1 x R2 of the two-stage transforms, the two as equal as they come; false
-// when N has no such factors (then the radix-4/2/3/5 stages)
+// when N has no such factors (then the radix-4/2/3/5 stages).  Plans of the mixed
+// form ask for the stages as well (PoissonPlan::stages): its FP32 fields turn
+// another last bit of the pressure into other FP32 roundings, 1.8e-6 after 40 steps,
+// as far as it is from FP64.  256 = 16 x 16 has the same bits either way.
 static bool two_factors(int N, int* R1, int* R2) {
   *R1 = 0;
   for (int a : {2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16})
@@ -1490,7 +1488,7 @@ static bool two_factors(int N, int* R1, int* R2) {
 // (the threads of a pair touch R2 adjacent samples on the way in and R1 on the
 // way out, so the longer factor goes where the samples are)
 static bool fft2_x(const PoissonPlan& pp, Fft2X* x, dim3* grid, int nj, bool inverse) {
-  if (!two_factors(pp.nx, &x->R1, &x->R2)) return false;
+  if (pp.stages || !two_factors(pp.nx, &x->R1, &x->R2)) return false;
   x->T = x->R2;
   if (inverse) std::swap(x->R1, x->R2);
   x->npair = F2_XT / x->T;
@@ -1523,17 +1521,19 @@ static void fwd_x(const PoissonPlan& pp, const Dims& d, const FwdSrc<S>& q, int 
       k_fft256_fwd_x<CT, S, 2><<<grid, 128, 0, s>>>(d, sv, q, twx_of<CT>(pp));
     return;
   }
-  Fft2X x2;
   dim3 grid;
-  if (fft2_x(pp, &x2, &grid, nj, false)) {
-    const size_t sm2 = (size_t)x2.npair * x2.pitch * sizeof(CT);
-    count_launch();
-    if (src_mode == 0)
-      k_fft2_fwd_x<CT, S, true><<<grid, F2_XT, sm2, s>>>(x2, d, sv, q, 0, twx_of<CT>(pp));
-    else
-      k_fft2_fwd_x<CT, S, false><<<grid, F2_XT, sm2, s>>>(x2, d, sv, q, src_mode,
-                                                          twx_of<CT>(pp));
-    return;
+  if constexpr (sizeof(CT) == 16) {  // (plans of the FP32 transforms keep the stages)
+    Fft2X x2;
+    if (fft2_x(pp, &x2, &grid, nj, false)) {
+      const size_t sm2 = (size_t)x2.npair * x2.pitch * sizeof(CT);
+      count_launch();
+      if (src_mode == 0)
+        k_fft2_fwd_x<CT, S, true><<<grid, F2_XT, sm2, s>>>(x2, d, sv, q, 0, twx_of<CT>(pp));
+      else
+        k_fft2_fwd_x<CT, S, false><<<grid, F2_XT, sm2, s>>>(x2, d, sv, q, src_mode,
+                                                            twx_of<CT>(pp));
+      return;
+    }
   }
   FFTShape sh = make_shape(pp.nx);
   int npair = row_pairs(pp);
@@ -1585,7 +1585,7 @@ static void fft_z(const PoissonPlan& pp, bool inverse, cudaStream_t s, int j0 = 
   const double nrm = (double)pp.nx * (double)pp.nz;
   int e2 = 0, R1, R2;
   const bool pow2 = !inverse && frexp(nrm, &e2) == 0.5;
-  if (two_factors(pp.nz, &R1, &R2)) {
+  if ((!pp.stages || pp.nz == 256) && two_factors(pp.nz, &R1, &R2)) {
     const int kx0 = 16 * g0, kx1 = ng > 0 ? std::min(pp.H, 16 * (g0 + ng)) : pp.H;
     dim3 grid((kx1 - kx0 + F2_W - 1) / F2_W, nj);
     const int nt = F2_W * R2;
@@ -1802,14 +1802,15 @@ static void inv_x(const PoissonPlan& pp, const Dims& d, double* FP, bool accumul
     k_fft256_inv_x<CT><<<grid, 128, 0, s>>>(d, sv, FP, twx_of<CT>(pp), accumulate ? 1 : 0);
     return;
   }
-  Fft2X x2;
   dim3 grid;
-  if (fft2_x(pp, &x2, &grid, nj, true)) {
-    count_launch();
-    auto kern = accumulate ? k_fft2_inv_x<CT, true> : k_fft2_inv_x<CT, false>;
-    kern<<<grid, F2_XT, (size_t)x2.npair * x2.pitch * sizeof(CT), s>>>(x2, d, sv, FP,
-                                                                       twx_of<CT>(pp));
-    return;
+  if constexpr (sizeof(CT) == 16) {
+    Fft2X x2;
+    if (!accumulate && fft2_x(pp, &x2, &grid, nj, true)) {
+      count_launch();
+      k_fft2_inv_x<CT><<<grid, F2_XT, (size_t)x2.npair * x2.pitch * sizeof(CT), s>>>(
+          x2, d, sv, FP, twx_of<CT>(pp));
+      return;
+    }
   }
   FFTShape sh = make_shape(pp.nx);
   int npair = row_pairs(pp);

@@ -1870,6 +1870,7 @@ int nse_ctx_create(const nse_config* cfg, nse_ctx** out) {
                          x->hdy12.data(), c.xl, c.zl, x->own);
   ok = ok && ((c.flags & NSE_FLAG_EXACT) || x->pb.build_tables(x->own));
   x->pb.pp.spn_cp = (c.flags & NSE_FLAG_SPN_CPASYNC) ? 1 : 0;
+  x->pb.pp.stages = x->mixed;
   ok = ok && build_line_tables(x);
   if (!ok) {
     nse_ctx_destroy(x);
