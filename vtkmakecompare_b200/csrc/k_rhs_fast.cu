@@ -268,9 +268,11 @@ __global__ void __launch_bounds__(TXW * TY, MINB) k_correct_pipe(
       const double ph = PH(qc, 0, 0), phx = PH(qc, 1, 0), phy = PH(qc, 0, 1), phz = PH(qp, 0, 0),
                    phxm = PH(qc, -1, 0), phym = PH(qc, 0, -1), phzm = PH(qm, 0, 0);
       const double gx = (phx - ph) * rx12, gy = (phy - ph) * ry12, gz = (phz - ph) * rz12;
-      const double un = corrected((double)fc[Lay::ui(tx, ty, 0)], dt, gx);
-      const double vn = corrected((double)fc[Lay::VO + Lay::vi(tx, ty, 0)], dt, gy);
-      const double wn = corrected((double)fc[Lay::WO + Lay::wi(tx, ty)], dt, gz);
+      // (the operations of corrected(), whose products u_ta takes as well)
+      const double ax = __dmul_rn(dt, gx), ay = __dmul_rn(dt, gy), az = __dmul_rn(dt, gz);
+      const double un = __dsub_rn((double)fc[Lay::ui(tx, ty, 0)], ax);
+      const double vn = __dsub_rn((double)fc[Lay::VO + Lay::vi(tx, ty, 0)], ay);
+      const double wn = __dsub_rn((double)fc[Lay::WO + Lay::wi(tx, ty)], az);
       const double um = (double)fc[Lay::ui(tx, ty, -1)] - dt * ((ph - phxm) * rx12m);
       const double vm = (double)fc[Lay::VO + Lay::vi(tx, ty, -1)] - dt * ((ph - phym) * ry12m);
       const double wm = (double)fm[Lay::WO + Lay::wi(tx, ty)] - dt * ((ph - phzm) * rz12m);
@@ -287,9 +289,9 @@ __global__ void __launch_bounds__(TXW * TY, MINB) k_correct_pipe(
       v_ep2[c] = (H)((double)old[TILE] - dt * (pyp - ph) * ry12);
       w_ep2[c] = (H)((double)old[2 * TILE] - dt * (pzp - ph) * rz12);
       divu[c] = (H)((un - um) * rx + (vn - vm) * ry + (wn - wm) * rz);
-      u_ta[c] = (H)(dt * gx);
-      v_ta[c] = (H)(dt * gy);
-      w_ta[c] = (H)(dt * gz);
+      u_ta[c] = (H)ax;
+      v_ta[c] = (H)ay;
+      w_ta[c] = (H)az;
     }
     if constexpr (!TMA) cp_async_wait<F - 1>();
     __syncthreads();
