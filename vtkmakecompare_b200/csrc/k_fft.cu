@@ -1178,8 +1178,8 @@ __global__ void __launch_bounds__(64) k_spn_babe(int H, int ny, int nz, int m, R
 // leave by one TMA store.  Lane = 16 half + kxl (kxl < 12): each lane runs the
 // re and im recurrences of its half (half 0: rows 0..m-1 downwards, half 1:
 // rows ny-1..m upwards), which share the pivots; a half-warp's accesses to a
-// row are contiguous (no bank conflicts).  The row loads run SPN_U rows ahead of
-// the recurrence, so the shared-memory latencies overlap the dependent FMA chain.
+// row are contiguous (no bank conflicts).  The row loads run four rows ahead of
+// the recurrence (eight without COEFS), so the shared-memory latencies overlap the dependent FMA chain.
 // The coefficients are copied beside the tile while it is under way: from L1 each
 // row waited for them, and each line of 16 rows for L2.  Columns kx >= H are outside both tensor
 // maps (zero-filled on load, not stored); columns kx0 + ... >= kx1 (the end of
@@ -1187,18 +1187,17 @@ __global__ void __launch_bounds__(64) k_spn_babe(int H, int ny, int nz, int m, R
 // march SP0B on the tile's kx = 0 column.  Forward solve only (the
 // transposed solve keeps k_spn_babe).  Bounded waits: a TMA copy that does
 // not arrive sets g_spn2_wait_err and the tile is not stored.
-constexpr int SPN_KT = 12, SPN_U = 4;
+constexpr int SPN_KT = 12;
 // One sweep of the two-ended recurrence over n rows of a lane's half: row j
 // of the sweep is v[j sv], w[j sv], c[j sc].  DOWN: elimination y(j) =
 // (d(j) - c(j) y(j-1)) w(j); else back substitution x(j) = y(j) - c(j) w(j)
 // x(j-1); each result replaces the row's value.  A row's registers take the
-// row SPN_U further on as soon as they are used, and the addresses step by
+// row U further on as soon as they are used, and the addresses step by
 // additions: 44 cycles a row of one warp alone, 56 with two buffers of 8 rows
 // filled in turn and their last rows loaded as they are needed.
-template <bool DOWN>
+template <bool DOWN, int U>
 __device__ __forceinline__ void spn_sweep(double2* v, const double* w, const double* c, int sv,
                                           int sc, int n, double2& y) {
-  constexpr int U = SPN_U;
   double2 d[U];
   double wr[U], cr[U];
   double2* o = v;
@@ -1302,22 +1301,23 @@ __device__ int g_spn2_wait_err = 0;
 __host__ __device__ inline size_t spn_tile_piv_off(int ny) {
   return ((size_t)ny * 2 * SPN_KT * sizeof(double) + 127) & ~(size_t)127;
 }
-__host__ __device__ inline size_t spn_tile_smem(int ny) {
-  return spn_tile_piv_off(ny) + (size_t)ny * (SPN_KT + 4) * sizeof(double) + 16;
+__host__ __device__ inline size_t spn_tile_smem(int ny, bool coefs) {
+  return spn_tile_piv_off(ny) + (size_t)ny * (SPN_KT + (coefs ? 4 : 0)) * sizeof(double) + 16;
 }
 
+template <bool COEFS>
 __global__ void __launch_bounds__(32) k_spn_babe_tma(const __grid_constant__ CUtensorMap tv,
                                                      const __grid_constant__ CUtensorMap tp,
                                                      int H, int ny, int m,
                                                      const double* __restrict__ AC,
                                                      const double* __restrict__ rAC3, int kx0,
                                                      int kx1) {
-  constexpr int KT = SPN_KT;
+  constexpr int KT = SPN_KT, U = COEFS ? 4 : 8;
   extern __shared__ __align__(128) unsigned char sbt_sm[];
   double* vs = reinterpret_cast<double*>(sbt_sm);                        // [ny][2 KT]
   double* ws = reinterpret_cast<double*>(sbt_sm + spn_tile_piv_off(ny));  // [ny][KT]
   double* cs = ws + (size_t)ny * KT;  // AC1, AC2, AC3, 1/AC3
-  uint64_t* bar = reinterpret_cast<uint64_t*>(cs + 4 * (size_t)ny);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(cs + (COEFS ? 4 * (size_t)ny : 0));
   const int lane = threadIdx.x;
   const int kb = kx0 + KT * blockIdx.x, kz = blockIdx.y;
   const bool aligned = ((reinterpret_cast<uintptr_t>(&tv) & 63) == 0) &&
@@ -1334,8 +1334,10 @@ __global__ void __launch_bounds__(32) k_spn_babe_tma(const __grid_constant__ CUt
     tma_load_3d(vs, &tv, 2 * kb, 0, kz, bar);
     tma_load_3d(ws, &tp, kb, 0, kz, bar);
   }
-  for (int r = lane; r < 3 * ny; r += 32) cs[r] = __ldg(AC + r);
-  for (int r = lane; r < ny; r += 32) cs[3 * ny + r] = __ldg(rAC3 + r);
+  if (COEFS) {
+    for (int r = lane; r < 3 * ny; r += 32) cs[r] = __ldg(AC + r);
+    for (int r = lane; r < ny; r += 32) cs[3 * ny + r] = __ldg(rAC3 + r);
+  }
   __syncwarp();
   if (!tma_wait(bar, 0)) {
     // the copies of this tile did not arrive: record it, give them one more
@@ -1348,12 +1350,12 @@ __global__ void __launch_bounds__(32) k_spn_babe_tma(const __grid_constant__ CUt
   const int kx = kb + kxl;
   const bool mean = (kx == 0 && kz == 0);
   const bool valid = kxl < KT && kx < kx1 && kx < H && !mean;
-  const double* AC1 = cs;
-  const double* AC3 = cs + 2 * ny;
+  const double* AC1 = COEFS ? cs : AC;
+  const double* AC3 = AC1 + 2 * ny;
   double2* v2 = reinterpret_cast<double2*>(vs) + (kxl < KT ? kxl : 0);  // row r at v2[KT r]
   const double* w = ws + (kxl < KT ? kxl : 0);                           // row r at w[KT r]
   // (the two lanes of the mean column: part 0 its real part, part 1 its imaginary)
-  if (mean) sp0b_march<2 * KT>(vs + part, AC1, cs + ny, cs + 3 * ny, ny);
+  if (mean) sp0b_march<2 * KT>(vs + part, AC1, AC1 + ny, COEFS ? cs + 3 * ny : rAC3, ny);
   // this lane's rows: q = 0 .. cnt-1 is row r0 + dr q
   const int cnt = part ? ny - m : m;
   const int r0 = part ? ny - 1 : 0, dr = part ? -1 : 1;
@@ -1369,7 +1371,7 @@ __global__ void __launch_bounds__(32) k_spn_babe_tma(const __grid_constant__ CUt
     const double w0 = wb[0];
     y = make_double2(spn_down(true, d0.x, 0.0, 0.0, w0), spn_down(true, d0.y, 0.0, 0.0, w0));
     vb[0] = y;
-    spn_sweep<true>(vb + sv, wb + sv, cfe + dr, sv, dr, cnt - 1, y);
+    spn_sweep<true, U>(vb + sv, wb + sv, cfe + dr, sv, dr, cnt - 1, y);
   }
   // y(m-1) of the top lane, z(m) of the bottom lane
   double2 o;
@@ -1388,7 +1390,7 @@ __global__ void __launch_bounds__(32) k_spn_babe_tma(const __grid_constant__ CUt
     // half) over q = cnt-2 .. 0, from the meeting point outwards
     const int qs = r0 + dr * (cnt - 2);
     const double* cfb = (part ? AC1 : AC3) + qs;
-    spn_sweep<false>(v2 + KT * qs, w + KT * qs, cfb, -sv, -dr, cnt - 1, x);
+    spn_sweep<false, U>(v2 + KT * qs, w + KT * qs, cfb, -sv, -dr, cnt - 1, x);
   }
   fence_async_smem();
   __syncwarp();
@@ -1663,13 +1665,19 @@ static bool spn_babe_tma(const PoissonPlan& pp, cudaStream_t s, int g0 = 0, int 
                      1) ||
       !tma_encode_3d(&tp, pp.spn_im, true, pp.H, pp.ny, pp.nz, sp1, sp2, SPN_KT, pp.ny, 1))
     return false;
-  const size_t sm = spn_tile_smem(pp.ny);
-  smem_optin((const void*)k_spn_babe_tma, sm);
+  // the coefficients beside the tile as long as an SM holds three (228 KB and 1 KB
+  // a CTA): at 256^3 two take 98 us and three that read them through L1 88; at
+  // 256x192x256 three take 62.6 and four without 63.4
+  auto tiles = [&](bool coefs) { return 228 * 1024 / (spn_tile_smem(pp.ny, coefs) + 1024); };
+  const bool coefs = tiles(true) >= 3 || tiles(true) == tiles(false);
+  const size_t sm = spn_tile_smem(pp.ny, coefs);
+  auto kern = coefs ? k_spn_babe_tma<true> : k_spn_babe_tma<false>;
+  smem_optin((const void*)kern, sm);
   const int kx0 = ng > 0 ? 16 * g0 : 0;
   const int kx1 = ng > 0 ? std::min(16 * (g0 + ng), pp.H) : pp.H;
   if (kx1 <= kx0) return true;
   count_launch();
-  k_spn_babe_tma<<<dim3((kx1 - kx0 + SPN_KT - 1) / SPN_KT, pp.nz), 32, sm, s>>>(
+  kern<<<dim3((kx1 - kx0 + SPN_KT - 1) / SPN_KT, pp.nz), 32, sm, s>>>(
       tv, tp, pp.H, pp.ny, m, pp.AC, pp.rAC3, kx0, kx1);
   return true;
 }
