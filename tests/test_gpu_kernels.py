@@ -288,3 +288,50 @@ def test_spn_tiles_of_any_height(ny):
             ctx.poisson()
             out.append(ctx.download("phi"))
     assert out[0].any() and np.array_equal(out[0], out[1])
+
+
+# The adjoint's recorded steps start from device memory that held something else
+# before and must not read a cell that no one wrote.  Blocks below 1 MB share the
+# driver's 2 MB chunks, so holes between live blocks of NaN are what the adjoint's
+# fields get.  Same bits as with a checkpoint before every step, whose start state
+# is a copy of the context's fields.
+@pytest.mark.parametrize("n,every", [((12, 13, 12), 2), ((12, 13, 12), 4), ((16, 14, 15), 3)])
+def test_adjoint_on_recycled_memory(n, every):
+    import ctypes as C
+
+    import torch
+    cu = C.CDLL("libcuda.so.1")
+    g, f, c1, par = make_case(*n, seed=8)
+    out = []
+    for k in (1, every):
+        cfg = S.Config(*n, par["dt"], par["Re"], par["Sc"], 50.0, g["xl"], g["yl"], g["zl"],
+                       y0=-1.0, ystretch=2.0, body_force=par["force"], t_bot=1.0,
+                       t_solid=par["tsolid"])
+        with S.Context(cfg) as ctx:
+            for name in ("u", "v", "w", "T"):
+                ctx.upload(name, f[name])
+            ctx.upload("cellvalue", c1)
+            ctx.project()
+            ctx.start()
+            ctx.step(2)
+            ctx.sync()
+            torch.cuda.synchronize()
+            blocks = []
+            for fields in (4, 7 * k, 10, 11, 16 * k):
+                for _ in range(16):
+                    p, size = C.c_uint64(), C.c_size_t(fields * f["u"].nbytes)
+                    assert cu.cuMemAlloc_v2(C.byref(p), size) == 0
+                    blocks.append(p)
+                    assert cu.cuMemsetD8_v2(p, C.c_ubyte(255), size) == 0
+            torch.cuda.synchronize()
+            for p in blocks[::2]:
+                assert cu.cuMemFree_v2(p) == 0
+            with S.Adjoint(ctx, 9, checkpoint_every=k, avg_from=5) as adj:
+                adj.set_weight("v", f["w"])
+                J, grad = adj.gradient()
+                out.append([np.array(J), grad] + [adj.initial_adjoint(q)[1:-1, 1:-1, 1:-1]
+                                                  for q in ("u", "v", "w", "T", "u_ta", "w_pre")])
+            for p in blocks[1::2]:
+                assert cu.cuMemFree_v2(p) == 0
+    for q, (a, b) in enumerate(zip(*out)):
+        assert np.linalg.norm(a) > 0 and np.array_equal(a, b), q

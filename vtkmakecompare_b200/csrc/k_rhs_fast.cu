@@ -387,7 +387,8 @@ __global__ void __launch_bounds__(256) k_correct_step(
     }
     if (edge || k == 1 || k == d.nz) {
       // the ghost images of this cell: periodic in x and z, u and w negated
-      // behind the walls (v's wall faces are zero already)
+      // behind the walls, v zero on the lower wall's face (its row j = ny + 1, which
+      // SET_BC leaves, is left)
       const int xi[3] = {i, i == 1 ? d.nx + 1 : -1, i == d.nx ? 0 : -1};
       const int zi[3] = {k, k == 1 ? d.nz + 1 : -1, k == d.nz ? 0 : -1};
       const int yi[3] = {j, j == 1 ? 0 : -1, top ? d.ny + 1 : -1};
@@ -399,7 +400,7 @@ __global__ void __launch_bounds__(256) k_correct_step(
             const long g = d.P(xi[a], yi[e], zi[b]);
             u[g] = e ? -un : un;
             w[g] = e ? -wn : wn;
-            if (e == 0) v[g] = vn;
+            if (e < 2) v[g] = e ? 0.0 : vn;
           }
         }
     }
