@@ -477,6 +477,9 @@ long long nse_alloc_bytes(void);
 
 /* number of kernel launches this process has issued through the library */
 long long nse_launch_count(void);
+/* number of CUDA graphs this process has made through the library, or (launches
+ * not 0) of graph launches it has issued */
+long long nse_graph_count(int launches);
 
 #ifdef __cplusplus
 }

@@ -358,3 +358,32 @@ def test_transform_error_against_80_bits(n, forward, inverse):
     P = O.field(n, ny, n)
     G.s2p(F, P, n, ny, n)
     assert np.linalg.norm(P[:n, 1:-1, :n] - want) <= inverse * np.linalg.norm(want)
+
+
+# Graphs of steps are made where they are used often: a call of 5 steps makes those of
+# the steps in between, and a call of 20 or 21 after it none; the ones that begin
+# and end a call come with its third use, a mask change starts over.
+@pytest.mark.parametrize("prec", [S.FP64, S.MIXED])
+@pytest.mark.parametrize("steps", [20, 21])
+def test_long_call_after_a_short_one_makes_no_graph(prec, steps):
+    g, f, c1, par = make_case(64, 24, 18, seed=4)
+    cfg = S.Config(64, 24, 18, par["dt"], par["Re"], par["Sc"], par["eta"], g["xl"], g["yl"],
+                   g["zl"], y0=-1.0, ystretch=2.0, precision=prec)
+    with S.Context(cfg) as ctx:
+        for k in ("u", "v", "w", "T"):
+            ctx.upload(k, f[k])
+        ctx.upload("cellvalue", c1)
+        ctx.project()
+        ctx.start()
+        made = []
+        for m in [5] + [steps] * 9:
+            n0 = S.graph_count()
+            ctx.step(m)
+            made.append(S.graph_count() - n0)
+        assert made[0] == (2 if prec == S.FP64 else 1) and made[1] == 0 and made[-1] == 0, made
+        assert sum(made[2:]) > 0
+        ctx.upload("cellvalue", np.asfortranarray(1.0 * (c1 > 0.5)))
+        n0, r0 = S.graph_count(), S.graph_count(True)
+        ctx.step(steps)
+        assert S.graph_count() - n0 == made[0]
+        assert S.graph_count(True) - r0 == steps - 3

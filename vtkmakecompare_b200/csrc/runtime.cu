@@ -166,6 +166,16 @@ static std::atomic<long long> g_launches{0};
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 // a graph replay launches the kernels its capture counted
 static void count_launches(long long n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
+// graphs made and graph launches (nse_graph_count)
+static std::atomic<long long> g_graphs[2];
+static cudaError_t make_graph(cudaGraphExec_t* ex, cudaGraph_t g) {
+  g_graphs[0].fetch_add(1, std::memory_order_relaxed);
+  return cudaGraphInstantiate(ex, g, 0);
+}
+static cudaError_t launch_graph(cudaGraphExec_t ex, cudaStream_t s) {
+  g_graphs[1].fetch_add(1, std::memory_order_relaxed);
+  return cudaGraphLaunch(ex, s);
+}
 
 DBuf& arena(int slot) {
   static DBuf slots[48];
@@ -254,6 +264,7 @@ const char* nse_last_error(void) { return g_msg; }
 void nse_set_alloc_limit(long long bytes) { g_alloc_limit.store(bytes > 0 ? bytes : 0); }
 long long nse_alloc_bytes(void) { return g_alloc_bytes.load(); }
 long long nse_launch_count(void) { return g_launches.load(); }
+long long nse_graph_count(int launches) { return g_graphs[launches ? 1 : 0].load(); }
 int nse_last_status(void) { return g_status; }
 void nse_clear_error(void) {
   g_status = NSE_OK;
@@ -1313,9 +1324,9 @@ static bool run_levelset(const Dims& d, const GridDev& g, const GridRcp* rg, dou
     cudaGraph_t gr = nullptr;
     cudaGraphExec_t ex = nullptr;
     if (cudaStreamEndCapture(s, &gr) == cudaSuccess && gr &&
-        cudaGraphInstantiate(&ex, gr, 0) == cudaSuccess)
+        make_graph(&ex, gr) == cudaSuccess)
       for (; ok && left >= LS_SWEEPS; left -= LS_SWEEPS) {
-        ok = NSE_CUDA(cudaGraphLaunch(ex, s));
+        ok = NSE_CUDA(launch_graph(ex, s));
         count_launches(LS_SWEEPS);
       }
     cudaGetLastError();
@@ -1529,8 +1540,10 @@ unsigned long long shape_sig(const nse_ctx* x) {
 }
 void drop_step_graphs(nse_ctx* x) {
   for (auto& g : x->sg) {
-    if (g.ex) cudaGraphExecDestroy(g.ex);
+    if (!g.ex) continue;
+    cudaGraphExecDestroy(g.ex);
     g.ex = nullptr;
+    g.uses = 0;
   }
 }
 }  // namespace
@@ -2886,7 +2899,7 @@ static void ctx_step(nse_ctx* x, int in = END_FULL, int out = END_FULL) {
 }  // extern "C"
 
 extern "C" {
-static int step_replay(nse_ctx* x, int in, int out);
+static int step_replay(nse_ctx* x, int in, int out, int after);
 }
 
 // internal hooks of the adjoint driver (adjoint.cu)
@@ -2907,7 +2920,7 @@ int ctx_get_l(nse_ctx* x) { return x->l; }
 void ctx_set_l(nse_ctx* x, int l) { x->l = l; }
 bool ctx_lean_ok(nse_ctx* x) { return lean_ok(x); }
 void ctx_step_rec(nse_ctx* x, double* const* rec, int in, int out) {
-  if (!rec && step_replay(x, in, out) == 1) return;
+  if (!rec && step_replay(x, in, out, 2) == 1) return;
   x->rec = rec;
   ctx_step(x, in, out);
   x->rec = nullptr;
@@ -3008,16 +3021,16 @@ extern "C" {
 // launches depend on the host-side state only through the step counter
 // (l == 1 is the Euler start), the way it starts and ends (in, out) and the
 // temperature buffer pair (the FP64 form swaps T and its work buffer every
-// step), so the second and later steps of one kind and starting buffer replay
-// its graph.  Step l = 1, the first of each kind and buffer, steps after the
-// mask changed, profiled and recorded steps, and steps on a stream that is
-// being captured run eagerly (false).  The
-// capture leaves the host-side state of the step behind (counter, buffer
-// pair) and is launched at once; a replay sets that state the same way.
+// step), so later steps of one kind and starting buffer replay its graph.  It is
+// made when a step of its kind comes for the `after`-th time (nse_step).  Step
+// l = 1, steps after the mask changed, profiled and recorded steps, and steps on
+// a stream that is being captured run eagerly (false).  The capture leaves the
+// host-side state of the step behind (counter, buffer pair) and is launched at
+// once; a replay sets that state the same way.
 // Returns 1 (replayed), 0 (step eagerly) or -1 (a CUDA error).  A launch
 // shape, a masked line list's length or a table's place that differs from
 // the capture drops the graphs (a new mask is tabulated by an eager step).
-static int step_replay(nse_ctx* x, int in, int out) {
+static int step_replay(nse_ctx* x, int in, int out, int after) {
   if (x->sg_off || x->mask_dirty || x->prof_n < x->prof_cap || x->rec) return 0;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(x->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
@@ -3032,14 +3045,16 @@ static int step_replay(nse_ctx* x, int in, int out) {
   if (!g) return 0;  // (nine kinds and two buffers: never)
   g->kind = kind;
   g->t = t0;
-  if (++g->uses < 2 || x->l < 2) return 0;
   const unsigned long long sig = shape_sig(x);
-  if (sig != x->sg_sig) {
+  if (x->l >= 2 && sig != x->sg_sig) {
     drop_step_graphs(x);
     x->sg_sig = sig;
   }
+  ++g->uses;
+  if (x->l < 2) return 0;
+  if (!g->ex && g->uses < after) return 0;
   if (g->ex) {
-    if (!NSE_CUDA(cudaGraphLaunch(g->ex, x->stream))) return -1;
+    if (!NSE_CUDA(launch_graph(g->ex, x->stream))) return -1;
     count_launches(g->nk);
     x->f[NSE_T] = g->T;
     x->uT = g->uT;
@@ -3059,7 +3074,7 @@ static int step_replay(nse_ctx* x, int in, int out) {
   cudaGraph_t gr = nullptr;
   const cudaError_t ce = cudaStreamEndCapture(x->stream, &gr);
   cudaGraphExec_t ex = nullptr;
-  const bool ok = ce == cudaSuccess && gr && cudaGraphInstantiate(&ex, gr, 0) == cudaSuccess;
+  const bool ok = ce == cudaSuccess && gr && make_graph(&ex, gr) == cudaSuccess;
   if (gr) cudaGraphDestroy(gr);
   if (!ok) {
     // nothing ran: put the host-side state back and step eagerly
@@ -3071,7 +3086,7 @@ static int step_replay(nse_ctx* x, int in, int out) {
     x->sg_off = true;
     return 0;
   }
-  if (!NSE_CUDA(cudaGraphLaunch(ex, x->stream))) {
+  if (!NSE_CUDA(launch_graph(ex, x->stream))) {
     cudaGraphExecDestroy(ex);
     count_launches(-nk);
     x->l = l0;
@@ -3089,9 +3104,19 @@ static int step_replay(nse_ctx* x, int in, int out) {
 int nse_step(nse_ctx* x, int nsteps) {
   if (!x || nsteps < 0) return NSE_ERR_ARG;
   int in = END_FULL;
+  bool lean = false;  // this call has lean steps
   for (int n = 1; n <= nsteps; ++n) {
     const int out = step_end(x, n, nsteps);
-    const int r = step_replay(x, in, out);
+    lean = lean || out == END_LEAN;
+    // Making a graph takes 0.45 ms of host time (and as long as the driver is busy for
+    // another process that reads the GPU's counters); an eager step takes 0.07 ms
+    // more than a replay where the GPU needs less than 0.13 ms for it, and nothing
+    // where it needs more.  So the step between lean ones, which a call repeats,
+    // gets its graph at once, and those that begin and end a call's lean steps, which
+    // come once a call, at the third call: with all of them at the second, 20 steps
+    // of 64^3 after a call of 5 took 2.27 ms, like this 1.49, later ones 1.36.
+    const int after = in == END_LEAN && out == END_LEAN ? 1 : lean ? 3 : 2;
+    const int r = step_replay(x, in, out, after);
     if (r < 0) return status_or(NSE_ERR_CUDA);
     if (r == 0) ctx_step(x, in, out);
     in = out;
@@ -3405,7 +3430,7 @@ static bool ens_capture(nse_ensemble* e, int in, int mid, int out) {
     if (g) cudaGraphDestroy(g);
     return false;
   }
-  ok = NSE_CUDA(cudaGraphInstantiate(&e->exec[in != END_FULL][out != END_FULL], g, 0));
+  ok = NSE_CUDA(make_graph(&e->exec[in != END_FULL][out != END_FULL], g));
   cudaGraphDestroy(g);
   return ok;
 }
@@ -3485,7 +3510,7 @@ int nse_ensemble_step(nse_ensemble* e, int nsteps) {
     on_graph = true;
     cudaGraphExec_t& ex = e->exec[a][b];
     if (!ex) ok = ok && ens_capture(e, in, e1, e2);
-    ok = ok && NSE_CUDA(cudaGraphLaunch(ex, e->origin));
+    ok = ok && NSE_CUDA(launch_graph(ex, e->origin));
     if (ok) count_launches(e->nk[a][b]);
     for (nse_ctx* x : e->cases) x->l += 2;
     in = e2;

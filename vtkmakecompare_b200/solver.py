@@ -84,6 +84,7 @@ def _sig():
     L.nse_ctx_set_line_shapes.argtypes = [vp, C.c_int, C.c_int]
     L.nse_ctx_phase_times.argtypes = [vp, vp, C.c_int, vp]
     L.nse_launch_count.restype = C.c_longlong
+    L.nse_graph_count.restype = C.c_longlong
     L.nse_ensemble_create.argtypes = [vp, C.c_int, C.c_int, C.POINTER(vp)]
     L.nse_ensemble_step.argtypes = [vp, C.c_int]
     L.nse_ensemble_set_stream.argtypes = [vp, vp]
@@ -101,6 +102,11 @@ def _sig():
 def launch_count():
     """Kernel launches issued by libnsegpu.so in this process."""
     return int(_sig().nse_launch_count())
+
+
+def graph_count(launches=False):
+    """CUDA graphs made (or, with `launches`, graph launches) in this process."""
+    return int(_sig().nse_graph_count(int(launches)))
 
 
 class Context:
