@@ -222,8 +222,12 @@ __device__ __forceinline__ void load_hist_async(char* sm, const Dims& d, int i0,
 // H: storage type of the histories, u_ta and the outputs (double; float in
 // the mixed-precision form); CT: arithmetic type (FP32 arithmetic rounds the
 // FP64 state as it is read from the ring).  TM: how the ring is filled (see
-// RhsLay; tm holds the tensor maps of a TMA fill).
-template <class H, class CT, int TY, int NS, int MINB, int TM>
+// RhsLay; tm holds the tensor maps of a TMA fill).  LEAN: u_ta, v_ta, w_ta are
+// dt grad(phi) of the previous step, whose correction did not write them.  A form of
+// its own: one kernel that asks for phi at run time has 6 registers more and takes
+// longer in full steps as well (us a launch, one kernel -> two: 128x96x128 69.9 -> 66.3,
+// 512x192x256 637.7 -> 636; FP32 storage 66.3 -> 61.9, 642 -> 634.5).
+template <class H, class CT, int TY, int NS, int MINB, int TM, bool LEAN>
 __global__ void __launch_bounds__(TXW * TY, MINB) k_rhs_fast(
     Dims d, GridDev g, GridRcp rg, StepParams sp, const double* __restrict__ U,
     const double* __restrict__ V, const double* __restrict__ W, const double* __restrict__ T,
@@ -241,7 +245,8 @@ __global__ void __launch_bounds__(TXW * TY, MINB) k_rhs_fast(
   const int i0 = 1 + blockIdx.x * TXW, j0 = 1 + blockIdx.y * TY;
   const int I = i0 + threadIdx.x, J = j0 + threadIdx.y;
   const bool valid = (I <= d.nx) && (J <= d.ny);
-  const int k0 = 1 + blockIdx.z * kc;  // (kc <= KCHUNK planes per CTA)
+  __builtin_assume(kc >= 1 && kc <= KCHUNK);  // (2 registers and 0.3% of the time)
+  const int k0 = 1 + blockIdx.z * kc;
   const int k1 = min(d.nz, k0 + kc - 1);
   const int kmax = k1 + 1;  // last plane any iteration reads
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + NS * Lay::SLOT);
@@ -348,11 +353,11 @@ __global__ void __launch_bounds__(TXW * TY, MINB) k_rhs_fast(
       const R c4 = (K < d.nz) ? (cc1 + C1AT(pp, 0, 0)) * R(0.5) : cc1;
       const H* hist = reinterpret_cast<const H*>(pc + Lay::HOFF) + t0;
       const bool solid = (c2 != R(0)) || (c3 != R(0)) || (c4 != R(0)) || (cc1 != R(0));
-      // u_ta, v_ta, w_ta: the fields, or with PHI given dt grad(phi) of the
-      // previous step, whose correction then did not write them (the same
-      // value: the correction's expression, from interior cells of phi)
-      auto ta = [&](const H* f, long nb, double r12) {
-        return PHI ? (R)(H)(sp.dt * ((LD(PHI, nb) - LD(PHI, c)) * r12)) : (R)LD(f, c);
+      // u_ta, v_ta, w_ta: the fields, or (LEAN) the same value from phi: the
+      // correction's expression, from interior cells
+      auto ta = [&](const H* f, long nb, const double* r12, int q) {
+        if constexpr (LEAN) return (R)(H)(sp.dt * ((LD(PHI, nb) - LD(PHI, c)) * LD(r12, q)));
+        else return (R)LD(f, c);
       };
     // u
     {
@@ -376,7 +381,7 @@ __global__ void __launch_bounds__(TXW * TY, MINB) k_rhs_fast(
       R ua = a1 * uv + a2 * (R)hist[0] + kd * L;
       U_PRE[c] = uv;
       if (solid && c2 != R(0)) {
-        ua += (R)sp.eta * c2 * ta(U_TA, I < d.nx ? c + 1 : c + 1 - d.nx, LD(rg.rdx12, I)) * DT;
+        ua += (R)sp.eta * c2 * ta(U_TA, I < d.nx ? c + 1 : c + 1 - d.nx, rg.rdx12, I) * DT;
         U_A[c] = (uc + ua) / (R(1) + (R)sp.eta * c2 * DT);
       } else {
         U_A[c] = uc + ua;
@@ -404,7 +409,7 @@ __global__ void __launch_bounds__(TXW * TY, MINB) k_rhs_fast(
       R va = a1 * vv + a2 * (R)hist[TILE] + kd * L;
       V_PRE[c] = vv;
       if (solid && c3 != R(0))
-        va += (R)sp.eta * c3 * ta(V_TA, J < d.ny ? c + d.sx : c, LD(rg.rdy12, J)) * DT;
+        va += (R)sp.eta * c3 * ta(V_TA, J < d.ny ? c + d.sx : c, rg.rdy12, J) * DT;
       if (J == d.ny) va = R(0);  // set_bc(u_a,v_a,...) zeroes v_a(:,ny,:)
       if (solid && c3 != R(0)) V_A[c] = (vc + va) / (R(1) + (R)sp.eta * c3 * DT);
       else V_A[c] = vc + va;
@@ -432,7 +437,7 @@ __global__ void __launch_bounds__(TXW * TY, MINB) k_rhs_fast(
       W_PRE[c] = wv;
       if (solid && c4 != R(0)) {
         wa += (R)sp.eta * c4 *
-              ta(W_TA, K < d.nz ? c + d.sy : c - (d.nz - 1) * d.sy, LD(rg.rdz12, K)) * DT;
+              ta(W_TA, K < d.nz ? c + d.sy : c - (d.nz - 1) * d.sy, rg.rdz12, K) * DT;
         W_A[c] = (wc + wa) / (R(1) + (R)sp.eta * c4 * DT);
       } else {
         W_A[c] = wc + wa;
@@ -513,7 +518,7 @@ static bool rhs_go(const Dims& d, const GridDev& g, const GridRcp& rg, const Ste
   }
   dim3 block(TXW, TY, 1);
   dim3 grid((d.nx + TXW - 1) / TXW, (d.ny + TY - 1) / TY, (d.nz + kc - 1) / kc);
-  auto kern = k_rhs_fast<H, CT, TY, NS, MINB, TM>;
+  auto kern = phi ? k_rhs_fast<H, CT, TY, NS, MINB, TM, true> : k_rhs_fast<H, CT, TY, NS, MINB, TM, false>;
   cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   count_launch();
   kern<<<grid, block, smem, s>>>(d, g, rg, sp, u, v, w, T, u_ta, v_ta, w_ta, u_pre, v_pre, w_pre,
