@@ -2610,10 +2610,13 @@ static void autotune_rhs(nse_ctx* x, const StepParams& sp) {
   // few give a small grid more CTAs than the 2 x 2 x 4 .. of 16 planes and a
   // shorter march.  Measured per launch, 16 planes against the fastest:
   // 64^3 29.7 -> 17.4 us (4), 100x75x90 38.6 -> 29.7 (8), 128x96x128 65.2 ->
-  // 57.7 (8), 160x92x135 78.8 -> 68.6, 128^3 75.4 -> 72.0, 256x192x256 323
-  // either way (16 stays)
+  // 57.7 (8), 160x92x135 78.8 -> 68.6, 192x96x192 106.8 -> 102.0, 256x128x192
+  // 172 -> 169, 192^3 189 either way.  From 2048 tiles of 32 x 8 x 16 cells on
+  // the 16 stay (256x160x256 270 -> 269, 256^3 424 -> 422, 320x200x300 480 either
+  // way), untimed: at 512x256x512 the timing would take 30 ms.
   const int fewer[4] = {12, 8, 4, 2};
-  for (int cand = 0; cand < nshape + 4; ++cand) {
+  const long tiles = (long)((d.nx + 31) / 32) * ((d.ny + 7) / 8) * ((d.nz + 15) / 16);
+  for (int cand = 0; cand < nshape + (tiles < 2048 ? 4 : 0); ++cand) {
     const int shape = cand < nshape ? cand : best, kc = cand < nshape ? 0 : fewer[cand - nshape];
     auto run = [&]() {
       if (x->mixed)
