@@ -90,7 +90,7 @@ bool run_forward(nse_adjoint* a) {
     // one, else what the next step reads
     int out = n + 2 > N ? END_FULL : (n % K == 0 ? END_TA : END_LEAN);
     if (!ctx_lean_ok(a->x)) out = END_FULL;
-    ctx_step_rec(a->x, nullptr, in, out);
+    if (!ctx_step_rec(a->x, nullptr, in, out)) return false;
     in = out;
     if (n >= n0)
       launch_wall_flux(ci.d, g, ctx_field(a->x, NSE_T), c.t_bot, c.thc, c.xl, c.zl, w, J, ci.s);
@@ -318,7 +318,8 @@ int nse_adjoint_gradient(nse_adjoint* a, double* J, double* grad_c1) {
       if (!lean || r == 0)
         if (!copy_fields(a, seg(r, 0), segIds, kSeg, false)) return NSE_ERR_CUDA;
       if (!lean) {
-        ctx_step_rec(a->x, recp.data() + (size_t)r * kRec, END_FULL, END_FULL);
+        if (!ctx_step_rec(a->x, recp.data() + (size_t)r * kRec, END_FULL, END_FULL))
+          return NSE_ERR_CUDA;
         continue;
       }
       RecordedStep io;

@@ -345,8 +345,9 @@ int ctx_get_l(nse_ctx* x);
 void ctx_set_l(nse_ctx* x, int l);
 // one step of the context; with rec given, the line-solve passes record their
 // inputs and outputs (16 padded fields, see nse_ctx::rec).  in, out: see
-// StepEnd (out is taken as END_FULL where ctx_lean_ok says no)
-void ctx_step_rec(nse_ctx* x, double* const* rec, int in, int out);
+// StepEnd (out is taken as END_FULL where ctx_lean_ok says no).  False: the replay
+// of a captured step failed, and nothing ran
+bool ctx_step_rec(nse_ctx* x, double* const* rec, int in, int out);
 // What a step leaves behind, and what the next one may start from.  END_FULL:
 // every field, as MKP writes them.  END_LEAN: u, v, w with their ghosts, T and
 // the histories (phi holds the pressure); END_TA: u_ta, v_ta, w_ta as well.

@@ -2922,11 +2922,14 @@ double* ctx_field(nse_ctx* x, int id) { return F(x, id); }
 int ctx_get_l(nse_ctx* x) { return x->l; }
 void ctx_set_l(nse_ctx* x, int l) { x->l = l; }
 bool ctx_lean_ok(nse_ctx* x) { return lean_ok(x); }
-void ctx_step_rec(nse_ctx* x, double* const* rec, int in, int out) {
-  if (!rec && step_replay(x, in, out, 2) == 1) return;
-  x->rec = rec;
-  ctx_step(x, in, out);
-  x->rec = nullptr;
+bool ctx_step_rec(nse_ctx* x, double* const* rec, int in, int out) {
+  const int r = rec ? 0 : step_replay(x, in, out, 2);
+  if (r == 0) {
+    x->rec = rec;
+    ctx_step(x, in, out);
+    x->rec = nullptr;
+  }
+  return r >= 0;
 }
 // A step of the lean form (ctx_lean_ok) whose fields live where its record is
 // kept, so that nothing is copied but the x passes' inputs: the right-hand side
