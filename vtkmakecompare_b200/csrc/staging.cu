@@ -180,9 +180,14 @@ bool host_copies(const HostCopy* list, int n, bool to_device, cudaStream_t s) {
     ok = good;
   } else {
     for (int q = 0; ok && q < n; ++q) ok = plain(list[q], to_device, s);
+    // (a page-locked array's copy is still under way here)
+    if (ok && !to_device) ok = cudaStreamSynchronize(s) == cudaSuccess;
   }
   if (ok) return true;
   const cudaError_t e = cudaGetLastError();
+  // copies that were queued before one failed still use the slots and the caller's
+  // arrays: wait for them while the slots are this call's
+  cudaStreamSynchronize(s);
   return cuda_ok(e != cudaSuccess ? e : cudaErrorUnknown, "copy between a host array and the GPU");
 }
 
