@@ -399,8 +399,10 @@ int nse_ctx_phase_times(nse_ctx* ctx, double* ms, int nphase, int* nsteps);
  * together.  Case i runs on stream i mod nstreams (owned by the ensemble;
  * nse_ensemble_destroy gives each case its own stream back).  The first step
  * of every case runs eagerly (the Euler start; it also builds the mask's
- * line tables); later steps replay a CUDA graph captured from two steps of
- * all cases, with an eager step for an odd remainder.  A case's mask and
+ * line tables); later steps replay CUDA graphs captured from two steps of all
+ * cases.  Eager are also the first step of a call that follows one of odd length, its
+ * last step where an odd number is left, and the first calls' first and last pairs of
+ * steps, which differ from those between them.  A case's mask and
  * parameters must not change while it belongs to an ensemble, and contexts
  * with NSE_FLAG_CHECK_FINITE are refused.  Asynchronous; nse_ensemble_sync
  * waits for all cases. */

@@ -3378,11 +3378,16 @@ struct nse_ensemble {
   bool own_origin = true;
   cudaEvent_t fork = nullptr;
   std::vector<cudaEvent_t> join;
-  // by how the step before it ended and how its second step ends (the first
-  // of two steps of a call ends lean unless it is the last but one)
-  cudaGraphExec_t exec[2][2] = {};
-  long long nk[2][2] = {};  // kernels in each graph (counted once per replay)
-  int uses[2][2] = {};
+  // by how the step before a pair ended and how its two steps end (lean or full: only
+  // the last two steps of a call end full)
+  struct PairGraph {
+    cudaGraphExec_t ex = nullptr;
+    long long nk = 0;  // its kernels (counted once per replay)
+    int uses = 0;
+  } pair[2][2][2];
+  PairGraph& graph(int in, int mid, int out) {
+    return pair[in != END_FULL][mid != END_FULL][out != END_FULL];
+  }
   // each case's temperature buffer when a graph was captured: the FP64
   // form swaps it with the work buffer every step, so a replay is valid only
   // after an even number of eager steps since the capture
@@ -3420,14 +3425,14 @@ static bool ens_capture(nse_ensemble* e, int in, int mid, int out) {
   for (nse_ctx* x : e->cases) l0.push_back(x->l);
   if (e->tbuf.empty())
     for (nse_ctx* x : e->cases) e->tbuf.push_back(x->f[NSE_T].p);
-  long long& nk = e->nk[in != END_FULL][out != END_FULL];
+  nse_ensemble::PairGraph& pg = e->graph(in, mid, out);
   if (!NSE_CUDA(cudaStreamBeginCapture(e->origin, cudaStreamCaptureModeRelaxed))) return false;
   const long long k0 = g_launches.load();
   bool ok = ens_fork_from_origin(e);
   for (int st = 0; ok && st < 2; ++st)
     for (nse_ctx* x : e->cases) ctx_step(x, st ? mid : in, st ? out : mid);
-  nk = g_launches.load() - k0;
-  count_launches(-nk);  // counted by each replay instead
+  pg.nk = g_launches.load() - k0;
+  count_launches(-pg.nk);  // counted by each replay instead
   ok = ok && ens_join_into_origin(e);
   cudaGraph_t g = nullptr;
   cudaError_t ce = cudaStreamEndCapture(e->origin, &g);
@@ -3436,7 +3441,7 @@ static bool ens_capture(nse_ensemble* e, int in, int mid, int out) {
     if (g) cudaGraphDestroy(g);
     return false;
   }
-  ok = NSE_CUDA(make_graph(&e->exec[in != END_FULL][out != END_FULL], g));
+  ok = NSE_CUDA(make_graph(&pg.ex, g));
   cudaGraphDestroy(g);
   return ok;
 }
@@ -3496,14 +3501,12 @@ int nse_ensemble_step(nse_ensemble* e, int nsteps) {
     // how the next two steps end (every case the same way; step_end)
     const int e1 = lean && nsteps > 2 ? END_LEAN : END_FULL;
     const int e2 = lean && nsteps > 3 ? END_LEAN : END_FULL;
-    // three left: one eagerly, so that a pair ends the call
-    eager = eager || (lean && nsteps == 3);
     for (size_t i = 0; i < e->tbuf.size(); ++i)
       eager = eager || e->cases[i]->f[NSE_T].p != e->tbuf[i];
-    // the first and the last two steps of a call take a graph of their own
-    // from the second call on (its capture costs more than one eager step)
-    const int a = in != END_FULL, b = e2 != END_FULL;
-    eager = eager || (lean && a + b < 2 && ++e->uses[a][b] < 2);
+    // the pairs that begin and end a call take a graph of their own from the
+    // second call on (its capture costs more than one eager step)
+    nse_ensemble::PairGraph& pg = e->graph(in, e1, e2);
+    if (!eager && lean && !(in && e1 && e2)) eager = ++pg.uses < 2;
     if (eager) {
       if (on_graph) ok = ens_fork_from_origin(e);
       on_graph = false;
@@ -3514,10 +3517,9 @@ int nse_ensemble_step(nse_ensemble* e, int nsteps) {
     }
     if (!on_graph) ok = ok && ens_join_into_origin(e);
     on_graph = true;
-    cudaGraphExec_t& ex = e->exec[a][b];
-    if (!ex) ok = ok && ens_capture(e, in, e1, e2);
-    ok = ok && NSE_CUDA(launch_graph(ex, e->origin));
-    if (ok) count_launches(e->nk[a][b]);
+    if (!pg.ex) ok = ok && ens_capture(e, in, e1, e2);
+    ok = ok && NSE_CUDA(launch_graph(pg.ex, e->origin));
+    if (ok) count_launches(pg.nk);
     for (nse_ctx* x : e->cases) x->l += 2;
     in = e2;
     nsteps -= 2;
@@ -3548,9 +3550,10 @@ int nse_ensemble_destroy(nse_ensemble* e) {
   for (cudaStream_t st : e->streams)
     if (st) cudaStreamSynchronize(st);
   for (size_t i = 0; i < e->cases.size(); ++i) e->cases[i]->stream = e->saved[i];
-  for (auto& row : e->exec)
-    for (cudaGraphExec_t ex : row)
-      if (ex) cudaGraphExecDestroy(ex);
+  for (auto& plane : e->pair)
+    for (auto& row : plane)
+      for (auto& g : row)
+        if (g.ex) cudaGraphExecDestroy(g.ex);
   for (cudaEvent_t ev : e->join)
     if (ev) cudaEventDestroy(ev);
   if (e->fork) cudaEventDestroy(e->fork);
