@@ -387,3 +387,10 @@ def test_long_call_after_a_short_one_makes_no_graph(prec, steps):
         ctx.step(steps)
         assert S.graph_count() - n0 == made[0]
         assert S.graph_count(True) - r0 == steps - 3
+
+
+# SPN by pipelined columns at the edges of its chunks of 8 rows: one row less, whole
+# chunks, one and two rows more.
+@pytest.mark.parametrize("ny", [7, 8, 9, 10, 15, 23, 24, 25, 26])
+def test_spn_columns_at_chunk_edges(ny):
+    test_spn_columns_match_oracle((10, ny, 9))

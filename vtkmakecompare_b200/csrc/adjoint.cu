@@ -144,7 +144,7 @@ void adjoint_step(nse_adjoint* a, double* const* sg, bool bc, double* const* rc,
     // kernel between solves; the first pass's is launch_adj_point's)
     if (comp == 3)
       launch_adj_line_scale(D, g, dirs[2], comp, false, bar[comp], nullptr, nullptr, c1, nullptr,
-                            c.dt, c.eta, cs);
+                            c.dt, c.eta, cs, -1);
     for (int p = 2; p >= 0; --p) {
       ctx_line_solve(a->x, dirs[p], comp, bar[comp], cs);
       if (p > 0)

@@ -442,9 +442,10 @@ __global__ void k_adj_point(PArgs a) {
 // A = D^-1 (D + S) with D = diag(alpha_j w_j), A^T = D A D^-1 and
 // A^-T = D A^-1 D^-1: the transposed solve is the step's own line solve
 // between two diagonal scalings.  `out` = 0: xb /= alpha w (before the
-// solve); 1: rbar = alpha w y, c_bar += rbar dt eta / alpha (r - x), and
-// when the pass has a predecessor (next >= 0, its direction) the result is
-// scaled at once for that pass's solve: xb = rbar / (alpha w_next).
+// solve); 1: rbar = alpha w y, c_bar += rbar dt eta / alpha (r - x), and the
+// result is scaled at once for the solve of the pass before it, of direction
+// `next`: xb = rbar / (alpha w_next).  (The first pass's output scaling is
+// k_adj_point's.)
 struct SArgs {
   Dims D;
   AdjGrid g;
@@ -472,11 +473,10 @@ __global__ void k_adj_line_scale(SArgs a) {
     a.xb[c] = cm == 0.0 ? v : v / (a.dte * cm + 1.0);
     return;
   }
-  // (rbar / alpha: alpha cancels in both results but the last pass's)
+  // (rbar / alpha: alpha cancels in both results)
   const double ra = x * line_w(a.g, a.dir, a.comp, ijk[a.dir]);
   a.cbar[D.C(i, j, k)] += ra * a.dte * (a.rin[c] - a.xout[c]);
-  if (a.next < 0) a.xb[c] = cm == 0.0 ? ra : (a.dte * cm + 1.0) * ra;
-  else a.xb[c] = ra * line_rw(a.g, a.next, a.comp, ijk[a.next]);
+  a.xb[c] = ra * line_rw(a.g, a.next, a.comp, ijk[a.next]);
 }
 
 // -------------------------------------------------------- MKP transposes --
@@ -882,7 +882,7 @@ void launch_adj_line_scale(const Dims& D, const AdjGrid& g, int dir, int comp, b
                            double* cbar, double dt, double eta, cudaStream_t s, int next) {
   SArgs a;
   a.D = D; a.g = g; a.xb = xb; a.rin = rin; a.xout = xout; a.c1 = c1; a.cbar = cbar;
-  a.dir = dir; a.comp = comp; a.out = out ? 1 : 0; a.next = out ? next : -1;
+  a.dir = dir; a.comp = comp; a.out = out ? 1 : 0; a.next = next;
   a.dte = dt * eta;
   count_launch();
   k_adj_line_scale<<<cell_grid(D, 128), 128, 0, s>>>(a);

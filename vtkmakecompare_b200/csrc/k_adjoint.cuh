@@ -43,10 +43,11 @@ void launch_adj_point(const Dims& D, double* const A[4], double* const B[4],
                       cudaStream_t s);
 // diagonal scalings around the step's own line solve that make it the
 // transposed solve (A^-T = D A^-1 D^-1, D = diag(alpha w)); out = false
-// before the solve, true after (with the mask gradient of the pass)
+// before the solve; true after it, with the mask gradient of the pass and the
+// scaling before the solve of the pass in front of it (direction `next`)
 void launch_adj_line_scale(const Dims& D, const AdjGrid& g, int dir, int comp, bool out,
                            double* xb, const double* rin, const double* xout, const double* c1,
-                           double* cbar, double dt, double eta, cudaStream_t s, int next = -1);
+                           double* cbar, double dt, double eta, cudaStream_t s, int next);
 // MKP transposed: phi_bar at the P2S samples, transposed SPN/SP0B on the
 // spectrum, divergence transposed with the scaling before the x passes
 void launch_adj_phibar(const Dims& D, const AdjGrid& g, const double* const ub[3],
