@@ -379,6 +379,10 @@ int nse_ctx_launch_shapes(nse_ctx* ctx, int* out);
  * the same values.  NSE_ERR_ARG for a code outside -1..6 (right-hand side)
  * or -1..15 (correction). */
 int nse_ctx_set_shapes(nse_ctx* ctx, int rhs_shape, int corr_shape);
+/* Fix the number of z planes that a CTA of the right-hand-side kernel marches, 1..16
+ * (a shape fixed by nse_ctx_set_shapes runs with 16), once that shape is fixed or tuned;
+ * every number gives the same values.  NSE_ERR_ARG before that and out of range. */
+int nse_ctx_set_rhs_planes(nse_ctx* ctx, int planes);
 /* Fix the launch shapes of every partitioned line pass (y/z: 0..3 as in
  * nse_ctx_launch_shapes; x: 1..4 lines per warp iteration / staged loads)
  * before the first step instead of the autotuner's choice; every shape gives

@@ -394,3 +394,53 @@ def test_long_call_after_a_short_one_makes_no_graph(prec, steps):
 @pytest.mark.parametrize("ny", [7, 8, 9, 10, 15, 23, 24, 25, 26])
 def test_spn_columns_at_chunk_edges(ny):
     test_spn_columns_match_oracle((10, ny, 9))
+
+
+# The explicit terms, full and lean form, with every number of z planes per CTA that the
+# tuning tries, and one and five, in every launch shape, bit for bit those of 16 planes in
+# the first: whole and partial tiles, nz below, at and past multiples, an obstacle.
+@pytest.mark.parametrize("prec,n", [(S.FP64, (64, 17, 45)), (S.FP64, (50, 15, 20)),
+                                    (S.MIXED, (96, 17, 15))])
+def test_explicit_terms_with_each_plane_count(prec, n):
+    g, f, c1, par = make_case(*n, seed=6)
+    ref = None
+    for shape in range(7):
+        for planes in (16, 12, 8, 5, 4, 2, 1):
+            cfg = S.Config(*n, par["dt"], par["Re"], par["Sc"], 50.0, g["xl"], g["yl"], g["zl"],
+                           y0=-1.0, ystretch=2.0, body_force=par["force"], t_bot=par["tbot"],
+                           t_solid=par["tsolid"], precision=prec, flags=S.FLAG_NO_AUTOTUNE)
+            with S.Context(cfg) as ctx:
+                ctx.set_shapes(rhs=shape, correct=0)
+                ctx.set_rhs_planes(planes)
+                for k in ("u", "v", "w", "T"):
+                    ctx.upload(k, f[k])
+                ctx.upload("cellvalue", c1)
+                ctx.start()
+                ctx.step(1)
+                ctx.step(4)  # two lean steps and two full ones
+                got = [ctx.download(k) for k in STATE]
+            ref = ref or got
+            for k, a, b in zip(STATE, ref, got):
+                assert np.isfinite(a).all() and np.array_equal(a, b), (k, shape, planes)
+
+
+def test_plane_counts_out_of_range_are_refused():
+    from vtkmakecompare_b200 import NseError
+    g, _, _, par = make_case(36, 9, 10, seed=6)
+    cfg = S.Config(36, 9, 10, par["dt"], par["Re"], par["Sc"], 50.0, g["xl"], g["yl"], g["zl"])
+    with S.Context(cfg) as ctx:
+        with pytest.raises(NseError):
+            ctx.set_rhs_planes(8)  # no shape fixed yet
+        ctx.set_shapes(rhs=1)
+        for planes in (0, 17, -1):
+            with pytest.raises(NseError):
+                ctx.set_rhs_planes(planes)
+        ctx.set_rhs_planes(16)
+
+
+# Level-set sweeps that march 4 and 8 cells a thread (from 600k and 2.5M cells), and 2
+# and 4 in replayed graphs, with nz off their multiples.
+@pytest.mark.parametrize("n,nnn", [((90, 60, 75), 130), ((96, 80, 81), 3), ((96, 80, 81), 129),
+                                   ((160, 128, 125), 3), ((150, 135, 135), 2)])
+def test_levelset_marches_match_oracle_bit_for_bit(n, nnn):
+    test_levelset_sweeps_match_oracle_bit_for_bit(n, nnn, 0)

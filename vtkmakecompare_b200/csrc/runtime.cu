@@ -3332,6 +3332,12 @@ int nse_ctx_set_shapes(nse_ctx* x, int rhs_shape, int corr_shape) {
   return NSE_OK;
 }
 
+int nse_ctx_set_rhs_planes(nse_ctx* x, int planes) {
+  if (!x || !x->rhs_tuned || planes < 1 || planes > 16) return NSE_ERR_ARG;
+  x->rhs_kc = planes;
+  return NSE_OK;
+}
+
 int nse_ctx_launch_shapes(nse_ctx* x, int* out) {
   if (!x || !out) return NSE_ERR_ARG;
   for (int dir = 1; dir <= 2; ++dir)

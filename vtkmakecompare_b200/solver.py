@@ -81,6 +81,7 @@ def _sig():
     L.nse_ctx_profile.argtypes = [vp, C.c_int]
     L.nse_ctx_launch_shapes.argtypes = [vp, vp]
     L.nse_ctx_set_shapes.argtypes = [vp, C.c_int, C.c_int]
+    L.nse_ctx_set_rhs_planes.argtypes = [vp, C.c_int]
     L.nse_ctx_set_line_shapes.argtypes = [vp, C.c_int, C.c_int]
     L.nse_ctx_phase_times.argtypes = [vp, vp, C.c_int, vp]
     L.nse_launch_count.restype = C.c_longlong
@@ -216,6 +217,10 @@ class Context:
         """Fix the right-hand-side and correction launch shapes (-1: autotuned);
         nsegpu.h, nse_ctx_set_shapes."""
         check(self.L.nse_ctx_set_shapes(self.h, int(rhs), int(correct)))
+
+    def set_rhs_planes(self, planes):
+        """Fix the z planes per CTA of the right-hand-side kernel (1..16)."""
+        check(self.L.nse_ctx_set_rhs_planes(self.h, int(planes)))
 
     def levelset(self, phi0, nnn=2000, dtau=1.0e-3, width=1.0, want_phi=True):
         a = np.asfortranarray(phi0, dtype=np.float64)
