@@ -444,3 +444,33 @@ def test_plane_counts_out_of_range_are_refused():
                                    ((160, 128, 125), 3), ((150, 135, 135), 2)])
 def test_levelset_marches_match_oracle_bit_for_bit(n, nnn):
     test_levelset_sweeps_match_oracle_bit_for_bit(n, nnn, 0)
+
+
+# Rounding of x lines of any length: one step of heat conduction along x alone (no flow,
+# cells 1e11 wide in y and z), so T is (I - b D)^-1 (I + b D) T0 with b D of order 0.1,
+# against long doubles.  Of T's roundings the right-hand side makes three and a solve that
+# adds its corrections up before it adds them to T one, sqrt(4 / 12) = 0.58 units in
+# the last place in the mean square; one that rounds T in every operation has 5 to 13
+# more a row, 0.9 units and above.  Bound: half way.
+@pytest.mark.parametrize("nx", [20, 36, 50, 75, 90, 100, 125, 150, 225, 270, 405, 500])
+def test_x_lines_of_any_length_round_once(nx):
+    ny, nz = 13, 12
+    cfg = S.Config(nx, ny, nz, 0.2, 1.0, 1.0, 1.0, float(nx), 1e11 * ny, 1e11 * nz,
+                   body_force=0.0, heat_source=0.0)
+    rng = np.random.default_rng(nx)
+    T = np.asfortranarray(1.0 + rng.random((nx + 2, ny + 2, nz + 2)))
+    with S.Context(cfg) as ctx:
+        ctx.upload("T", T)
+        ctx.start()
+        ctx.step(1)
+        got = ctx.download("T")[1:-1, 1:-1, 1:-1]
+    T0 = T[1:-1, 1:-1, 1:-1].reshape(nx, -1).astype(np.longdouble)
+    D = lambda x: np.roll(x, 1, 0) - 2 * x + np.roll(x, -1, 0)
+    b = np.longdouble(0.2) / 2
+    r = T0 + b * D(T0)
+    M = np.eye(nx) - float(b) * D(np.eye(nx))
+    x = np.zeros_like(r)
+    for _ in range(4):
+        x += np.linalg.solve(M, (r - (x - b * D(x))).astype(float))
+    err = (got.reshape(nx, -1) - x).astype(float) / 2.0 ** -52
+    assert np.sqrt(np.mean(err ** 2)) < 0.75, np.sqrt(np.mean(err ** 2))
