@@ -88,3 +88,23 @@ def test_ensemble_calls_of_odd_length_replay_their_pairs():
     finally:
         for c in ens_cases + solo:
             c.close()
+
+
+# A first call of one pair makes the graph of the pairs inside longer calls, so that the
+# long call after it makes none.
+@pytest.mark.parametrize("first", [2, 3])
+def test_ensemble_long_call_after_a_short_one_makes_no_graph(first):
+    cases = [make(n, p, 30 + i) for i, (n, p) in enumerate(SHAPES[-2:])]
+    try:
+        with S.Ensemble(cases, nstreams=2) as ens:
+            ens.step(1)
+            counts = []
+            for n_steps in (first, 20):
+                g0, l0 = S.graph_count(), S.graph_count(True)
+                ens.step(n_steps)
+                ens.sync()
+                counts.append((S.graph_count() - g0, S.graph_count(True) - l0))
+        assert counts[0][0] == 1 and counts[1][0] == 0 and counts[1][1] >= 8, counts
+    finally:
+        for c in cases:
+            c.close()

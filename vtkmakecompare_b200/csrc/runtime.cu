@@ -3513,6 +3513,13 @@ int nse_ensemble_step(nse_ensemble* e, int nsteps) {
     // third call on, as nse_step's steps do: making one takes 3 to 5 ms of host time for
     // eight cases of 64^3 to 160x128x160, their eager steps 0.7 ms of a call more than
     // replays.
+    // The graph of the pairs inside a call is made by the first call that has a pair, even
+    // where none of its own is one: a call of 20 steps of 32 cases after one of 2 took
+    // 146 ms when it made that graph itself, 136 without.
+    if (!eager && lean && !e->graph(END_LEAN, END_LEAN, END_LEAN).ex) {
+      ok = ens_capture(e, END_LEAN, END_LEAN, END_LEAN);
+      if (!ok) break;
+    }
     nse_ensemble::PairGraph& pg = e->graph(in, e1, e2);
     if (!eager && lean && !(in && e1 && e2)) eager = ++pg.uses < 3;
     if (eager) {
