@@ -315,7 +315,7 @@ __device__ __forceinline__ int periodic_pre(int p, int n, int* q) {
 // A CTA covers an (x, y) tile of one plane, so the y neighbours every cell
 // gathers are mostly the tile's own rows (L1 hits).  Bound by the latency of
 // those loads (1.5 TB/s of HBM, 1.2 instructions a cycle): 740 us for the four
-// fields at 128^3 with every neighbour checked, 460 through Near, 390 with 128
+// fields at 128^3 with every neighbour checked, 460 through Near, 363 with 128
 // threads at 64 registers, eight CTAs to an SM.
 template <int F>
 __global__ void __launch_bounds__(128, 8) k_adj_explicit(XArgs a, double* __restrict__ out) {

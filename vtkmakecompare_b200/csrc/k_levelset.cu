@@ -55,7 +55,8 @@ __device__ __forceinline__ double upwind(double lo, double hi) {
 // phi, where both sides count, crosses half of all warps).  *big: a value of
 // phi is too large for `quotient` (a sweep that writes one sets it, the
 // sweeps after it divide); so do grids with spacings out of its range (!RCP).
-// Bound by instruction issue (FP64, selects), not by memory: the sign factored
+// Bound by the latency of each cell's chain, not by memory (ncu at 256x192x256: issue
+// 52%, FP64 pipe 37%, DRAM 2.7 TB/s at 45% of the warp slots): the sign factored
 // out, five quotients for seven divisions and a square root, and no separate
 // ghost pass take a sweep of 256x192x256 from 218 to 101 us (46 us of HBM
 // traffic), of 128x96x128 from 30.6 to 13.6, of 64x48x64 from 11.1 to 3.7.

@@ -29,8 +29,8 @@
 //     through shared memory (k_xlines_any).
 //   y and z lines (strided): one CTA per 16 adjacent lines, one thread per
 //     (line, partition), threads of a partition adjacent; the reduced
-//     system goes through shared memory and is applied as its tabulated
-//     inverse (two rows per partition).
+//     system goes through shared memory and is solved by the same cyclic
+//     reduction over the partitions.
 #include <algorithm>
 
 #include "k_lines.cuh"
